@@ -47,7 +47,7 @@ enum {
 /* Contraction precision (slgpu_matrix_process / slgpu_rhs_assemble). */
 enum {
     SLGPU_PREC_FP64 = 0,  /* plain FP64 */
-    SLGPU_PREC_SPLIT = 1, /* FP64 operands split into 7 INT8 slices on the tensor cores (tcgen05 kind::i8), exact INT32
+    SLGPU_PREC_SPLIT = 1, /* FP64 operands split into 6 INT8 slices on the tensor cores (tcgen05 kind::i8), exact INT32
                              accumulation, FP64 recombination; <= 1e-10 relative per element matrix */
     SLGPU_PREC_FP32 = 2   /* same with 5 slices: FP32-level tier, <= 1e-6 */
 };
@@ -303,7 +303,7 @@ int slgpu_check_coefficient_kernels(slgpu_ctx* ctx, int handle, char* log, size_
  *   "contract_fp64"       FLOPs, 2*ntf*ndof*nterms*ngp per element
  *   "slice_cols"          bytes: coefficients read, slices and exponents written
  *   "contract_split"      INT8 tensor operations, 2*pairs*ntf*ndof*nterms*ngp per
- *   "contract_split_fp32" element (pairs = 28 for the split tier, 15 for FP32)
+ *   "contract_split_fp32" element (pairs = 21 for the split tier, 15 for FP32)
  *   "row_values"          bytes: kept element values + slots, incidences, row
  *                         pointers read; A and D values written
  * A family that did not run reports zeros.  No counterpart in the reference

@@ -38,7 +38,7 @@ struct JitGroup {
     const double* fielddata;
     const double* term_scale;
     double* C;
-    int* elemexp;
+    int* elemtop;
 };
 )";
 
@@ -171,14 +171,14 @@ std::string jit_coef_source(const std::vector<const GroupDev*>& batch)
         // second group of a transposed pair) gets C = null.
         s << "  if (grp.g[" << k << "].C != nullptr) {\n    const JitGroup q = grp.g[" << k << "];\n";
         emit_nodes(s, G, node_closure(G, all_terms(G)), ngp, "    ");
-        s << "    double cmax = 0;\n";
+        s << "    int top = 0;\n";
         for (int t = 0; t < G.nterms; t++) {
             const int c = G.term_node[t];
             s << "    { const double c = v" << c << " * q.term_scale[" << t << "] * wdet; q.C[((i64)" << t << " * " << ngp
-              << " + g) * p.nelem + e] = c; cmax = fmax(cmax, fabs(c)); }\n";
+              << " + g) * p.nelem + e] = c; top = max(top, __double2hiint(c) & 0x7fffffff); }\n";
         }
-        // Exponent of the element's largest coefficient for split precision.
-        s << "    if (q.elemexp != nullptr && cmax > 0) { int ex; frexp(cmax, &ex); atomicMax(q.elemexp + e, ex); }\n";
+        // High word of the element's largest coefficient for split precision.
+        s << "    if (q.elemtop != nullptr && top > 0) atomicMax(q.elemtop + e, top);\n";
         s << "  }\n";
     }
     s << "}\n";

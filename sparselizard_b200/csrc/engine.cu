@@ -1456,7 +1456,7 @@ static std::shared_ptr<Pattern> get_pattern(Ctx* ctx, Matrix& M, const std::vect
 
 // ------------------------------------------------------------ split precision (host side)
 
-// Tier 0: 7 slices, levels <= 8 (28 INT8 products; about 1e-12 relative per
+// Tier 0: 6 slices, levels <= 7 (21 INT8 products; about 1e-13 relative per
 // element matrix, well inside 1e-10); tier 1: 5 slices, levels <= 6 (15
 // products; about 1e-8, inside the FP32-level 1e-6).
 // Whether the split contraction of a group computes only the upper triangle
@@ -1512,8 +1512,8 @@ static GroupDev::Split& build_split(Ctx* ctx, GroupDev& g, int slot)
         return *sp;
     const int tier = slot & 1, form = slot >> 1;
     sp.reset(new GroupDev::Split());
-    sp->S = tier == 0 ? 7 : 5;
-    sp->L = tier == 0 ? 8 : 6;
+    sp->S = tier == 0 ? 6 : 5;
+    sp->L = tier == 0 ? 7 : 6;
     const int Q = g.nterms * g.ngp, P = g.ntf * g.ndof;
     sp->Qpad = std::max(kSplitKStep, (Q + kSplitKStep - 1) / kSplitKStep * kSplitKStep);
     sp->nrows = form == 1 ? g.ntf * (g.ntf + 1) / 2 : P;
@@ -1521,7 +1521,7 @@ static GroupDev::Split& build_split(Ctx* ctx, GroupDev& g, int slot)
     if (form != 0)
         upload(ctx, sp->rowmap, mirrored_rows(g.ntf, g.ndof, form == 1));
     sp->slices.alloc(ctx, (size_t)sp->S * g.norient * sp->Qpad * sp->Ppad);
-    sp->rowexp.alloc(ctx, (size_t)g.norient * sp->Ppad * 4);
+    sp->rowscale.alloc(ctx, (size_t)g.norient * sp->Ppad * 8);
     RowSliceParams rp{};
     rp.rowmap = sp->rowmap.empty() ? nullptr : sp->rowmap.as<int2>();
     rp.nrows = sp->nrows;
@@ -1534,14 +1534,18 @@ static GroupDev::Split& build_split(Ctx* ctx, GroupDev& g, int slot)
     rp.ntf = g.ntf;
     rp.ndof = g.ndof;
     rp.norient = g.norient;
-    rp.S = sp->S;
+    rp.L = sp->L;
     rp.Qpad = sp->Qpad;
     rp.Ppad = sp->Ppad;
     rp.slices = sp->slices.as<int8_t>();
-    rp.rowexp = sp->rowexp.as<int32_t>();
+    rp.rowscale = sp->rowscale.as<double>();
     if (g.norient > 65535)
         fail(SLGPU_E_UNSUPPORTED, "too many orientation variants");
-    k_slice_rows<<<dim3((unsigned)sp->Ppad, (unsigned)g.norient), 256, 0, ctx->x->stream>>>(rp);
+    const dim3 rgrid((unsigned)sp->Ppad, (unsigned)g.norient);
+    if (tier == 0)
+        k_slice_rows<8, 6><<<rgrid, 256, 0, ctx->x->stream>>>(rp);
+    else
+        k_slice_rows<7, 5><<<rgrid, 256, 0, ctx->x->stream>>>(rp);
     cuda_check(cudaGetLastError(), "k_slice_rows");
     ctx->launches++;
     return *sp;
@@ -1582,19 +1586,19 @@ static bool split_supported(const GroupDev& g)
     return Q > 0 && Q <= 16384;
 }
 
-template <int S, int L, int NE>
+template <int B, int S, int L, int NE>
 static void launch_split(Ctx* ctx, const SplitParams& p)
 {
     static bool attr = false;
     constexpr size_t smem = split_smem_bytes<NE>();
     if (!attr) {
-        cuda_check(cudaFuncSetAttribute(k_contract_split<S, L, NE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+        cuda_check(cudaFuncSetAttribute(k_contract_split<B, S, L, NE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                    "smem attribute");
         attr = true;
     }
     const int64_t grid = std::min<int64_t>(p.nwork, std::max(ctx->nsm, 1));
     cuda_check(cudaMemsetAsync(p.next, 0, sizeof(unsigned long long), ctx->x->stream), "memset");
-    k_contract_split<S, L, NE><<<(unsigned)grid, kSplitThreads, smem, ctx->x->stream>>>(p);
+    k_contract_split<B, S, L, NE><<<(unsigned)grid, kSplitThreads, smem, ctx->x->stream>>>(p);
 }
 
 // Element-tile width of the split kernel forced by SLGPU_SPLIT_TILE=32 or 64;
@@ -1611,14 +1615,14 @@ static int split_tile_forced()
 }
 
 // One split-precision contraction of a launch: group, tier, form and where
-// its coefficients, exponents and element matrices (and, for a transposed
+// its coefficients, their largest magnitudes and element matrices (and, for a transposed
 // pair, the partner's) are.
 struct SplitJob {
     GroupDev* g;
     int tier;
     bool paired;
     const double* C;
-    const int32_t* elemexp;
+    const int32_t* elemtop;
     double* out;
     double* out2;
     bool f32;  // out and out2 hold floats
@@ -1631,18 +1635,18 @@ static size_t split_col_bytes(const GroupDev& g, const GroupDev::Split& sp)
 {
     return ((size_t)sp.S * sp.Qpad * g.tiles.size() * 64 + 255) & ~size_t(255);
 }
-static size_t split_exp_bytes(const GroupDev& g) { return (g.tiles.size() * 64 * 4 + 255) & ~size_t(255); }
+static size_t split_scale_bytes(const GroupDev& g) { return (g.tiles.size() * 64 * 8 + 255) & ~size_t(255); }
 
-template <int S, int NE>
+template <int B, int S, int NE>
 static void launch_slices(Ctx* ctx, const ColSliceParams& cs)
 {
-    k_slice_cols<S, NE><<<grid_for(cs.ntiles * 64, 128), 128, 0, ctx->x->stream>>>(cs);
+    k_slice_cols<B, S, NE><<<grid_for(cs.ntiles * 64, 128), 128, 0, ctx->x->stream>>>(cs);
 }
 
 // Column slicing and the tcgen05 contraction of a set of jobs of one tier
 // with element-tile width NE: one slicing launch and one persistent
 // contraction launch per kSplitBatch jobs.  Every job's column slices and
-// exponents get their own block of the execution state's scratch.
+// scales get their own block of the execution state's scratch.
 static void run_split_jobs(Ctx* ctx, const std::vector<SplitJob>& jobs, int NE)
 {
     if (jobs.empty())
@@ -1652,40 +1656,38 @@ static void run_split_jobs(Ctx* ctx, const std::vector<SplitJob>& jobs, int NE)
     for (const SplitJob& j : jobs) {
         const GroupDev::Split& sp = ensure_split(ctx, *j.g, tier, j.paired);
         colb += split_col_bytes(*j.g, sp);
-        expb += split_exp_bytes(*j.g);
+        expb += split_scale_bytes(*j.g);
     }
     {
         ArenaPause keep(*ctx->x);  // per-state scratch, kept between requests
         if (ctx->x->split_cols.bytes() < colb)
             ctx->x->split_cols.alloc(ctx, colb);
-        if (ctx->x->split_colexp.bytes() < expb)
-            ctx->x->split_colexp.alloc(ctx, expb);
+        if (ctx->x->split_colscale.bytes() < expb)
+            ctx->x->split_colscale.alloc(ctx, expb);
     }
     int8_t* cols = ctx->x->split_cols.as<int8_t>();
-    int32_t* cexp = ctx->x->split_colexp.as<int32_t>();
+    double* cscale = ctx->x->split_colscale.as<double>();
     for (size_t b0 = 0; b0 < jobs.size(); b0 += kSplitBatch) {
         const size_t b1 = std::min(jobs.size(), b0 + kSplitBatch);
         ColSliceParams cs{};
         SplitParams sp{};
         double slice_bytes = 0, ops = 0;
-        int S = 0;
         for (size_t k = b0; k < b1; k++) {
             const SplitJob& j = jobs[k];
             const GroupDev& g = *j.g;
             const GroupDev::Split& s = *g.split[tier + 2 * (j.paired ? 2 : symmetric_form(g) ? 1 : 0)];
-            S = s.S;
             const int64_t ntiles = (int64_t)g.tiles.size();
             const int Q = g.nterms * g.ngp;
             ColSliceGroup& c = cs.g[cs.ngroups++];
             c.C = j.C;
-            c.elemexp = j.elemexp;
+            c.elemtop = j.elemtop;
             c.tiles = g.tiles_d.as<Tile>();
             c.Q = Q;
             c.Qpad = s.Qpad;
             c.nelem = g.nelem;
             c.ntiles = ntiles;
             c.slices = cols;
-            c.colexp = cexp;
+            c.colscale = cscale;
             c.t0 = cs.ntiles;
             cs.ntiles += ntiles;
             SplitGroup& G = sp.g[sp.ngroups++];
@@ -1699,48 +1701,46 @@ static void run_split_jobs(Ctx* ctx, const std::vector<SplitJob>& jobs, int NE)
             G.tiles = g.tiles_d.as<Tile>();
             G.A = s.slices.as<int8_t>();
             G.B = cols;
-            G.rowexp = s.rowexp.as<int32_t>();
-            G.colexp = cexp;
+            G.rowscale = s.rowscale.as<double>();
+            G.colscale = cscale;
             G.out = j.out;
             G.w0 = sp.nwork;
             G.nwork = (int64_t)G.ntp * ntiles * (64 / NE);
             sp.nwork += G.nwork;
             const size_t cb = split_col_bytes(g, s);
-            slice_bytes += 8.0 * Q * g.nelem + 4.0 * g.nelem + (double)cb + 4.0 * ntiles * 64;
+            slice_bytes += 8.0 * Q * g.nelem + 4.0 * g.nelem + (double)cb + 8.0 * ntiles * 64;
             // Algorithmic INT8 operations: 2 per product, pairs (a, b) with a + b <= L.
             int pairs = 0;
             for (int a = 1; a <= s.S; a++)
                 for (int bb = 1; bb <= s.S; bb++) pairs += (a + bb <= s.L);
             ops += 2.0 * pairs * s.nrows * Q * g.nelem;
             cols += cb;
-            cexp += split_exp_bytes(g) / 4;
+            cscale += split_scale_bytes(g) / 8;
         }
         sp.error = ctx->x->split_error.as<unsigned int>();
         sp.f32 = jobs[b0].f32 ? 1 : 0;
         sp.next = reinterpret_cast<unsigned long long*>(ctx->x->split_error.as<char>() + 16);
         const int kt = kstat_start(ctx, "slice_cols", slice_bytes);
-        if (S == 7 && NE == 64)
-            launch_slices<7, 64>(ctx, cs);
-        else if (S == 7)
-            launch_slices<7, 32>(ctx, cs);
-        else if (S == 5 && NE == 64)
-            launch_slices<5, 64>(ctx, cs);
-        else if (S == 5)
-            launch_slices<5, 32>(ctx, cs);
+        if (tier == 0 && NE == 64)
+            launch_slices<8, 6, 64>(ctx, cs);
+        else if (tier == 0)
+            launch_slices<8, 6, 32>(ctx, cs);
+        else if (NE == 64)
+            launch_slices<7, 5, 64>(ctx, cs);
         else
-            fail(SLGPU_E_UNSUPPORTED, "unsupported slice count");
+            launch_slices<7, 5, 32>(ctx, cs);
         kstat_stop(ctx, kt);
         cuda_check(cudaGetLastError(), "k_slice_cols");
         ctx->launches++;
-        const int kc = kstat_start(ctx, S == 7 ? "contract_split" : "contract_split_fp32", ops);
-        if (S == 7 && NE == 64)
-            launch_split<7, 8, 64>(ctx, sp);
-        else if (S == 7)
-            launch_split<7, 8, 32>(ctx, sp);
+        const int kc = kstat_start(ctx, tier == 0 ? "contract_split" : "contract_split_fp32", ops);
+        if (tier == 0 && NE == 64)
+            launch_split<8, 6, 7, 64>(ctx, sp);
+        else if (tier == 0)
+            launch_split<8, 6, 7, 32>(ctx, sp);
         else if (NE == 64)
-            launch_split<5, 6, 64>(ctx, sp);
+            launch_split<7, 5, 6, 64>(ctx, sp);
         else
-            launch_split<5, 6, 32>(ctx, sp);
+            launch_split<7, 5, 6, 32>(ctx, sp);
         kstat_stop(ctx, kc);
         cuda_check(cudaGetLastError(), "k_contract_split");
         ctx->launches++;
@@ -2041,7 +2041,7 @@ struct JitGroup {
     const double* fielddata;
     const double* term_scale;
     double* C;
-    int32_t* elemexp;  // nullptr, or per element: atomicMax of frexp exponents of |C|
+    int32_t* elemtop;  // nullptr, or per element: atomicMax of the high words of |C|
 };
 
 // Geometry + coefficients of every group into C (offsets coff).  Consecutive
@@ -2052,7 +2052,7 @@ struct JitGroup {
 // each) are one by-value kernel parameter.
 constexpr int kJitBatch = 64;
 
-static void launch_coefficients(Ctx* ctx, const Matrix& M, double* C, const std::vector<int64_t>& coff, int32_t* elemexp,
+static void launch_coefficients(Ctx* ctx, const Matrix& M, double* C, const std::vector<int64_t>& coff, int32_t* elemtop,
                                 const std::vector<int64_t>& eoff, const std::vector<GroupData>* ov, const std::vector<int>& pair)
 {
     // The second group of a transposed pair needs no coefficients.
@@ -2097,7 +2097,7 @@ static void launch_coefficients(Ctx* ctx, const Matrix& M, double* C, const std:
                     const double* fd = ov != nullptr && (*ov)[j].fielddata != nullptr ? (*ov)[j].fielddata : G.fielddata.as<double>();
                     const double* ts = ov != nullptr && (*ov)[j].term_scale != nullptr ? (*ov)[j].term_scale : G.term_scale_d.as<double>();
                     jg.push_back(JitGroup{G.tables.as<double>(), ed, fd, ts, skip(j) ? nullptr : C + coff[j],
-                                          eoff[j] >= 0 && !skip(j) ? elemexp + eoff[j] : nullptr});
+                                          eoff[j] >= 0 && !skip(j) ? elemtop + eoff[j] : nullptr});
                 }
                 const MeshDev& m = ctx->meshes.at(g0.mesh);
                 JitGeom geom{m.xyz.as<double>(), m.types.at(g0.elemtype).conn.as<int32_t>(), g0.elems.as<int32_t>(), g0.orient.as<int32_t>(),
@@ -2127,7 +2127,7 @@ static void launch_coefficients(Ctx* ctx, const Matrix& M, double* C, const std:
                     continue;
                 GroupDev& G = *M.groups[j];
                 CoefParams cp = coef_params(ctx, G, C + coff[j]);
-                cp.elemexp = eoff[j] >= 0 ? elemexp + eoff[j] : nullptr;
+                cp.elemtop = eoff[j] >= 0 ? elemtop + eoff[j] : nullptr;
                 if (ov != nullptr && (*ov)[j].elemdata != nullptr)
                     cp.elemdata = (*ov)[j].elemdata;
                 if (ov != nullptr && (*ov)[j].fielddata != nullptr)
@@ -2184,8 +2184,8 @@ void launch_contractions(Ctx* ctx, const Matrix& M, int precision, const std::ve
         cuda_check(cudaEventCreate(&e), "cudaEventCreate");
         ctx->x->evpool.push_back(e);
     }
-    // Split-precision groups: per-element exponents of the coefficients,
-    // gathered by the coefficient kernels (atomicMax from a very negative start).
+    // Split-precision groups: the high word of each element's largest
+    // coefficient, gathered by the coefficient kernels (atomicMax from 0).
     std::vector<int64_t> eoff(M.groups.size(), -1);
     int64_t etot = 0;
     for (size_t k = 0; k < M.groups.size(); k++)
@@ -2196,7 +2196,7 @@ void launch_contractions(Ctx* ctx, const Matrix& M, int precision, const std::ve
     DevBuf E;
     if (etot > 0) {
         E.alloc(ctx, (size_t)etot * 4);
-        cuda_check(cudaMemsetAsync(E.as<void>(), 0x80, (size_t)etot * 4, ctx->x->stream), "memset");
+        cuda_check(cudaMemsetAsync(E.as<void>(), 0, (size_t)etot * 4, ctx->x->stream), "memset");
     }
     const std::vector<int> pair = cross_pairs(M, precision, ov);
     phase_event(ctx, ctx->x->evpool[0]);
@@ -2519,14 +2519,14 @@ void prepare_value_path(Ctx* ctx, const Matrix& M, int precision)
                 ensure_split(ctx, *g, tier, true);
             // The groups of a step are sliced and contracted together.
             colbytes += split_col_bytes(*g, sp);
-            expbytes += split_exp_bytes(*g);
+            expbytes += split_scale_bytes(*g);
         }
     }
     Exec& x = *ctx->x;
     if (x.split_cols.bytes() < colbytes)
         x.split_cols.alloc(ctx, colbytes);
-    if (x.split_colexp.bytes() < expbytes)
-        x.split_colexp.alloc(ctx, expbytes);
+    if (x.split_colscale.bytes() < expbytes)
+        x.split_colscale.alloc(ctx, expbytes);
     if (x.split_error.empty())
         x.split_error.alloc(ctx, 32);
 }
@@ -2567,7 +2567,7 @@ static std::vector<uint64_t> value_signature(Ctx* ctx, const Matrix& M, int prec
     u(ctx->timers ? 1 : 0);
     u(ctx->jit_broken ? 1 : 0);
     p(x.split_cols.as<void>());
-    p(x.split_colexp.as<void>());
+    p(x.split_colscale.as<void>());
     p(x.split_error.as<void>());
     const std::vector<int> pair = cross_pairs(M, precision, nullptr);
     size_t gi = 0;
@@ -2585,7 +2585,7 @@ static std::vector<uint64_t> value_signature(Ctx* ctx, const Matrix& M, int prec
         }
         for (int t = 0; t < 6; t++) {
             p(g.split[t] ? g.split[t]->slices.as<void>() : nullptr);
-            p(g.split[t] ? g.split[t]->rowexp.as<void>() : nullptr);
+            p(g.split[t] ? g.split[t]->rowscale.as<void>() : nullptr);
         }
         for (int t = 0; t < 3; t++) p(g.fmt[t] ? g.fmt[t]->Mt.as<void>() : nullptr);
         auto mi = ctx->meshes.find(g.mesh);
@@ -2920,7 +2920,7 @@ void slgpu_ctx_destroy(slgpu_ctx* ctx)
     // Every device buffer the context owns is freed on its stream, so all of
     // them must go before the stream does.
     ctx->x->split_cols.release();
-    ctx->x->split_colexp.release();
+    ctx->x->split_colscale.release();
     ctx->x->split_error.release();
     ctx->rhs_record.clear();
     for (cudaLibrary_t lib : ctx->jit_libs) cudaLibraryUnload(lib);

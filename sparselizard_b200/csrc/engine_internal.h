@@ -136,7 +136,7 @@ struct GroupDev {
     // slot tier + 2 form.
     struct Split {
         int S = 0, L = 0, Qpad = 0, Ppad = 0, nrows = 0;
-        DevBuf slices, rowexp, rowmap;
+        DevBuf slices, rowscale, rowmap;
     };
     std::unique_ptr<Split> split[6];
     // FP64 tensor-core operand M^T per form (0 every entry, 1 upper triangle
@@ -267,7 +267,7 @@ struct Exec {
     std::vector<cudaEvent_t> kev;                          // start/stop pairs
     std::vector<std::pair<std::string, double>> kev_tag;   // family, work of each pair
     std::map<std::string, KernelStat> kstats;
-    DevBuf split_cols, split_colexp;   // split precision: column slices of the current group
+    DevBuf split_cols, split_colscale;   // split precision: column slices of the current group
     DevBuf split_error;                // bytes 0-15: flags set by a timed-out wait; 16-23: split work counter
     // Page-locked staging for the small uploads of one call (kernel argument
     // arrays), so that they never wait for the stream: reset at the start of

@@ -63,7 +63,7 @@ struct CoefParams {
     const double* term_scale;
     int nterms;
     double* C;  // [nterms][ngp][nelem]
-    int32_t* elemexp;  // nullptr, or [nelem]: atomicMax of the frexp exponents of |C|
+    int32_t* elemtop;  // nullptr, or [nelem]: atomicMax of the high words of |C| (as integers; NaN above infinity)
     int64_t nnodes;    // > 0: node numbers outside [0, nnodes) are not read and give NaN coefficients
 };
 
@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(128) k_geometry_coef(CoefParams p)
         inv[2][2] = (J[0][0] * J[1][1] - J[0][1] * J[1][0]) / det;
     }
     const double wdet = p.weights[g] * fabs(det);
-    double cmax = 0;
+    int top = 0;
 
     double s[kMaxSlots];
     for (int k = 0; k < p.nprog; k++) {
@@ -205,17 +205,14 @@ __global__ void __launch_bounds__(128) k_geometry_coef(CoefParams p)
         case INSTR_STORE: {
             const double c = bad_node ? __longlong_as_double(0x7ff8000000000000ll) : s[in.a] * p.term_scale[in.b] * wdet;
             p.C[((int64_t)in.b * p.ngp + g) * p.nelem + e] = c;
-            cmax = fmax(cmax, fabs(c));
+            top = max(top, __double2hiint(c) & 0x7fffffff);
             continue;
         }
         }
         s[in.dst] = v;
     }
-    if (p.elemexp != nullptr && cmax > 0) {
-        int ex;
-        frexp(cmax, &ex);
-        atomicMax(p.elemexp + e, ex);
-    }
+    if (p.elemtop != nullptr && top > 0)
+        atomicMax(p.elemtop + e, top);
 }
 
 struct ContractParams {

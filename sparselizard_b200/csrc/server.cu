@@ -832,7 +832,7 @@ void slgpu_server_destroy(slgpu_server* S)
             cudaStreamSynchronize(s.ex.stream);
         // Slot buffers go before their stream.
         s.ex.split_cols.release();
-        s.ex.split_colexp.release();
+        s.ex.split_colscale.release();
         s.ex.split_error.release();
         s.ex.arena.release();
         if (s.ex.stream != nullptr)

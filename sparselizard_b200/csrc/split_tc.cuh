@@ -1,21 +1,34 @@
 // Split-precision element contraction on the sm_100a tensor cores.
 //
 // V[e][p] = sum_q M[p][q] C[q][e] is evaluated with FP64 operands cut into
-// 7-bit integer slices (Ozaki scheme):
-//   M[p][q] = 2^E_p   sum_a m_a[p][q] 2^-7a      (row exponent E_p, a = 1..S)
-//   C[q][e] = 2^F_e   sum_b c_b[q][e] 2^-7b      (column exponent F_e)
-//   V[e][p] ~ 2^(E_p+F_e) sum_{a+b <= L} 2^-7(a+b) sum_q m_a c_b
+// INT8 slices of B bits (Ozaki scheme):
+//   M[p][q] = R_p sum_a m_a[p][q] 2^-Ba      (row scale R_p, a = 1..S)
+//   C[q][e] = Q_e sum_b c_b[q][e] 2^-Bb      (column scale Q_e)
+//   V[e][p] ~ R_p Q_e sum_{a+b <= L} 2^-B(a+b) sum_q m_a c_b
 // Each sum_q m_a c_b is an INT8 x INT8 product summed exactly in INT32 by
 // tcgen05.mma (kind::i8); all pairs with the same level l = a+b accumulate
 // in the same TMEM accumulator (still exact: at most S products of
-// |m c| <= 127^2 per q).  The epilogue recombines the levels.
+// |m c| <= 2^14 per q, q <= 2^14).  The epilogue recombines the levels.
+//
+// Split tier: B = 8, the balanced base-256 digits -128 .. 127 of the operand
+// rounded to an integer, S = 6, L = 7 (21 products).  FP32-level tier: B = 7,
+// the operand truncated to signed 7-bit fields, scales the power of two above
+// the largest magnitude, S = 5, L = 6 (15 products).
+// A balanced digit carries a bit more than a truncated one, rounding has half
+// the error of truncation, and the scale uses the largest value itself (to
+// 2^-20): six balanced digits err 4 to 8 times less than seven truncated ones
+// with L = 8, for 21 products instead of 28.  (Relative Frobenius error of
+// the element matrices, order-2 elasticity on hexahedra / on tetrahedra /
+// order-5 Helmholtz: 6.1e-14 / 1.8e-14 / 2.9e-14 against 5.0e-13 / 6.6e-14 /
+// 2.1e-13.)  A step of mixed orders 1-5 on 48,000 tetrahedra, whose contraction
+// the products bound: 1725 -> 1451 us.
 //
 // Level accumulators sit side by side in TMEM (level l at columns
 // NE(l-2) .. NE(l-2)+NE-1 for an element tile of NE columns), and the column
 // slices of one K step sit side by side in shared memory, so A slice a times
 // the concatenation [c_1 | ... | c_k] (N = NE k <= 256) writes every pair
-// (a, b) straight into level a+b's columns: for S = 7, 10 MMAs per K step
-// (NE = 64) or 7 (NE = 32) instead of 28.
+// (a, b) straight into level a+b's columns: for S = 6, 8 MMAs per K step
+// (NE = 64) or 6 (NE = 32) instead of 21.
 //
 // Operands live in global memory already in the interleaved K-major layout
 // that the UMMA "no swizzle" canonical form expects, blocked so that one K
@@ -34,21 +47,21 @@ namespace slgpu {
 
 constexpr int kSplitM = 128;     // element-matrix entries per tile (TMEM lanes)
 constexpr int kSplitKStep = 32;  // bytes of K per pipeline stage (one MMA K)
-constexpr int kSplitMaxS = 7;    // slices per operand (levels 2..8)
+constexpr int kSplitMaxS = 6;    // most slices per operand
 constexpr int kSplitEpiWarps = 16;  // 4 per TMEM lane quarter, 16 columns each
 constexpr int kSplitThreads = 64 + 32 * kSplitEpiWarps;
 constexpr int kSplitABytes = 2 * kSplitM * 16;  // one slice of one K step of A
 
 // Element-tile width NE (columns of one accumulator level) and what follows
-// from it.  NE = 64: one accumulator (7 levels x 64 = 448 TMEM columns), the
+// from it.  NE = 64: one accumulator (6 levels x 64 = 384 TMEM columns), the
 // epilogue of a tile runs between its MMAs and the next tile's.  NE = 32: two
-// accumulators (2 x 224 columns), the epilogue of one tile overlaps the MMAs
+// accumulators (2 x 192 columns), the epilogue of one tile overlaps the MMAs
 // of the next; A (the rows of M) is read twice as often per element.
 template <int NE>
 struct SplitShape {
     static constexpr int kUnits = 64 / NE;               // element tiles per 64-element tile
     static constexpr int kBufs = NE == 32 ? 2 : 1;       // TMEM accumulators
-    static constexpr int kStages = NE == 32 ? 6 : 4;     // shared-memory pipeline depth
+    static constexpr int kStages = NE == 32 ? 7 : 6;     // shared-memory pipeline depth
     static constexpr int kBBytes = 2 * NE * 16;          // one slice of one K step of B
     static constexpr int kGroup = 256 / NE;              // B slices per MMA (N <= 256)
 };
@@ -65,8 +78,8 @@ struct SplitGroup {
     const Tile* tiles;      // 64-element tiles; unit u = tile u / kUnits, part u % kUnits
     const int8_t* A;        // row slices
     const int8_t* B;        // column slices
-    const int32_t* rowexp;  // [norient][Ppad]
-    const int32_t* colexp;  // [ntiles][64]: exponent of each slot
+    const double* rowscale;  // [norient][Ppad]: R_p 2^-(B L)
+    const double* colscale;  // [ntiles][64]: Q_e of each slot
     double* out;            // [nelem][P]
     int64_t w0, nwork;
 };
@@ -118,10 +131,73 @@ struct RowSliceParams {
     const int32_t* term_tf;
     const int32_t* term_dof;
     const int2* rowmap;
-    int nterms, ngp, ntf, ndof, norient, S, Qpad, Ppad, nrows;
+    int nterms, ngp, ntf, ndof, norient, Qpad, Ppad, nrows;
+    int L;            // largest level
     int8_t* slices;   // [orient][ptile][kstep][S][2][128][16]
-    int32_t* rowexp;  // [norient][Ppad]
+    double* rowscale; // [norient][Ppad]
 };
+
+// Scale of a row or column from the high word h of the largest magnitude in
+// it: *q, the value that 2^(B S) units stand for (R and Q above), and the
+// factor that turns a value into those units.
+//   B = 8: |x| < the double of high word h + 1, so |x| / Q < 0.498 and its S
+//   balanced digits represent it (the largest such number is 0.49804);
+//   B = 7: the power of two above |x|.
+// Magnitudes below 2^-900 take a power of two and a factor below the
+// overflow: *pre, by which values are multiplied first (1 otherwise).
+// Nothing set (h = 0): digits and scale are zero.  Infinities and NaN (h from
+// 0x7ff00000): the scale is NaN, so that the results are.
+template <int B, int S>
+__device__ __forceinline__ double split_scale(int h, double* q, double* pre)
+{
+    const double unit = __longlong_as_double((long long)(1023 + B * S) << 52);  // 2^(B S)
+    *pre = 1.0;
+    if (h <= 0) {
+        *q = 0.0;
+        return 0.0;
+    }
+    if (h >= 0x7ff00000) {
+        *q = __longlong_as_double(0x7ff8000000000000ll);
+        return 0.0;
+    }
+    const bool tiny = h < (1023 - 900) << 20;
+    if (tiny || B == 7) {
+        int ex;
+        frexp(__hiloint2double(h, -1), &ex);  // |x| < 2^ex
+        ex += B == 7 ? 0 : 2;
+        *q = ldexp(1.0, ex);
+        *pre = tiny ? 0x1p512 : 1.0;
+        return ldexp(unit, -ex - (tiny ? 512 : 0));
+    }
+    const double top = h >= 0x7fefffff ? __longlong_as_double(0x7fefffffffffffffll) : __hiloint2double(h + 1, 0);
+    *q = top * (1.0 / 0.498);
+    return 0.498 * unit / top;
+}
+
+// The S digits of x in units of 1 / f, byte k the digit S - 1 - k.
+// B = 8, each plus 128: 1.5 2^52 + rint(x f) holds the integer in its low
+// bits, and adding 128 to every digit makes them all non-negative.
+// B = 7, two's complement: the 7-bit fields of |x| f truncated, with x's sign.
+template <int B, int S>
+__device__ __forceinline__ unsigned long long split_digits(double x, double f)
+{
+    if constexpr (B == 8) {
+        constexpr unsigned long long kBias = 0x8080808080808080ull >> (8 * (8 - S));
+        return (unsigned long long)__double_as_longlong(fma(x, f, 0x1.8p52)) + kBias;
+    } else {
+        const unsigned long long mag = __double2ull_rz(fabs(x) * f);
+        unsigned long long u = 0;
+#pragma unroll
+        for (int k = 0; k < S; k++) {
+            const int d = (int)((mag >> (7 * k)) & 127);
+            u |= (unsigned long long)(uint8_t)(int8_t)(x < 0 ? -d : d) << (8 * k);
+        }
+        return u;
+    }
+}
+// What turns a byte of split_digits into the signed digit.
+template <int B>
+__host__ __device__ constexpr uint32_t split_flip() { return B == 8 ? 0x80808080u : 0u; }
 
 // M[pe][q] (pe < 0: zero).
 __device__ __forceinline__ double m_entry(const RowSliceParams& p, int o, int pe, int q)
@@ -137,61 +213,49 @@ __device__ __forceinline__ double m_entry(const RowSliceParams& p, int o, int pe
     return tv * dv;
 }
 
-// Splits x (|x| < 1 after scaling) into S signed 7-bit integers by repeated
-// truncation; every step is exact in FP64.
-__device__ __forceinline__ void split7(double x, int S, int8_t* out)
-{
-    for (int s = 0; s < S; s++) {
-        const double y = x * 128.0;
-        const double m = trunc(y);
-        out[s] = (int8_t)m;
-        x = y - m;
-    }
-}
-
+template <int B, int S>
 __global__ void k_slice_rows(RowSliceParams p)
 {
     const int pe = blockIdx.x, o = blockIdx.y;
     const int src = pe >= p.nrows ? -1 : p.rowmap != nullptr ? p.rowmap[pe].x : pe;
-    __shared__ double red[256];
-    double mx = 0;
-    for (int q = threadIdx.x; q < p.Qpad; q += blockDim.x) mx = fmax(mx, fabs(m_entry(p, o, src, q)));
-    red[threadIdx.x] = mx;
-    __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s)
-            red[threadIdx.x] = fmax(red[threadIdx.x], red[threadIdx.x + s]);
-        __syncthreads();
-    }
-    int ex = 0;
-    if (red[0] > 0)
-        frexp(red[0], &ex);  // red[0] = f * 2^ex, f in [0.5, 1)
+    __shared__ int top;
     if (threadIdx.x == 0)
-        p.rowexp[(int64_t)o * p.Ppad + pe] = ex;
+        top = 0;
+    __syncthreads();
+    // Magnitudes compare as their bit patterns (NaN above infinity).
+    int mx = 0;
+    for (int q = threadIdx.x; q < p.Qpad; q += blockDim.x) mx = max(mx, __double2hiint(m_entry(p, o, src, q)) & 0x7fffffff);
+    atomicMax(&top, mx);
+    __syncthreads();
+    double unit, pre;
+    const double f = split_scale<B, S>(top, &unit, &pre);
+    if (threadIdx.x == 0)
+        p.rowscale[(int64_t)o * p.Ppad + pe] = ldexp(unit, -B * p.L);
     const int ntp = p.Ppad / kSplitM, nk = p.Qpad / kSplitKStep;
     const int pt = pe / kSplitM, r = pe % kSplitM;
     for (int q = threadIdx.x; q < p.Qpad; q += blockDim.x) {
-        int8_t sl[kSplitMaxS];
-        split7(ldexp(m_entry(p, o, src, q), -ex), p.S, sl);
+        const unsigned long long u = split_digits<B, S>(m_entry(p, o, src, q) * pre, f);
         const int ks = q / kSplitKStep, c = (q / 16) & 1;
-        for (int s = 0; s < p.S; s++)
-            p.slices[(((((int64_t)o * ntp + pt) * nk + ks) * p.S + s) * 2 + c) * (kSplitM * 16) + r * 16 + (q & 15)] = sl[s];
+        for (int s = 0; s < S; s++)
+            p.slices[(((((int64_t)o * ntp + pt) * nk + ks) * S + s) * 2 + c) * (kSplitM * 16) + r * 16 + (q & 15)] =
+                (int8_t)((u >> (8 * (S - 1 - s))) ^ split_flip<B>());
     }
 }
 
 // Column slices of C: thread per (64-element tile, slot); C[q][e] is read
 // once, coalesced over the tile's consecutive elements, and 16-byte chunks
-// are written coalesced over slots.  The exponent of each element (largest
-// |C[q][e]| = f 2^ex, f in [0.5, 1)) comes from the coefficient kernel.
-// Empty slots get zero slices.
+// are written coalesced over slots.  The high word of each element's largest
+// |C[q][e]| comes from the coefficient kernel.  Empty slots get zero slices.
+// About 8 instructions per coefficient (one fma, the bias, byte permutes):
+// HBM-bound.
 struct ColSliceGroup {
     const double* C;  // [Q][nelem]
-    const int32_t* elemexp;  // [nelem]; below -1100: the column is zero
+    const int32_t* elemtop;  // [nelem]; 0: the column is zero
     const Tile* tiles;
     int Q, Qpad;
     int64_t nelem, ntiles;
     int8_t* slices;   // [unit][kstep][2][S][NE][16]
-    int32_t* colexp;  // [ntiles][64]
+    double* colscale; // [ntiles][64]
     int64_t t0;       // first tile of the group in the launch
 };
 
@@ -201,7 +265,22 @@ struct ColSliceParams {
     int64_t ntiles;   // sum over the groups
 };
 
-template <int S, int NE>
+// Word k4 of each slice: digit s of four values as signed bytes.
+template <int B, int S>
+__device__ __forceinline__ void split_words(const unsigned long long (&u)[4], uint32_t (&w)[S][4], int k4)
+{
+#pragma unroll
+    for (int s = 0; s < S; s++) {
+        const int b = S - 1 - s;  // byte of the digit
+        const uint32_t sel = (uint32_t)((b & 3) | ((b & 3) + 4) << 4);
+        uint32_t v[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) v[k] = b < 4 ? (uint32_t)u[k] : (uint32_t)(u[k] >> 32);
+        w[s][k4] = __byte_perm(__byte_perm(v[0], v[1], sel), __byte_perm(v[2], v[3], sel), 0x5410) ^ split_flip<B>();
+    }
+}
+
+template <int B, int S, int NE>
 __global__ void k_slice_cols(const __grid_constant__ ColSliceParams pb)
 {
     const int64_t gt = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -216,18 +295,13 @@ __global__ void k_slice_cols(const __grid_constant__ ColSliceParams pb)
     const Tile tile = p.tiles[t];
     const bool valid = slot < tile.ne;
     const int64_t e = tile.e0 + slot;
-    int ex = valid ? p.elemexp[e] : 0;
-    if (ex < -1100)
-        ex = 0;
-    p.colexp[t * 64 + slot] = ex;
+    double unit, pre;
+    const double f = split_scale<B, S>(valid ? p.elemtop[e] : 0, &unit, &pre);
+    p.colscale[t * 64 + slot] = unit;
     const int nchunk = p.Qpad / 16;
-    const int64_t unit = t * SplitShape<NE>::kUnits + slot / NE;
-    uint4* out = reinterpret_cast<uint4*>(p.slices) + unit * (int64_t)nchunk * S * NE + slot % NE;
+    const int64_t u0 = t * SplitShape<NE>::kUnits + slot / NE;
+    uint4* out = reinterpret_cast<uint4*>(p.slices) + u0 * (int64_t)nchunk * S * NE + slot % NE;
     const double* col = p.C + e;
-    // |C| 2^(7S - ex) < 2^(7S): its integer part holds the S 7-bit slices
-    // (the same digits repeated truncation of C 2^-ex by 128 produces).
-    const bool fast = 7 * S - ex <= 1023;
-    const double scale = fast ? __longlong_as_double((long long)(7 * S - ex + 1023) << 52) : 0.0;
     for (int c = 0; c < nchunk; c++) {
         double x[16];
 #pragma unroll
@@ -237,19 +311,11 @@ __global__ void k_slice_cols(const __grid_constant__ ColSliceParams pb)
         }
         uint32_t w[S][4];
 #pragma unroll
-        for (int s = 0; s < S; s++)
+        for (int k4 = 0; k4 < 4; k4++) {
+            unsigned long long u[4];
 #pragma unroll
-            for (int k = 0; k < 4; k++) w[s][k] = 0;
-#pragma unroll
-        for (int k = 0; k < 16; k++) {
-            const double ax = fast ? fabs(x[k]) * scale : ldexp(fabs(x[k]), 7 * S - ex);
-            const unsigned long long mag = __double2ull_rz(ax);
-            const bool neg = x[k] < 0;
-#pragma unroll
-            for (int s = 0; s < S; s++) {
-                const int d = (int)((mag >> (7 * (S - 1 - s))) & 127);
-                w[s][k >> 2] |= (uint32_t)(uint8_t)(int8_t)(neg ? -d : d) << (8 * (k & 3));
-            }
+            for (int k = 0; k < 4; k++) u[k] = split_digits<B, S>(pre == 1.0 ? x[4 * k4 + k] : x[4 * k4 + k] * pre, f);
+            split_words<B, S>(u, w, k4);
         }
         // chunk c of K step c/2 lands at [kstep][c&1][s][slot]: (c*S + s) * NE.
 #pragma unroll
@@ -352,21 +418,13 @@ __device__ __forceinline__ void tmem_ld16_nowait(uint32_t taddr, int32_t* r)
 
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-// 2^s as a double for a normal exponent, else ldexp (exact either way).
-__device__ __forceinline__ double scale2(double x, int s)
-{
-    if (s >= -1022 && s <= 1023)
-        return x * __longlong_as_double((long long)(s + 1023) << 52);
-    return ldexp(x, s);
-}
-
 // Exact int64 -> double for |x| < 2^51 on the integer and FP64 pipes instead
 // of the conversion unit (which the epilogue's two conversions per output
 // saturate): x is added to the bit pattern of 1.5 * 2^52, whose mantissa ulp
 // is 1, so the pattern encodes 1.5 * 2^52 + x exactly; subtracting 1.5 * 2^52
 // is exact (both operands lie in [2^52, 2^53)).  The level sums meet the
-// bound: level l holds at most l - 1 pair products of at most K * 127^2
-// each, with K <= 16384, so |H| < 5.7e14 < 2^51 and |Lo| is smaller still.
+// bound: a level holds at most 6 pair products of at most K * 2^14 each, with
+// K <= 16384, so |r| < 2^30.6 and three levels combined stay below 2^47.
 __device__ __forceinline__ double i64_to_f64_exact(long long x)
 {
     return __longlong_as_double(0x4338000000000000LL + x) - 0x1.8p52;
@@ -411,12 +469,13 @@ constexpr size_t split_smem_bytes() { return sizeof(SplitSmem<NE>) + 1024; }
 // accumulator b -> MMAs of the next tile using it).  Every wait is bounded: on
 // timeout the CTA records the failure, the roles stop, outstanding copies and
 // MMAs are waited for (bounded), the TMEM is freed and the CTA returns.
-template <int S, int L, int NE>
+template <int B, int S, int L, int NE>
 __global__ void __launch_bounds__(kSplitThreads, 1) k_contract_split(const __grid_constant__ SplitParams p)
 {
-    static_assert(S <= kSplitMaxS && L - 1 <= S && L >= 6 && L <= 8, "level layout");
+    constexpr int NL = L - 1;  // levels 2 .. L
+    static_assert(S <= kSplitMaxS && NL <= S && NL >= 5 && NL <= 6, "level layout");
     using Sh = SplitShape<NE>;
-    static_assert(Sh::kBufs == 1 ? (L - 1) * NE <= 512 : (L - 1) * NE <= 256, "accumulators fit the 512 TMEM columns");
+    static_assert(Sh::kBufs == 1 ? NL * NE <= 512 : NL * NE <= 256, "accumulators fit the 512 TMEM columns");
     constexpr int kSt = Sh::kStages;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     SplitSmem<NE>& sm = *reinterpret_cast<SplitSmem<NE>*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -585,8 +644,8 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_contract_split(const __gri
     } else if (warp >= 2) {
         // ------------------------------------------------ epilogue
         // Warp w reads TMEM lane quarter w % 4 and columns c0 .. c0+15 of
-        // each level.  Only levels 2..5 (combined into H) and then 6..L are
-        // held in registers before the accumulator is released; the rest of
+        // each level.  The first levels are combined into H before the last
+        // three are loaded; then the accumulator is released, and the rest of
         // the recombination and the stores overlap the next tile's MMAs.
         const int quarter = warp & 3;
         const int c0 = ((warp - 2) >> 2) * 16;
@@ -620,46 +679,40 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_contract_split(const __gri
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t col = lane_base + (uint32_t)(buf * 256 + c0);
-            // V = 2^-35 (H + 2^-21 Lo): H = sum_{l<=5} r_l 2^(7(5-l)),
-            // Lo = sum_{l>=6} r_l 2^(7(8-l)); both exact in int64.
+            // V = R_p Q_e 2^-(B L) (H 2^3B + Lo): Lo the last three levels, H
+            // the others, each r_l times 2^B per level; both exact in int64.
             long long H[16];
             {
-                int32_t r[4][16];
+                int32_t r[NL - 3][16];
 #pragma unroll
-                for (int l = 0; l < 4; l++) tmem_ld16_nowait(col + (uint32_t)(l * NE), r[l]);
-                tmem_ld_wait();
-#pragma unroll
-                for (int j = 0; j < 16; j++)
-                    H[j] = (((long long)r[0][j] * 128 + r[1][j]) * 128 + r[2][j]) * 128 + r[3][j];
-            }
-            // Levels 6..L give Lo; the recombined value (exact up to the one
-            // rounding of the fma) is formed before the stores' addresses are
-            // live, so the store loop holds 16 doubles instead of the level
-            // sums.
-            double d[16];
-            {
-                int32_t t[L - 5][16];
-#pragma unroll
-                for (int l = 0; l < L - 5; l++) tmem_ld16_nowait(col + (uint32_t)((4 + l) * NE), t[l]);
+                for (int l = 0; l < NL - 3; l++) tmem_ld16_nowait(col + (uint32_t)(l * NE), r[l]);
                 tmem_ld_wait();
 #pragma unroll
                 for (int j = 0; j < 16; j++) {
-                    long long lo = 0;
+                    H[j] = r[0][j];
 #pragma unroll
-                    for (int l = 0; l < L - 5; l++) lo = lo * 128 + t[l][j];
-                    lo <<= 7 * (8 - L);
-                    d[j] = fma(i64_to_f64_exact(lo), 0x1p-21, i64_to_f64_exact(H[j]));
+                    for (int l = 1; l < NL - 3; l++) H[j] = H[j] * (1 << B) + r[l][j];
                 }
             }
+            int32_t t[3][16];
+#pragma unroll
+            for (int l = 0; l < 3; l++) tmem_ld16_nowait(col + (uint32_t)((NL - 3 + l) * NE), t[l]);
+            tmem_ld_wait();
             // This warp's accumulators are in registers: release them.
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0)
                 mbar_arrive(&sm.tmem_empty[buf]);
+            double d[16];
+#pragma unroll
+            for (int j = 0; j < 16; j++) {
+                const long long lo = ((long long)t[0][j] * (1 << B) + t[1][j]) * (1 << B) + t[2][j];
+                d[j] = fma(i64_to_f64_exact(H[j]), (double)(1 << 3 * B), i64_to_f64_exact(lo));
+            }
             const int pe = pt * kSplitM + quarter * 32 + lane;
             if (pe < G.nrows) {
-                const int rex = G.rowexp[(int64_t)unit.orient * G.Ppad + pe] - 35;
-                const int32_t* ce = G.colexp + u * NE + c0;
+                const double rsc = G.rowscale[(int64_t)unit.orient * G.Ppad + pe];
+                const double* ce = G.colscale + u * NE + c0;
                 // Row pe is entry m.x and, for a symmetric group, also its
                 // mirror m.y (the same entry on the diagonal); with a
                 // transposed partner, entry (i, j) is also the partner's
@@ -671,13 +724,13 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_contract_split(const __gri
                 double* outm = G.out2 != nullptr ? G.out2 + ebase + m.y : m.y != m.x ? G.out + ebase + m.y : nullptr;
                 const int nj = min(16, unit.ne - c0);
 #pragma unroll
-                for (int j = 0; j < 16; j += 4) {
-                    const int4 c4 = *reinterpret_cast<const int4*>(ce + j);
-                    const int cx[4] = {c4.x, c4.y, c4.z, c4.w};
+                for (int j = 0; j < 16; j += 2) {
+                    const double2 c2 = *reinterpret_cast<const double2*>(ce + j);
+                    const double cx[2] = {c2.x, c2.y};
 #pragma unroll
-                    for (int jj = 0; jj < 4; jj++) {
+                    for (int jj = 0; jj < 2; jj++) {
                         if (j + jj < nj) {
-                            const double v = scale2(d[j + jj], rex + cx[jj]);
+                            const double v = d[j + jj] * rsc * cx[jj];
                             if (p.f32) {
                                 // Entry k of a float matrix is float k of the same buffer.
                                 const int64_t o = (int64_t)(j + jj) * P;

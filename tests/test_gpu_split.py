@@ -209,3 +209,28 @@ def test_split_dropin_elasticity(ref_lib, gpu_lib, tmp_path):
     P.check_pattern(ref, got)
     _, _, fro = P.scaled_errors(ref, got)
     assert fro <= 1e-10, f"assembled Frobenius-relative error {fro:.3e}"
+
+
+@pytest.mark.parametrize("factor", [1e-290, 1e-180, 1.0, 1e200])
+def test_split_scales(ctx, factor):
+    """Columns of extreme magnitudes (the scales' branches), a zero column,
+    and columns that are not finite, which reach their own element only."""
+    rng = np.random.Generator(np.random.PCG64(10))
+    gb, xyz, conn = S.group(rng, nelem_grid=13, ntf=9, ndof=9, nterms=3, ngp1=3, norient=2, ndests=1)
+    g = gb.g
+    for t in range(g.nterms):
+        g.terms[t].coef_node = 5  # the per-element coefficient alone
+    e = np.ctypeslib.as_array(g.elemdata[0], (g.nelem,))
+    e *= factor * np.where(np.arange(g.nelem) % 3 == 0, 1e-6, 1.0)
+    e[7], e[20], e[33] = 0.0, np.inf, np.nan
+    ref = _element_matrices(ctx, gb, xyz, conn, abi.PREC_FP64)
+    fine = np.ones(g.nelem, bool)
+    fine[[20, 33]] = False
+    for prec, tol in ((abi.PREC_SPLIT, 1e-10), (abi.PREC_FP32, 1e-6)):
+        if prec == abi.PREC_FP32 and not 1e-30 < factor < 1e30:
+            continue  # its element matrices are stored as floats
+        got = _element_matrices(ctx, gb, xyz, conn, prec)
+        assert not got[7].any() and np.isnan(got[~fine]).all()
+        r, d = ref[fine] / factor, (got[fine] - ref[fine]) / factor
+        err = np.linalg.norm(d, axis=1) / np.maximum(np.linalg.norm(r, axis=1), 1e-300)
+        assert np.all(np.isfinite(got[fine])) and err.max() <= tol, f"precision {prec}: error {err.max():.3e} > {tol:g}"
