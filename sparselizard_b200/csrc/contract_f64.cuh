@@ -18,9 +18,12 @@
 //    K advances 16 at a time through a 3-stage cp.async ring of C^T and M^T
 //    tiles in shared memory (rows padded to 68 and BP + 4 doubles so that the
 //    fragment loads of a half-warp hit distinct banks).
-//  * Fragments are stored straight to global memory: each value at its
-//    entry, and for the mirrored forms also at its mirror entry (same matrix
-//    or the partner's).
+//  * The finished tile is staged in shared memory and stored as whole 32-byte
+//    sectors (one 4-value store per thread), at the entries and, for the
+//    mirrored forms, at their mirrors (same matrix or the partner's), by a
+//    list of stores per bin of rows.  Stored straight from the fragments, 8
+//    bytes at a time, most sectors were written in parts, each part about as
+//    dear as ten whole sectors (149 x 149 order-3 quadrangles: 50 -> 46 us).
 #pragma once
 
 #include "engine_internal.h"
@@ -34,12 +37,23 @@ constexpr int kMmaBPMax = 128;  // most rows (entries) per block; M^T rows are p
 constexpr int kMmaBQ = 16;    // (term, Gauss point) pairs per stage
 constexpr int kMmaStages = 3;
 constexpr int kMmaCS = kMmaBE + 4;  // C^T tile row stride (doubles)
+constexpr int kMmaBin = 64;         // rows that stores take together
+
+// One store: the values of 4 rows of a bin (-1: zero) at `place` .. place + 3
+// of an element matrix of out, or of out2; where rows are not on sectors, one
+// value.
+struct StoreOp {
+    int32_t place, mirror;
+    int16_t src[4];
+};
 template <int BP>
 struct MmaShape {
     static constexpr int MS = BP + 4;  // M^T tile row stride (doubles)
     static constexpr int StageDoubles = kMmaBQ * (kMmaCS + MS);
     static constexpr size_t Smem = (size_t)kMmaStages * StageDoubles * sizeof(double);
     static constexpr int NT = BP / 32;  // 8-row MMA tiles per warp
+    static constexpr int OS = BP + 8;   // row stride of the staged tile [element][row]
+    static_assert((size_t)kMmaBE * OS * sizeof(double) <= Smem, "the staged tile reuses the ring");
 };
 
 struct BuildMtParams {
@@ -47,7 +61,7 @@ struct BuildMtParams {
     const int64_t* tab_off;
     const int32_t* term_tf;
     const int32_t* term_dof;
-    const int2* rowmap;  // nullptr: row r is entry r
+    const int32_t* rowentry;  // entry of each row (-1: a zero row); nullptr: row r is entry r
     int nterms, ngp, ntf, ndof, norient, nrows, Qpad, rpad;
     double* Mt;          // [norient][Qpad][rpad]
 };
@@ -64,8 +78,8 @@ __global__ void k_build_mt(BuildMtParams p)
         const int q = (int)(oq % p.Qpad);
         const int o = (int)(oq / p.Qpad);
         double v = 0.0;
-        if (q < Q && r < p.nrows) {
-            const int pe = p.rowmap != nullptr ? p.rowmap[r].x : r;
+        const int pe = r >= p.nrows ? -1 : p.rowentry != nullptr ? p.rowentry[r] : r;
+        if (q < Q && pe >= 0) {
             const int t = q / p.ngp, g = q - t * p.ngp;
             const int i = pe / p.ndof, j = pe - i * p.ndof;
             const double tv = p.tables[p.tab_off[p.term_tf[t]] + ((int64_t)o * p.ntf + i) * p.ngp + g];
@@ -81,13 +95,15 @@ struct MmaParams {
     const double* Mt;    // [norient][Qpad][rpad]
     const double* C;     // [Q][nelem]
     const Tile* tiles;   // orientation-uniform element runs of at most 64
-    const int2* rowmap;  // nullptr: row r is entry r
-    int Q, Qpad, rpad, nrows, P;
+    const StoreOp* ops;      // stores of each bin of kMmaBin rows
+    const int32_t* opstart;  // [rpad / kMmaBin + 1]
+    int sectors;             // stores of 4 values, on sectors
+    int Q, Qpad, rpad;
+    int es, es2;         // values per element matrix of out, of out2
     int nrt;             // row tiles (rpad / BP)
-    int mirror;          // 0 none, 1 mirror entry of the same matrix, 2 mirror entry of out2
     int64_t nelem;
-    double* out;         // [nelem][P]
-    double* out2;        // partner's [nelem][P] (mirror == 2)
+    double* out;         // [nelem][es]
+    double* out2;        // where the mirrors go, [nelem][es2]: out, or the transposed partner's matrices
 };
 
 __device__ __forceinline__ void cp_async8(double* dst, const double* src, bool valid)
@@ -195,35 +211,44 @@ __global__ void __launch_bounds__(256, 2) k_contract_f64mma(MmaParams p)
         }
     }
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();  // the ring is free
 
-    // Fragment (m, n): rows e = base + gid (+8), columns r = base + 2 tig (+1).
+    // Fragment (m, n): elements e = base + gid (+8), rows r = base + 2 tig (+1).
 #pragma unroll
     for (int m = 0; m < 2; m++)
 #pragma unroll
         for (int h = 0; h < 2; h++) {
             const int e = we * 32 + m * 16 + gid + 8 * h;
-            if (e >= tile.ne)
-                continue;
-            double* orow = p.out + (int64_t)(tile.e0 + e) * p.P;
-            double* mrow = (p.mirror == 2 ? p.out2 : p.out) + (int64_t)(tile.e0 + e) * p.P;
 #pragma unroll
             for (int n = 0; n < NT; n++)
-#pragma unroll
-                for (int k = 0; k < 2; k++) {
-                    const int r = r0 + wr * (8 * NT) + n * 8 + 2 * tig + k;
-                    if (r >= p.nrows)
-                        continue;
-                    const double v = acc[m][n][2 * h + k];
-                    if (p.rowmap == nullptr) {
-                        orow[r] = v;
-                    } else {
-                        const int2 mp = p.rowmap[r];
-                        orow[mp.x] = v;
-                        if (p.mirror == 2 || mp.y != mp.x)
-                            mrow[mp.y] = v;
-                    }
-                }
+                *reinterpret_cast<double2*>(sm_mma + e * Sh::OS + wr * (8 * NT) + n * 8 + 2 * tig) =
+                    make_double2(acc[m][n][2 * h], acc[m][n][2 * h + 1]);
         }
+    __syncthreads();
+    // Each warp stores every eighth element; a lane keeps its store for all
+    // of them.
+#pragma unroll
+    for (int bin = 0; bin < BP / kMmaBin; bin++) {
+        const int o1 = p.opstart[r0 / kMmaBin + bin + 1];
+        const double* st = sm_mma + bin * kMmaBin;
+        for (int o = p.opstart[r0 / kMmaBin + bin] + lane; o < o1; o += 32) {
+            const StoreOp op = p.ops[o];
+            const int es = op.mirror ? p.es2 : p.es;
+            double* dst = (op.mirror ? p.out2 : p.out) + (int64_t)tile.e0 * es + op.place;
+            if (p.sectors) {
+                for (int e = warp; e < tile.ne; e += 8) {
+                    double v[4];
+#pragma unroll
+                    for (int k = 0; k < 4; k++) v[k] = op.src[k] >= 0 ? st[e * Sh::OS + op.src[k]] : 0.0;
+                    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(dst + (int64_t)e * es), "d"(v[0]), "d"(v[1]), "d"(v[2]),
+                                 "d"(v[3])
+                                 : "memory");
+                }
+            } else {
+                for (int e = warp; e < tile.ne; e += 8) dst[(int64_t)e * es] = st[e * Sh::OS + op.src[0]];
+            }
+        }
+    }
 }
 
 }  // namespace slgpu

@@ -638,6 +638,7 @@ static std::shared_ptr<GroupDev> make_group(Ctx* ctx, const slgpu_group& g,
     gd->ncn = g.ncurvednodes;
     gd->ntf = g.ntf;
     gd->ndof = g.ndof;
+    gd->ld = row_stride(g.ntf, g.ndof);
     gd->nterms = g.nterms;
     gd->ndests = g.ndests;
     gd->rhs = g.terms[0].dof_table < 0;
@@ -903,8 +904,10 @@ std::vector<Segment> build_segments(const Matrix& M, std::vector<int64_t>* group
             segs.push_back(Segment{coo, P * g->nelem, vb, g->dest_mult[d]});
             coo += P * g->nelem;
         }
-        // Float values take half as many doubles of the buffer.
-        vb += f32 ? (P * g->nelem + 1) / 2 : P * g->nelem;
+        // Float values take half as many doubles of the buffer; every group
+        // starts on a sector.
+        const int64_t nv = (int64_t)g->ntf * g->ld * g->nelem;
+        vb = (vb + (f32 ? (nv + 1) / 2 : nv) + 3) & ~int64_t(3);
     }
     for (auto& f : M.frags) {
         const int64_t n = (int64_t)f->nr * f->nc;
@@ -1483,23 +1486,87 @@ static bool symmetric_form(const GroupDev& g)
 
 bool group_symmetric(const GroupDev& g) { return symmetric_form(g); }
 
-// Rows of A for the mirrored forms (the upper triangle of a symmetric group,
-// or every entry of a group with a transposed partner), each with the entry
-// it is and the entry its value also goes to: (j, i) of the same matrix, or
-// (j, i) of the partner's.  They come in blocks of 4 rows i by 8 columns j
-// (row-major inside a block), so that a warp's 32 stores of one element
-// cover 4 runs of 8 entries and their mirrors 8 runs of 4, rather than one
-// run of 32 and 32 scattered entries.
-static std::vector<int2> mirrored_rows(int ntf, int ndof, bool upper)
+// The computed rows of a contraction: the entry of M that each holds (-1: a
+// zero row), and the places in an element matrix (row stride ld) that its
+// value and its mirror go to (-1: nowhere).  Form 0: every entry.  Form 1, the
+// upper triangle of a symmetric group: (i, j) also goes to (j, i).  Form 2,
+// every entry of a group with a transposed partner: (i, j) also goes to (j, i)
+// of the partner's matrix.
+//
+// `whole` (rows of both matrices on sectors): blocks of 4 x 4 entries, 16
+// consecutive rows each, so that one store instruction of a warp covers whole
+// 32-byte sectors at both places; the blocks reach over the matrix' edge into
+// the padding of its rows (zero rows), and a block on the diagonal of a
+// symmetric group is computed whole, its lower entries from the rows of their
+// mirrors.  That takes up to a row tile more (27 x 27: 444 rows instead of
+// 378, 783 instead of 729), which pays where the stores bound the contraction
+// (K of up to 512); with longer K only what needs no other tile is added.
+// Otherwise blocks of 4 rows i by 8 columns j.
+struct ComputedRows {
+    std::vector<int32_t> entry;
+    std::vector<int2> place;
+};
+
+// Rows that must be computed in a form.
+static int64_t needed_rows(const GroupDev& g, int form)
 {
-    std::vector<int2> map;
-    for (int bi = 0; bi < ntf; bi += 4)
-        for (int bj = 0; bj < ndof; bj += 8)
-            for (int i = bi; i < std::min(bi + 4, ntf); i++)
-                for (int j = bj; j < std::min(bj + 8, ndof); j++)
-                    if (!upper || j >= i)
-                        map.push_back(make_int2(i * ndof + j, j * ntf + i));
-    return map;
+    return form == 1 ? (int64_t)g.ntf * (g.ntf + 1) / 2 : (int64_t)g.ntf * g.ndof;
+}
+
+static ComputedRows entry_rows(const GroupDev& g, int form, bool whole)
+{
+    ComputedRows rows;
+    const int ntf = g.ntf, ndof = g.ndof, ld = g.ld, ld2 = form == 2 ? row_stride(ndof, ntf) : ld;
+    auto add = [&](int entry, int x, int y) {
+        rows.entry.push_back(entry);
+        rows.place.push_back(make_int2(x, y));
+    };
+    whole = whole && ld % 4 == 0 && ld2 % 4 == 0;
+    if (form == 0) {
+        for (int i = 0; i < ntf; i++)
+            for (int j = 0; j < ld; j++) add(j < ndof ? i * ndof + j : -1, i * ld + j, -1);
+    } else if (whole) {
+        for (int bi = 0; bi < ntf; bi += 4)
+            for (int bj = form == 1 ? bi : 0; bj < ndof; bj += 4)
+                for (int i = bi; i < bi + 4; i++)
+                    for (int j = bj; j < bj + 4; j++) {
+                        if (form == 1 && bj == bi) {
+                            if (i < ntf)
+                                add(j >= ndof ? -1 : j >= i ? i * ndof + j : j * ndof + i, i * ld + j, -1);
+                            continue;
+                        }
+                        const int x = i < ntf ? i * ld + j : -1, y = j < ndof ? j * ld2 + i : -1;
+                        if (x >= 0 || y >= 0)
+                            add(i < ntf && j < ndof ? i * ndof + j : -1, x, y);
+                    }
+    } else {
+        for (int bi = 0; bi < ntf; bi += 4)
+            for (int bj = 0; bj < ndof; bj += 8)
+                for (int i = bi; i < std::min(bi + 4, ntf); i++)
+                    for (int j = bj; j < std::min(bj + 8, ndof); j++)
+                        if (form != 1 || j >= i)
+                            add(i * ndof + j, i * ld + j, form == 1 && i == j ? -1 : j * ld2 + i);
+    }
+    const int64_t fit = (needed_rows(g, form) + kSplitM - 1) / kSplitM * kSplitM;
+    if ((int64_t)g.nterms * g.ngp > 512 && (int64_t)rows.entry.size() > fit) {
+        // Long K: zero rows that would need another tile are left out, the
+        // last ones first.
+        ComputedRows kept;
+        int64_t drop = (int64_t)rows.entry.size() - fit;
+        for (size_t r = rows.entry.size(); r-- > 0;)
+            if (rows.entry[r] < 0 && drop > 0) {
+                drop--;
+            } else {
+                kept.entry.push_back(rows.entry[r]);
+                kept.place.push_back(rows.place[r]);
+            }
+        if (drop > 0)
+            return entry_rows(g, form, false);
+        std::reverse(kept.entry.begin(), kept.entry.end());
+        std::reverse(kept.place.begin(), kept.place.end());
+        return kept;
+    }
+    return rows;
 }
 
 // Row slices of a group for a tier (0 split, 1 FP32 level) and form (0 every
@@ -1514,16 +1581,21 @@ static GroupDev::Split& build_split(Ctx* ctx, GroupDev& g, int slot)
     sp.reset(new GroupDev::Split());
     sp->S = tier == 0 ? 6 : 5;
     sp->L = tier == 0 ? 7 : 6;
-    const int Q = g.nterms * g.ngp, P = g.ntf * g.ndof;
+    const int Q = g.nterms * g.ngp;
     sp->Qpad = std::max(kSplitKStep, (Q + kSplitKStep - 1) / kSplitKStep * kSplitKStep);
-    sp->nrows = form == 1 ? g.ntf * (g.ntf + 1) / 2 : P;
+    const ComputedRows rows = entry_rows(g, form, tier == 0);
+    sp->nrows = (int)rows.entry.size();
     sp->Ppad = (sp->nrows + kSplitM - 1) / kSplitM * kSplitM;
-    if (form != 0)
-        upload(ctx, sp->rowmap, mirrored_rows(g.ntf, g.ndof, form == 1));
+    if (form != 0 || g.ld != g.ndof) {
+        std::vector<int32_t> both(3 * rows.entry.size());
+        std::memcpy(both.data(), rows.place.data(), rows.place.size() * sizeof(int2));
+        std::copy(rows.entry.begin(), rows.entry.end(), both.begin() + 2 * (long)rows.entry.size());
+        upload(ctx, sp->rows, both);
+    }
     sp->slices.alloc(ctx, (size_t)sp->S * g.norient * sp->Qpad * sp->Ppad);
     sp->rowscale.alloc(ctx, (size_t)g.norient * sp->Ppad * 8);
     RowSliceParams rp{};
-    rp.rowmap = sp->rowmap.empty() ? nullptr : sp->rowmap.as<int2>();
+    rp.rowentry = sp->entries();
     rp.nrows = sp->nrows;
     rp.tables = g.tables.as<double>();
     rp.tab_off = g.tab_off_d.as<int64_t>();
@@ -1691,12 +1763,13 @@ static void run_split_jobs(Ctx* ctx, const std::vector<SplitJob>& jobs, int NE)
             c.t0 = cs.ntiles;
             cs.ntiles += ntiles;
             SplitGroup& G = sp.g[sp.ngroups++];
-            G.P = g.ntf * g.ndof;
+            G.es = g.ntf * g.ld;
+            G.es2 = g.ndof * row_stride(g.ndof, g.ntf);
             G.Ppad = s.Ppad;
             G.ntp = s.Ppad / kSplitM;
             G.nk = s.Qpad / kSplitKStep;
             G.nrows = s.nrows;
-            G.rowmap = s.rowmap.empty() ? nullptr : s.rowmap.as<int2>();
+            G.rowmap = s.rows.empty() ? nullptr : s.rows.as<int2>();
             G.out2 = j.out2;
             G.tiles = g.tiles_d.as<Tile>();
             G.A = s.slices.as<int8_t>();
@@ -1713,7 +1786,7 @@ static void run_split_jobs(Ctx* ctx, const std::vector<SplitJob>& jobs, int NE)
             int pairs = 0;
             for (int a = 1; a <= s.S; a++)
                 for (int bb = 1; bb <= s.S; bb++) pairs += (a + bb <= s.L);
-            ops += 2.0 * pairs * s.nrows * Q * g.nelem;
+            ops += 2.0 * pairs * needed_rows(g, j.paired ? 2 : symmetric_form(g) ? 1 : 0) * Q * g.nelem;
             cols += cb;
             cscale += split_scale_bytes(g) / 8;
         }
@@ -1841,6 +1914,94 @@ static bool mirror_eligible(const GroupDev& g, int precision)
     return precision == SLGPU_PREC_FP64 ? fp64_mirrored(g) : uses_split(g, precision);
 }
 
+// Rows and stores of an FP64 contraction.  The entries of the computed part
+// (form 0 every entry, 1 the upper triangle, 2 every entry and its transposed
+// partner's) come in blocks of up to 4 x 4, each inside one bin of kMmaBin
+// rows (first fit, large blocks first), so that every run of 4 values that a
+// block gives -- along i for its own rows, along j for the mirrored ones --
+// is one store of a whole sector from one thread; runs over a row's end store
+// zeros into its padding.  Where rows are not padded to sectors (row_stride),
+// the stores are single values in ascending order.
+struct StorePlan {
+    std::vector<int32_t> entry;    // [bins * kMmaBin]: entry of each row, -1 zero row
+    std::vector<StoreOp> ops;      // per bin, ascending places
+    std::vector<int32_t> opstart;  // [bins + 1]
+    bool sectors = false;
+};
+
+static StorePlan store_plan(const GroupDev& g, int form)
+{
+    const int ntf = g.ntf, ndof = g.ndof, ld = g.ld, ld2 = form == 2 ? row_stride(ndof, ntf) : ld;
+    struct Block {
+        int bi, bj, n;
+    };
+    std::vector<Block> blocks;
+    for (int bi = 0; bi < ntf; bi += 4)
+        for (int bj = form == 1 ? bi : 0; bj < ndof; bj += 4) {
+            const int ni = std::min(4, ntf - bi), nj = std::min(4, ndof - bj);
+            blocks.push_back({bi, bj, form == 1 && bi == bj ? ni * (ni + 1) / 2 : ni * nj});
+        }
+    std::stable_sort(blocks.begin(), blocks.end(), [](const Block& a, const Block& b) { return a.n > b.n; });
+    StorePlan p;
+    p.sectors = ld % 4 == 0 && ld2 % 4 == 0;
+    std::vector<std::vector<Block>> bins;
+    std::vector<int> fill;
+    size_t first = 0;  // bins before it are full
+    for (const Block& b : blocks) {
+        size_t k = first;
+        while (k < bins.size() && fill[k] + b.n > kMmaBin) k++;
+        if (k == bins.size()) {
+            bins.emplace_back();
+            fill.push_back(0);
+        }
+        bins[k].push_back(b);
+        fill[k] += b.n;
+        while (first < bins.size() && fill[first] == kMmaBin) first++;
+    }
+    p.opstart.push_back(0);
+    for (auto& bin : bins) {
+        const size_t r0 = p.entry.size();
+        const size_t o0 = p.ops.size();
+        for (const Block& b : bin) {
+            const bool diag = form == 1 && b.bi == b.bj;
+            int row[4][4];
+            for (int i = 0; i < 4; i++)
+                for (int j = 0; j < 4; j++) {
+                    row[i][j] = -1;
+                    if (b.bi + i < ntf && b.bj + j < ndof && !(diag && j < i)) {
+                        row[i][j] = (int)(p.entry.size() - r0);
+                        p.entry.push_back((b.bi + i) * ndof + b.bj + j);
+                    }
+                }
+            if (diag)
+                for (int i = 0; i < 4; i++)
+                    for (int j = 0; j < i; j++) row[i][j] = row[j][i];
+            auto run = [&](int place, bool mirror, int s0, int s1, int s2, int s3, int len) {
+                const int src[4] = {s0, s1, s2, s3};
+                if (p.sectors) {
+                    p.ops.push_back(StoreOp{place, mirror ? 1 : 0, {(int16_t)s0, (int16_t)s1, (int16_t)s2, (int16_t)s3}});
+                } else {
+                    for (int k = 0; k < len; k++) p.ops.push_back(StoreOp{place + k, mirror ? 1 : 0, {(int16_t)src[k], -1, -1, -1}});
+                }
+            };
+            for (int i = 0; i < 4 && b.bi + i < ntf; i++)
+                run((b.bi + i) * ld + b.bj, false, row[i][0], row[i][1], row[i][2], row[i][3], std::min(4, ndof - b.bj));
+            if (form != 0 && !diag)
+                for (int j = 0; j < 4 && b.bj + j < ndof; j++)
+                    run((b.bj + j) * ld2 + b.bi, true, row[0][j], row[1][j], row[2][j], row[3][j], std::min(4, ntf - b.bi));
+        }
+        std::sort(p.ops.begin() + (long)o0, p.ops.end(),
+                  [](const StoreOp& a, const StoreOp& b) { return a.mirror != b.mirror ? a.mirror < b.mirror : a.place < b.place; });
+        p.opstart.push_back((int32_t)p.ops.size());
+        p.entry.resize(r0 + kMmaBin, -1);
+    }
+    while (p.entry.size() % kMmaBPMax != 0) {  // whole row tiles
+        p.entry.resize(p.entry.size() + kMmaBin, -1);
+        p.opstart.push_back((int32_t)p.ops.size());
+    }
+    return p;
+}
+
 // Resident M^T of a group for the FP64 tensor-core kernel, built on first use
 // in the main execution state's stream order (a request stream waits for it).
 static GroupDev::Fp64Mt& ensure_fmt(Ctx* ctx, GroupDev& g, int form)
@@ -1852,25 +2013,30 @@ static GroupDev::Fp64Mt& ensure_fmt(Ctx* ctx, GroupDev& g, int form)
     ctx->x = &ctx->main;
     try {
         f.reset(new GroupDev::Fp64Mt());
-        const int Q = g.nterms * g.ngp, P = g.ntf * g.ndof;
-        f->nrows = form == 1 ? g.ntf * (g.ntf + 1) / 2 : P;
+        const int Q = g.nterms * g.ngp;
+        const StorePlan plan = store_plan(g, form);
         f->Qpad = (Q + kMmaBQ - 1) / kMmaBQ * kMmaBQ;
-        f->rpad = (f->nrows + kMmaBPMax - 1) / kMmaBPMax * kMmaBPMax;
-        if (form != 0)
-            upload(ctx, f->rowmap, mirrored_rows(g.ntf, g.ndof, form == 1));
+        f->rpad = ((int)plan.entry.size() + kMmaBPMax - 1) / kMmaBPMax * kMmaBPMax;
+        f->sectors = plan.sectors;
+        f->nops = (int)plan.ops.size();
+        std::vector<int32_t> all(sizeof(StoreOp) / 4 * plan.ops.size());
+        std::memcpy(all.data(), plan.ops.data(), plan.ops.size() * sizeof(StoreOp));
+        all.insert(all.end(), plan.opstart.begin(), plan.opstart.end());
+        all.insert(all.end(), plan.entry.begin(), plan.entry.end());
+        upload(ctx, f->plan, all);
         f->Mt.alloc(ctx, (size_t)g.norient * f->Qpad * f->rpad * sizeof(double));
         BuildMtParams bp{};
         bp.tables = g.tables.as<double>();
         bp.tab_off = g.tab_off_d.as<int64_t>();
         bp.term_tf = g.term_tf_d.as<int32_t>();
         bp.term_dof = g.term_dof_d.as<int32_t>();
-        bp.rowmap = f->rowmap.empty() ? nullptr : f->rowmap.as<int2>();
+        bp.rowentry = f->plan.as<int32_t>() + sizeof(StoreOp) / 4 * plan.ops.size() + plan.opstart.size();
         bp.nterms = g.nterms;
         bp.ngp = g.ngp;
         bp.ntf = g.ntf;
         bp.ndof = g.ndof;
         bp.norient = g.norient;
-        bp.nrows = f->nrows;
+        bp.nrows = (int)plan.entry.size();
         bp.Qpad = f->Qpad;
         bp.rpad = f->rpad;
         bp.Mt = f->Mt.as<double>();
@@ -1923,16 +2089,17 @@ static void contract_fp64_mma(Ctx* ctx, GroupDev& g, const double* C, double* ou
     mp.Mt = f.Mt.as<double>();
     mp.C = C;
     mp.tiles = g.tiles_d.as<Tile>();
-    mp.rowmap = f.rowmap.empty() ? nullptr : f.rowmap.as<int2>();
+    mp.ops = f.plan.as<StoreOp>();
+    mp.opstart = f.plan.as<int32_t>() + sizeof(StoreOp) / 4 * f.nops;
+    mp.sectors = f.sectors ? 1 : 0;
     mp.Q = g.nterms * g.ngp;
     mp.Qpad = f.Qpad;
     mp.rpad = f.rpad;
-    mp.nrows = f.nrows;
-    mp.P = g.ntf * g.ndof;
-    mp.mirror = form;
+    mp.es = g.ntf * g.ld;
+    mp.es2 = form == 2 ? g.ndof * row_stride(g.ndof, g.ntf) : mp.es;
     mp.nelem = g.nelem;
     mp.out = out;
-    mp.out2 = out2;
+    mp.out2 = form == 2 ? out2 : out;
     static const int forced = [] {
         const char* v = std::getenv("SLGPU_F64_TILE");
         return v == nullptr ? 0 : std::strcmp(v, "64") == 0 ? 64 : std::strcmp(v, "128") == 0 ? 128 : 0;
@@ -1954,7 +2121,7 @@ static void contract_fp64_mma(Ctx* ctx, GroupDev& g, const double* C, double* ou
         else
             bp = 128;
     }
-    const int kt = kstat_start(ctx, "contract_fp64", 2.0 * f.nrows * mp.Q * g.nelem);
+    const int kt = kstat_start(ctx, "contract_fp64", 2.0 * needed_rows(g, form) * mp.Q * g.nelem);
     run(bp);
     kstat_stop(ctx, kt);
 }
@@ -2259,8 +2426,10 @@ void launch_contractions(Ctx* ctx, const Matrix& M, int precision, const std::ve
     phase_event(ctx, ctx->x->evpool[2]);
     C.release();
     {
-        int64_t vb = 0;
-        for (auto& g : M.groups) vb += (int64_t)g->ntf * g->ndof * g->nelem;
+        // Where build_segments put the first fragment's values (steps with
+        // fragments hold no float values).
+        int64_t vb = M.groups.empty() ? 0 : gvb.back() + (int64_t)M.groups.back()->ntf * M.groups.back()->ld * M.groups.back()->nelem;
+        vb = (vb + 3) & ~int64_t(3);
         for (auto& f : M.frags) {
             int64_t n = (int64_t)f->nr * f->nc;
             if (n > 0)
@@ -2290,13 +2459,13 @@ static int row_kernel_forced()
     return k;
 }
 
-std::vector<RowSeg> row_segments(const Matrix& M, const std::vector<Segment>& segs, bool f32)
+std::vector<RowSeg> row_segments(const Matrix& M, const std::vector<Segment>& segs)
 {
     std::vector<RowSeg> rsegs(segs.size());
     size_t s = 0;
     for (auto& g : M.groups)
-        for (int d = 0; d < g->ndests; d++, s++) rsegs[s] = RowSeg{segs[s].coo_base, segs[s].val_base, segs[s].mult, g->ndof, f32 ? 1 : 0};
-    for (size_t f = 0; f < M.frags.size(); f++, s++) rsegs[s] = RowSeg{segs[s].coo_base, segs[s].val_base, 1.0, 1, 0};
+        for (int d = 0; d < g->ndests; d++, s++) rsegs[s] = RowSeg{segs[s].coo_base, segs[s].val_base, segs[s].mult, g->ndof, g->ld};
+    for (size_t f = 0; f < M.frags.size(); f++, s++) rsegs[s] = RowSeg{segs[s].coo_base, segs[s].val_base, 1.0, 1, 1};
     return rsegs;
 }
 
@@ -2415,7 +2584,7 @@ void launch_warp_rows(Ctx* ctx, RowParams rp, bool f32)
 // the context's own stream times both on its data and keeps the faster one
 // for the pattern.
 void launch_row_values(Ctx* ctx, const Matrix& M, Pattern& P, const std::vector<RowSeg>& rsegs, const RowSeg* dsegs, bool rhs,
-                       const double* vals, double* Avals, double* Dvals)
+                       bool f32, const double* vals, double* Avals, double* Dvals)
 {
     if (P.nA <= 0)
         return;
@@ -2432,8 +2601,6 @@ void launch_row_values(Ctx* ctx, const Matrix& M, Pattern& P, const std::vector<
     rp.Avals = Avals;
     rp.Dvals = rhs ? nullptr : Dvals;
     rp.dense = rhs ? Avals : nullptr;
-    // Element values stored as floats (every segment alike, float_values()).
-    const bool f32 = !rsegs.empty() && rsegs[0].f32 != 0;
     // Segments of one width (<= 32) with multiplier 1: the warp kernel takes
     // both from the launch instead of from each incidence.
     rp.uniform_width = 0;
@@ -2441,7 +2608,10 @@ void launch_row_values(Ctx* ctx, const Matrix& M, Pattern& P, const std::vector<
         bool uni = true;
         for (const RowSeg& sg : rsegs)
             uni = uni && sg.width == rsegs[0].width && sg.mult == 1.0;
-        if (uni)
+        // Its value offsets are 32 bits: fewer than 2^32 values.
+        const RowSeg& last = rsegs.back();
+        const int64_t nvals = last.val_base * (f32 ? 2 : 1) + (P.ncoo - last.coo_base) / std::max(1, (int)last.width) * last.ld;
+        if (uni && nvals < int64_t(0xFFFFFFFF))
             rp.uniform_width = rsegs[0].width;
     }
     // Bytes: kept element values and their slots, incidences, row
@@ -2629,7 +2799,7 @@ static void capture_value_graph(Ctx* ctx, Matrix& M, int precision, bool rhs, co
     try {
         launch_contractions(ctx, M, precision, gvb, M.vals.as<double>(), nullptr, float_values(M, precision));
         phase_event(ctx, ctx->x->ev[2]);
-        launch_row_values(ctx, M, *M.pattern, M.rsegs_host, M.rsegs_dev.as<RowSeg>(), rhs, M.vals.as<double>(), Av, Dv);
+        launch_row_values(ctx, M, *M.pattern, M.rsegs_host, M.rsegs_dev.as<RowSeg>(), rhs, float_values(M, precision), M.vals.as<double>(), Av, Dv);
     } catch (const std::exception& e) {
         err = e.what();
     }
@@ -2751,7 +2921,7 @@ static void process_matrix(Ctx* ctx, Matrix& M, const uint8_t* isconstrained, in
     // Resident segment array of the value kernels (updated in place while its
     // size is unchanged, so that captured graphs stay valid).
     {
-        std::vector<RowSeg> rsegs = row_segments(M, segs, f32v);
+        std::vector<RowSeg> rsegs = row_segments(M, segs);
         const size_t nb = rsegs.size() * sizeof(RowSeg);
         const bool same = rsegs.size() == M.rsegs_host.size() && std::memcmp(rsegs.data(), M.rsegs_host.data(), nb) == 0;
         if (!same || M.rsegs_dev.empty()) {
@@ -2791,7 +2961,7 @@ static void process_matrix(Ctx* ctx, Matrix& M, const uint8_t* isconstrained, in
     if (!graphed) {
         launch_contractions(ctx, M, precision, gvb, M.vals.as<double>(), nullptr, float_values(M, precision));
         phase_event(ctx, ctx->x->ev[2]);
-        launch_row_values(ctx, M, P, M.rsegs_host, M.rsegs_dev.as<RowSeg>(), rhs, M.vals.as<double>(), Av, Dv);
+        launch_row_values(ctx, M, P, M.rsegs_host, M.rsegs_dev.as<RowSeg>(), rhs, f32v, M.vals.as<double>(), Av, Dv);
     }
     ev_record(ctx, 3);
     cuda_check(cudaEventSynchronize(ctx->x->ev[3]), "sync");

@@ -82,6 +82,7 @@ struct GroupDev {
     int mesh = 0, elemtype = 0, elemdim = 0, problemdim = 0;
     int64_t nelem = 0;
     int norient = 1, ngp = 0, ncn = 0, ntf = 0, ndof = 0, nterms = 0, ndests = 0;
+    int ld = 0;  // values from one row of an element matrix to the next in the value buffer (row_stride)
     bool rhs = false;
     std::vector<Instr> prog;
     std::vector<int64_t> tab_off;
@@ -136,14 +137,19 @@ struct GroupDev {
     // slot tier + 2 form.
     struct Split {
         int S = 0, L = 0, Qpad = 0, Ppad = 0, nrows = 0;
-        DevBuf slices, rowscale, rowmap;
+        DevBuf slices, rowscale;
+        DevBuf rows;  // int2 [nrows] places, then int32 [nrows] entries; empty: row r is entry and value r
+        const int32_t* entries() const { return rows.empty() ? nullptr : rows.as<int32_t>() + 2 * nrows; }
     };
     std::unique_ptr<Split> split[6];
     // FP64 tensor-core operand M^T per form (0 every entry, 1 upper triangle
     // of a symmetric group, 2 every entry with its transposed partner's).
     struct Fp64Mt {
-        int Qpad = 0, rpad = 0, nrows = 0;
-        DevBuf Mt, rowmap;
+        int Qpad = 0, rpad = 0;
+        bool sectors = false;  // stores of 4 values (else single ones)
+        DevBuf Mt;
+        DevBuf plan;  // StoreOp [nops], then int32 [rpad / kMmaBin + 1] first store of each bin, then int32 [rpad] entries
+        int nops = 0;
     };
     std::unique_ptr<Fp64Mt> fmt[3];
 
@@ -174,7 +180,7 @@ struct Pattern {
     DevBuf ainds, dinds;   // int32 [nA], [nD]: global DOF of each local row of A / column of D
     DevBuf slotmap;        // int16 [ncoo]: position in the row's [A | D] segment, -1 = dropped
     DevBuf inc_ptr;        // uint32 [nA+1]: incidences of each row
-    DevBuf inc;            // uint64 [ninc]: segment << 40 | COO index of the incidence's first entry
+    DevBuf inc;            // uint64 [ninc]: serial << 63 | segment << 40 | number of the incidence in its segment
     uint64_t last_use = 0;
     // Right-hand-side patterns: the rows (DOFs) that receive at least one
     // entry, ascending, on the host and the device (built on first use).
@@ -184,16 +190,31 @@ struct Pattern {
 };
 
 // Per COO segment, as the CSR value kernels read it: where its entries
-// values start in the element-value buffer, its destination multiplier, the
-// width of its incidences (ndof of a group, 1 for a raw fragment) and whether
-// the values are stored as floats (FP32-level steps, float_values(): entry k
-// of the segment is float number 2 * val_base + k of the buffer).
-struct RowSeg {
+// start in COO order and its values in the element-value buffer, its
+// destination multiplier, the width of its incidences (ndof of a group, 1 for
+// a raw fragment) and the values from one incidence to the next.  Values
+// stored as floats (FP32-level steps, float_values()): value k of the segment
+// is float number 2 * val_base + k of the buffer.  32 bytes, two loads.
+struct alignas(16) RowSeg {
     int64_t coo_base;
     int64_t val_base;
     double mult;
-    int32_t width, f32;
+    int32_t width, ld;
 };
+
+// Values from one row of an ntf x ndof element matrix to the next in the
+// value buffer.  The rows of the larger matrices start on 32-byte sectors
+// where that costs at most an eighth more (27 -> 28, 35 -> 36): a store that
+// covers a sector partly costs about as much as ten whole sectors (measured:
+// 18e9 partly written sectors a second against 170e9 whole ones), and the
+// contractions' blocks of 4 x 4 entries can then be stored as whole sectors
+// both ways (entry_rows in engine.cu).  10 -> 12 was measured too: the larger
+// buffer cost the value kernel more than the stores gained.
+inline int row_stride(int ntf, int ndof)
+{
+    const int ld = (ndof + 3) & ~3;
+    return (int64_t)ntf * ndof > 32 && 8 * (ld - ndof) <= ndof ? ld : ndof;
+}
 
 struct Segment {
     int64_t coo_base;
@@ -360,9 +381,9 @@ bool float_values(const Matrix& M, int precision);
 std::vector<Segment> build_segments(const Matrix& M, std::vector<int64_t>* group_val_base, int64_t* total_vals, bool f32 = false);
 void launch_contractions(Ctx* ctx, const Matrix& M, int precision, const std::vector<int64_t>& gvb, double* vals,
                          const std::vector<GroupData>* ov, bool f32 = false);
-std::vector<RowSeg> row_segments(const Matrix& M, const std::vector<Segment>& segs, bool f32 = false);
+std::vector<RowSeg> row_segments(const Matrix& M, const std::vector<Segment>& segs);
 void launch_row_values(Ctx* ctx, const Matrix& M, Pattern& P, const std::vector<RowSeg>& rsegs, const RowSeg* dsegs, bool rhs,
-                       const double* vals, double* Avals, double* Dvals);
+                       bool f32, const double* vals, double* Avals, double* Dvals);
 // Copies `bytes` from host memory to a new device buffer through the current
 // execution state's page-locked staging (asynchronous, stream-ordered).
 void upload_staged(Ctx* ctx, DevBuf& buf, const void* src, size_t bytes);

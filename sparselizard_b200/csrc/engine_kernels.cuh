@@ -659,9 +659,9 @@ __global__ void k_inc_keys(const IncSeg* segs, int s, const uint8_t* constrained
     count_valid(nvalid, valid);
 }
 
-// inc[k] = (serial << 63) | (segment << 40) | COO index of the incidence's
-// first entry; serial marks an incidence with repeated addresses, whose
-// entries must be added one after the other.
+// inc[k] = (serial << 63) | (segment << 40) | the incidence's number in its
+// segment; serial marks an incidence with repeated addresses, whose entries
+// must be added one after the other.
 __global__ void k_inc_finalize(const uint32_t* skeys, const uint32_t* sids, int64_t ninc, const IncSeg* segs, int nsegs,
                                const int32_t* renum, const uint8_t* dup, unsigned long long* inc, uint32_t* rowcount)
 {
@@ -688,7 +688,7 @@ __global__ void k_inc_finalize(const uint32_t* skeys, const uint32_t* sids, int6
     }
     unsigned long long serial = 0;
     for (int j = 0; j < sg.width; j++) serial |= dup[coo + j];
-    inc[k] = (serial << 63) | ((unsigned long long)lo << 40) | (unsigned long long)coo;
+    inc[k] = (serial << 63) | ((unsigned long long)lo << 40) | (unsigned long long)local;
     atomicAdd(&rowcount[renum[skeys[k]]], 1u);
 }
 
@@ -789,9 +789,9 @@ __global__ void __launch_bounds__(kThreadRows) k_row_thread(RowParams p)
     for (uint32_t k = k0; k < k1; k++) {
         const unsigned long long pk = p.inc[k];
         const RowSeg sg = p.segs[(pk >> 40) & ((1ull << 23) - 1)];
-        const long long co = (long long)(pk & ((1ull << 40) - 1));
-        const V* v = vals + (sg.val_base * kScale + (co - sg.coo_base));
-        const int16_t* sl = p.slotmap + co;
+        const long long n = (long long)(pk & ((1ull << 40) - 1));
+        const V* v = vals + (sg.val_base * kScale + n * sg.ld);
+        const int16_t* sl = p.slotmap + (sg.coo_base + n * sg.width);
         for (int j = 0; j < sg.width; j++) {
             const int s = sl[j];
             if (s >= 0)
@@ -835,26 +835,30 @@ __global__ void __launch_bounds__(256, 6) k_row_values(RowParams p)
         i_lo = p.inc_ptr[r0 + lane];
     }
     __syncwarp();
-    constexpr int kGeneric = 1 << 17, kSerial = 1 << 16;
+    constexpr uint32_t kGeneric = 1u << 17, kSerial = 1u << 16;
     for (int rr = 0; rr < nr; rr++) {
         // The CSR bounds are fetched after the incidences (only the
         // write-back needs them): fewer registers live in the loop below.
         const uint32_t k0 = __shfl_sync(0xffffffffu, i_lo, rr), k1 = __shfl_sync(0xffffffffu, i_lo, rr + 1);
         for (uint32_t kb = k0; kb < k1; kb += 32) {
             const int nkb = (int)min(32u, k1 - kb);
-            // Lane l decodes incidence kb + l.  Value and COO offsets fit 32
-            // bits (fewer than 2^32 COO entries per matrix).
+            // Lane l decodes incidence kb + l.  COO offsets fit 32 bits (fewer
+            // than 2^32 COO entries per matrix); value offsets, with their
+            // row strides, 32 bits in the uniform form and 46 otherwise.
             uint32_t voff = 0, coo = 0;
             double mult = 0.0;
-            int info = 0;  // width | kSerial | kGeneric
+            uint32_t info = 0;  // width | kSerial | kGeneric | value offset bits 32 .. 45 from bit 18
             if (lane < nkb) {
                 const unsigned long long pk = p.inc[kb + lane];
                 const RowSeg sg = p.segs[(pk >> 40) & ((1ull << 23) - 1)];
-                coo = (uint32_t)(pk & ((1ull << 40) - 1));
-                voff = (uint32_t)(sg.val_base * kScale + ((long long)coo - sg.coo_base));
+                const uint32_t n = (uint32_t)pk;  // fewer than 2^32 incidences
+                coo = (uint32_t)sg.coo_base + n * (uint32_t)sg.width;
+                const uint64_t v = (uint64_t)sg.val_base * kScale + (uint64_t)n * (uint32_t)sg.ld;
+                voff = (uint32_t)v;
                 mult = sg.mult;
                 const bool serial = (pk >> 63) != 0;
-                info = sg.width | (serial ? kSerial : 0) | ((serial || sg.width > 32) ? kGeneric : 0);
+                info = (uint32_t)sg.width | (serial ? kSerial : 0) | ((serial || sg.width > 32) ? kGeneric : 0) |
+                       (uint32_t)(v >> 32) << 18;
             }
             if (!__any_sync(0xffffffffu, (info & kGeneric) != 0)) {
                 // Batches of kRowBatch incidences: every load issued before
@@ -865,14 +869,19 @@ __global__ void __launch_bounds__(256, 6) k_row_values(RowParams p)
 #pragma unroll
                     for (int x = 0; x < kRowBatch; x++) {
                         const int src = (u + x) & 31;
-                        const uint32_t vo = __shfl_sync(0xffffffffu, voff, src);
+                        uint64_t vo = __shfl_sync(0xffffffffu, voff, src);
                         const uint32_t co = __shfl_sync(0xffffffffu, coo, src);
-                        const int w = U ? p.uniform_width : (__shfl_sync(0xffffffffu, info, src) & 0xffff);
+                        int w = p.uniform_width;
+                        if constexpr (!U) {
+                            const uint32_t inf = __shfl_sync(0xffffffffu, info, src);
+                            w = (int)(inf & 0xffff);
+                            vo |= (uint64_t)(inf >> 18) << 32;
+                        }
                         slot[x] = -1;
                         val[x] = 0.0;
                         if (u + x < nkb && lane < w) {
                             slot[x] = p.slotmap[(uint64_t)co + lane];
-                            val[x] = (double)vals[(uint64_t)vo + lane];
+                            val[x] = (double)vals[vo + lane];
                         }
                     }
 #pragma unroll
@@ -893,11 +902,11 @@ __global__ void __launch_bounds__(256, 6) k_row_values(RowParams p)
                 }
             } else {
                 for (int x = 0; x < nkb; x++) {
-                    const uint32_t vo = __shfl_sync(0xffffffffu, voff, x);
+                    const uint32_t inf = __shfl_sync(0xffffffffu, info, x);
+                    const uint64_t vo = __shfl_sync(0xffffffffu, voff, x) | (uint64_t)(inf >> 18) << 32;
                     const uint32_t co = __shfl_sync(0xffffffffu, coo, x);
                     const double m = __shfl_sync(0xffffffffu, mult, x);
-                    const int inf = __shfl_sync(0xffffffffu, info, x);
-                    row_add_generic(buf, inf & 0xffff, m, vals + vo, p.slotmap + co, (inf & kSerial) != 0, lane);
+                    row_add_generic(buf, (int)(inf & 0xffff), m, vals + vo, p.slotmap + co, (inf & kSerial) != 0, lane);
                     __syncwarp();
                 }
             }

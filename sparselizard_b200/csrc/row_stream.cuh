@@ -124,9 +124,9 @@ __global__ void __launch_bounds__(kStreamWarps * 32) k_row_stream(RowStreamParam
         if ((uint32_t)lane < n) {
             const unsigned long long pkd = p.inc[pk + lane];
             const RowSeg sg = p.segs[(pkd >> 40) & ((1ull << 23) - 1)];
-            const long long co = (long long)(pkd & ((1ull << 40) - 1));
-            const long long vo = sg.val_base + (co - sg.coo_base);
             const int width = sg.width;
+            const long long n = (long long)(pkd & ((1ull << 40) - 1));
+            const long long co = sg.coo_base + n * width, vo = sg.val_base + n * sg.ld;
             const uint64_t vbyte = (uint64_t)vo * 8, sbyte = (uint64_t)co * 2;
             const uint32_t nv = (uint32_t)(((vbyte + (uint64_t)width * 8 + 15) >> 4) - (vbyte >> 4));
             const uint32_t ns = (uint32_t)(((sbyte + (uint64_t)width * 2 + 15) >> 4) - (sbyte >> 4));

@@ -121,7 +121,7 @@ int64_t estimate_bytes(const Matrix& M, int precision, const Request* r)
 {
     int64_t vals = 0, coef = 0, exps = 0, split = 0;
     for (auto& g : M.groups) {
-        vals += (int64_t)g->ntf * g->ndof * g->nelem;
+        vals += (int64_t)g->ntf * g->ld * g->nelem;
         coef += (int64_t)g->nterms * g->ngp * g->nelem;
         exps += g->nelem;
         // The split groups of a request are sliced and contracted together:
@@ -251,7 +251,7 @@ void launch(Server& S, Slot& s, Request& r)
     const double t2 = S.now();
     r.Avals.alloc(ctx, (size_t)std::max<int64_t>(P.nnzA, 1) * 8);
     r.Dvals.alloc(ctx, (size_t)std::max<int64_t>(P.nnzD, 1) * 8);
-    std::vector<RowSeg> rsegs = row_segments(M, segs, f32v);
+    std::vector<RowSeg> rsegs = row_segments(M, segs);
     // Destination multipliers of the request's scale updates (segments are
     // the groups' destinations in order).
     if (!r.scales.empty()) {
@@ -264,7 +264,7 @@ void launch(Server& S, Slot& s, Request& r)
     }
     DevBuf dsegs;
     upload_staged(ctx, dsegs, rsegs.data(), rsegs.size() * sizeof(RowSeg));
-    launch_row_values(ctx, M, P, rsegs, dsegs.as<RowSeg>(), false, r.vals.as<double>(), r.Avals.as<double>(), r.Dvals.as<double>());
+    launch_row_values(ctx, M, P, rsegs, dsegs.as<RowSeg>(), false, f32v, r.vals.as<double>(), r.Avals.as<double>(), r.Dvals.as<double>());
     r.vals.release();  // stream-ordered: after the value kernel
     double* hA = r.pinned_out ? r.Aout : static_cast<double*>(s.pinned);
     double* hD = r.pinned_out ? r.Dout : static_cast<double*>(s.pinned) + r.nnzA;
@@ -683,7 +683,7 @@ int slgpu_server_submit_template(slgpu_server* S, int handle, const uint8_t* isc
         int64_t ncoo = 0, nvals = 0;
         for (auto& g : M.groups) {
             ncoo += (int64_t)g->ntf * g->ndof * g->nelem * g->ndests;
-            nvals += (int64_t)g->ntf * g->ndof * g->nelem;
+            nvals += (int64_t)g->ntf * g->ld * g->nelem;
         }
         for (auto& f : M.frags) {
             ncoo += (int64_t)f->nr * f->nc;

@@ -70,17 +70,19 @@ struct SplitShape {
 // [w0, w0 + nwork) of the launch: item w0 + v is row tile v % ntp of element
 // unit v / ntp.
 struct SplitGroup {
-    int P, Ppad, ntp, nk;   // entries, padded rows, row tiles, K steps
-    int nrows, pad;         // rows of A computed (P, or the upper triangle)
-    const int2* rowmap;     // [nrows]: the entry and its mirror; null: row r is entry r
-    double* out2;           // null, or [nelem][P]: the transposed partner group's
-                            // element matrices (entry rowmap[r].y from row r)
+    int Ppad, ntp, nk;      // padded rows, row tiles, K steps
+    int nrows;              // rows of A computed
+    int es, es2;            // values per element matrix of out, of out2
+    const int2* rowmap;     // [nrows]: where row r's value goes in an element matrix of
+                            // out, and its mirror in out2, or out (-1: nowhere); null:
+                            // row r is value r, without a mirror
+    double* out2;           // null, or the transposed partner group's element matrices
     const Tile* tiles;      // 64-element tiles; unit u = tile u / kUnits, part u % kUnits
     const int8_t* A;        // row slices
     const int8_t* B;        // column slices
     const double* rowscale;  // [norient][Ppad]: R_p 2^-(B L)
     const double* colscale;  // [ntiles][64]: Q_e of each slot
-    double* out;            // [nelem][P]
+    double* out;            // [nelem][es]
     int64_t w0, nwork;
 };
 
@@ -123,14 +125,14 @@ __device__ __forceinline__ Tile split_unit(const Tile* tiles, int64_t u)
 
 // Row slices of M for one orientation: block per row p, threads over q.
 // M[p][q] = T_t[o][i][g] * D_t[o][j][g] as in the FP64 contraction.
-// Row r of A holds entry rowmap[r].x of M (entry r without a map); rows
-// from nrows to Ppad are zero.
+// Row r of A holds entry rowentry[r] of M (entry r without that array; -1: a
+// zero row); rows from nrows to Ppad are zero.
 struct RowSliceParams {
     const double* tables;
     const int64_t* tab_off;
     const int32_t* term_tf;
     const int32_t* term_dof;
-    const int2* rowmap;
+    const int32_t* rowentry;
     int nterms, ngp, ntf, ndof, norient, Qpad, Ppad, nrows;
     int L;            // largest level
     int8_t* slices;   // [orient][ptile][kstep][S][2][128][16]
@@ -217,7 +219,7 @@ template <int B, int S>
 __global__ void k_slice_rows(RowSliceParams p)
 {
     const int pe = blockIdx.x, o = blockIdx.y;
-    const int src = pe >= p.nrows ? -1 : p.rowmap != nullptr ? p.rowmap[pe].x : pe;
+    const int src = pe >= p.nrows ? -1 : p.rowentry != nullptr ? p.rowentry[pe] : pe;
     __shared__ int top;
     if (threadIdx.x == 0)
         top = 0;
@@ -406,28 +408,59 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar)
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
-// 16 consecutive 32-bit TMEM columns of this thread's lane (no wait).
-__device__ __forceinline__ void tmem_ld16_nowait(uint32_t taddr, int32_t* r)
+// 8 consecutive 32-bit TMEM columns of this thread's lane (no wait).
+__device__ __forceinline__ void tmem_ld8_nowait(uint32_t taddr, int32_t* r)
 {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-          "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr));
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr));
 }
 
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-// Exact int64 -> double for |x| < 2^51 on the integer and FP64 pipes instead
-// of the conversion unit (which the epilogue's two conversions per output
-// saturate): x is added to the bit pattern of 1.5 * 2^52, whose mantissa ulp
-// is 1, so the pattern encodes 1.5 * 2^52 + x exactly; subtracting 1.5 * 2^52
-// is exact (both operands lie in [2^52, 2^53)).  The level sums meet the
-// bound: a level holds at most 6 pair products of at most K * 2^14 each, with
-// K <= 16384, so |r| < 2^30.6 and three levels combined stay below 2^47.
-__device__ __forceinline__ double i64_to_f64_exact(long long x)
+// The NL levels r[l] of one output, most significant first, combined to
+// T = sum_l r[l] 2^(B (NL - 1 - l)) with one rounding.  The last three levels
+// make Lo, the others H; each is formed exactly in int64 on top of the bit
+// pattern of C = 1.5 2^52, whose mantissa ulp is 1, so the patterns are the
+// doubles C + H and C + Lo (no conversion instructions, which the outputs
+// would saturate).  A level holds at most 6 pair products of at most
+// K 2^14 each, with K <= 16384, so |r| < 2^30.6 and |H|, |Lo| < 2^47; then
+// H 2^3B - C is exact, and adding C + Lo rounds once.
+__device__ __forceinline__ long long mad_wide(int a, int b, long long c)
 {
-    return __longlong_as_double(0x4338000000000000LL + x) - 0x1.8p52;
+    long long d;
+    asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
+    return d;
+}
+template <int B, int NL>
+__device__ __forceinline__ double split_combine(const int32_t (&r)[NL])
+{
+    constexpr double C = 0x1.8p52, W = (double)(1 << 3 * B);
+    auto on_c = [](int32_t x) { return (long long)(((unsigned long long)(uint32_t)(0x43380000 + (x >> 31)) << 32) | (uint32_t)x); };
+    const long long lo = mad_wide(r[NL - 3], 1 << 2 * B, mad_wide(r[NL - 2], 1 << B, on_c(r[NL - 1])));
+    long long h = on_c(r[NL - 4]);
+#pragma unroll
+    for (int l = 0; l < NL - 4; l++) h = mad_wide(r[l], 1 << (B * (NL - 4 - l)), h);
+    return fma(__longlong_as_double(h), W, -C * W - C) + __longlong_as_double(lo);
+}
+
+// One row's values of nj consecutive elements (es and em values apart) at
+// its place and its mirror's (null: nowhere).
+template <class V>
+__device__ __forceinline__ void split_store(const double (&d)[16], V* out, int es, V* mirror, int em, int nj)
+{
+    if (out != nullptr) {
+#pragma unroll
+        for (int j = 0; j < 16; j++)
+            if (j < nj)
+                out[(int64_t)j * es] = (V)d[j];
+    }
+    if (mirror != nullptr) {
+#pragma unroll
+        for (int j = 0; j < 16; j++)
+            if (j < nj)
+                mirror[(int64_t)j * em] = (V)d[j];
+    }
 }
 
 // ---------------------------------------------------------------- contraction
@@ -444,6 +477,7 @@ struct SplitSmem {
     uint64_t tmem_full[2], tmem_empty[2], drain;
     uint64_t item_full[kSplitItems], item_empty[kSplitItems];
     int64_t items[kSplitItems];
+    double colscale[kSplitEpiWarps][16];  // each epilogue warp's columns of the unit at hand
     uint32_t tmem;
     int failed;
 };
@@ -644,9 +678,9 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_contract_split(const __gri
     } else if (warp >= 2) {
         // ------------------------------------------------ epilogue
         // Warp w reads TMEM lane quarter w % 4 and columns c0 .. c0+15 of
-        // each level.  The first levels are combined into H before the last
-        // three are loaded; then the accumulator is released, and the rest of
-        // the recombination and the stores overlap the next tile's MMAs.
+        // each level, 8 columns at a time; once they are in registers the
+        // accumulator is released, and the rest of the recombination and the
+        // stores overlap the next tile's MMAs.
         const int quarter = warp & 3;
         const int c0 = ((warp - 2) >> 2) * 16;
         const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16);
@@ -672,6 +706,16 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_contract_split(const __gri
             const int64_t u = v / G.ntp;
             const Tile unit = split_unit<NE>(G.tiles, u);
             const int buf = (int)(i % Sh::kBufs);
+            // What the stores need from global memory is requested before the
+            // accumulator is complete: a load issued after stores waits
+            // behind them.
+            const int pe = pt * kSplitM + quarter * 32 + lane;
+            const bool live = pe < G.nrows;
+            const double rsc = live ? __ldg(G.rowscale + (int64_t)unit.orient * G.Ppad + pe) : 0.0;
+            const int2 m = !live ? make_int2(-1, -1) : G.rowmap != nullptr ? __ldg(G.rowmap + pe) : make_int2(pe, -1);
+            if (lane < 16)
+                sm.colscale[warp - 2][lane] = __ldg(G.colscale + u * NE + c0 + lane);
+            __syncwarp();
             if (!mbar_wait(&sm.tmem_full[buf], (uint32_t)((i / Sh::kBufs) & 1), failed)) {
                 *failed = 1;
                 atomicOr(p.error, 1u);
@@ -679,72 +723,42 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_contract_split(const __gri
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t col = lane_base + (uint32_t)(buf * 256 + c0);
-            // V = R_p Q_e 2^-(B L) (H 2^3B + Lo): Lo the last three levels, H
-            // the others, each r_l times 2^B per level; both exact in int64.
-            long long H[16];
-            {
-                int32_t r[NL - 3][16];
-#pragma unroll
-                for (int l = 0; l < NL - 3; l++) tmem_ld16_nowait(col + (uint32_t)(l * NE), r[l]);
-                tmem_ld_wait();
-#pragma unroll
-                for (int j = 0; j < 16; j++) {
-                    H[j] = r[0][j];
-#pragma unroll
-                    for (int l = 1; l < NL - 3; l++) H[j] = H[j] * (1 << B) + r[l][j];
-                }
-            }
-            int32_t t[3][16];
-#pragma unroll
-            for (int l = 0; l < 3; l++) tmem_ld16_nowait(col + (uint32_t)((NL - 3 + l) * NE), t[l]);
-            tmem_ld_wait();
-            // This warp's accumulators are in registers: release them.
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0)
-                mbar_arrive(&sm.tmem_empty[buf]);
+            // V = R_p Q_e 2^-(B L) T.
             double d[16];
 #pragma unroll
-            for (int j = 0; j < 16; j++) {
-                const long long lo = ((long long)t[0][j] * (1 << B) + t[1][j]) * (1 << B) + t[2][j];
-                d[j] = fma(i64_to_f64_exact(H[j]), (double)(1 << 3 * B), i64_to_f64_exact(lo));
-            }
-            const int pe = pt * kSplitM + quarter * 32 + lane;
-            if (pe < G.nrows) {
-                const double rsc = G.rowscale[(int64_t)unit.orient * G.Ppad + pe];
-                const double* ce = G.colscale + u * NE + c0;
-                // Row pe is entry m.x and, for a symmetric group, also its
-                // mirror m.y (the same entry on the diagonal); with a
-                // transposed partner, entry (i, j) is also the partner's
-                // entry (j, i).
-                const int2 m = G.rowmap != nullptr ? G.rowmap[pe] : make_int2(pe, pe);
-                const int P = G.P;
-                const int64_t ebase = (int64_t)(unit.e0 + c0) * P;
-                double* outp = G.out + ebase + m.x;
-                double* outm = G.out2 != nullptr ? G.out2 + ebase + m.y : m.y != m.x ? G.out + ebase + m.y : nullptr;
-                const int nj = min(16, unit.ne - c0);
+            for (int h = 0; h < 16; h += 8) {
+                int32_t r[NL][8];
 #pragma unroll
-                for (int j = 0; j < 16; j += 2) {
-                    const double2 c2 = *reinterpret_cast<const double2*>(ce + j);
-                    const double cx[2] = {c2.x, c2.y};
-#pragma unroll
-                    for (int jj = 0; jj < 2; jj++) {
-                        if (j + jj < nj) {
-                            const double v = d[j + jj] * rsc * cx[jj];
-                            if (p.f32) {
-                                // Entry k of a float matrix is float k of the same buffer.
-                                const int64_t o = (int64_t)(j + jj) * P;
-                                reinterpret_cast<float*>(G.out)[ebase + m.x + o] = (float)v;
-                                if (outm != nullptr)
-                                    reinterpret_cast<float*>(G.out2 != nullptr ? G.out2 : G.out)[ebase + m.y + o] = (float)v;
-                            } else {
-                                outp[(int64_t)(j + jj) * P] = v;
-                                if (outm != nullptr)
-                                    outm[(int64_t)(j + jj) * P] = v;
-                            }
-                        }
-                    }
+                for (int l = 0; l < NL; l++) tmem_ld8_nowait(col + (uint32_t)(l * NE + h), r[l]);
+                tmem_ld_wait();
+                if (h == 8) {
+                    // This warp's accumulators are in registers: release them.
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0)
+                        mbar_arrive(&sm.tmem_empty[buf]);
                 }
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    int32_t x[NL];
+#pragma unroll
+                    for (int l = 0; l < NL; l++) x[l] = r[l][j];
+                    d[h + j] = split_combine<B, NL>(x) * rsc * sm.colscale[warp - 2][h + j];
+                }
+            }
+            __syncwarp();  // every lane has read the scales before the next unit's
+            const int64_t e = unit.e0 + c0;
+            const int nj = min(16, unit.ne - c0);
+            const int em = G.out2 != nullptr ? G.es2 : G.es;
+            double* const out = m.x >= 0 ? G.out : nullptr;
+            double* const mirror = m.y < 0 ? nullptr : G.out2 != nullptr ? G.out2 : G.out;
+            if (p.f32) {
+                // Value k of a float matrix is float k of the same buffer.
+                split_store<float>(d, out != nullptr ? reinterpret_cast<float*>(out) + e * G.es + m.x : nullptr, G.es,
+                                   mirror != nullptr ? reinterpret_cast<float*>(mirror) + e * em + m.y : nullptr, em, nj);
+            } else {
+                split_store<double>(d, out != nullptr ? out + e * G.es + m.x : nullptr, G.es,
+                                    mirror != nullptr ? mirror + e * em + m.y : nullptr, em, nj);
             }
             i++;
         }

@@ -6,6 +6,8 @@ split tier and <= 1e-6 for the FP32-level tier.  The drop-in check runs a
 small elasticity problem through sparselizard with SLGPU_PRECISION=split.
 """
 import ctypes
+import os
+import sys
 
 import numpy as np
 import pytest
@@ -13,6 +15,9 @@ import pytest
 import _pipeline as P
 import _synthetic as S
 from sparselizard_b200 import abi, meshgen, workloads as W
+
+sys.path.insert(0, os.path.join(P.ROOT, "oracle"))
+import slref  # noqa: E402
 
 pytestmark = pytest.mark.gpu
 
@@ -234,3 +239,60 @@ def test_split_scales(ctx, factor):
         r, d = ref[fine] / factor, (got[fine] - ref[fine]) / factor
         err = np.linalg.norm(d, axis=1) / np.maximum(np.linalg.norm(r, axis=1), 1e-300)
         assert np.all(np.isfinite(got[fine])) and err.max() <= tol, f"precision {prec}: error {err.max():.3e} > {tol:g}"
+
+
+@pytest.mark.parametrize("ntf,ndof,form", [(27, 27, "symmetric"), (27, 27, "pair"), (27, 27, "plain"), (29, 29, "symmetric"),
+                                           (35, 35, "symmetric"), (33, 33, "plain"), (27, 20, "pair"), (31, 27, "pair"),
+                                           (20, 20, "symmetric"), (10, 10, "symmetric"), (13, 9, "pair"), (40, 1, "plain"),
+                                           (9, 58, "plain")])
+def test_element_matrix_shapes(ctx, ntf, ndof, form):
+    """Both contractions over element matrices whose rows are and are not
+    padded to sectors, blocks cut by the edge, partly filled bins and row
+    tiles, two destinations, against the oracle's assembled matrix: the same
+    pattern, values within 1e-12 (FP64) and 1e-10 (split) of the sums of
+    magnitudes."""
+    rng = np.random.Generator(np.random.PCG64(100 * ntf + ndof))
+    ndofs = 700
+    gb, xyz, conn = S.group(rng, nelem_grid=9, ntf=ntf, ndof=ndof, nterms=3, ngp1=3, norient=2, ndests=2, ndofs=ndofs,
+                            symmetric=form == "symmetric")
+    groups = [gb.g]
+    if form == "pair":
+        g1, g2 = gb.g, abi.Group.from_buffer_copy(gb.g)
+        g2.ntf, g2.ndof = ndof, ntf
+        terms2 = (abi.Term * g1.nterms)(*[abi.Term(g1.terms[t].dof_table, g1.terms[t].tf_table, g1.terms[t].coef_node, 0,
+                                                   g1.terms[t].scale) for t in range(g1.nterms)])
+        g2.terms = terms2
+        dest2 = (abi.Dest * 2)()
+        for d in range(2):
+            dest2[d].tfaddr, dest2[d].dofaddr = g1.dests[d].dofaddr, g1.dests[d].tfaddr
+            dest2[d].multiplier = g1.dests[d].multiplier
+        g2.dests = dest2
+        groups.append(g2)
+    con = (rng.random(ndofs) < 0.1).astype(np.uint8)
+    conns = [conn] * len(groups)
+    ref = slref.matrix(groups, xyz, conns, ndofs, con)
+    mag = slref.matrix(groups, xyz, conns, ndofs, con, absmode=True)
+    L = ctx.lib
+    ctx.check(L.slgpu_mesh_set_nodes(ctx.h, 0, xyz.size // 3, abi.f64p(xyz)))
+    ctx.check(L.slgpu_mesh_set_elements(ctx.h, 0, 3, 4, conn.size // 4, abi.i32p(conn)))
+    h = ctypes.c_int()
+    ctx.check(L.slgpu_matrix_create(ctx.h, ndofs, ctypes.byref(h)))
+    for g in groups:
+        ctx.check(L.slgpu_matrix_add_group(ctx.h, h, ctypes.byref(g), None))
+    if form == "pair":
+        partner = ctypes.c_int32()
+        ctx.check(L.slgpu_matrix_group_symmetry(ctx.h, h, 0, None, None, ctypes.byref(partner)))
+        assert partner.value == 1
+    for prec, tol in ((abi.PREC_FP64, 1e-12), (abi.PREC_SPLIT, 1e-10), (abi.PREC_FP32, 1e-6)):
+        info = abi.CsrInfo()
+        ctx.check(L.slgpu_matrix_process(ctx.h, h, con.ctypes.data_as(ctypes.POINTER(ctypes.c_uint8)), prec, ctypes.byref(info)))
+        out = {k: np.zeros(max(1, n), t) for k, n, t in (("Arows", info.nA + 1, np.int32), ("Acols", info.nnzA, np.int32),
+                                                         ("Avals", info.nnzA, np.float64), ("Drows", info.nA + 1, np.int32),
+                                                         ("Dcols", info.nnzD, np.int32), ("Dvals", info.nnzD, np.float64))}
+        ctx.check(L.slgpu_matrix_download(ctx.h, h, *[abi.i32p(v) if v.dtype == np.int32 else abi.f64p(v) for v in out.values()]))
+        for k in ("Arows", "Acols", "Drows", "Dcols"):
+            assert np.array_equal(out[k][: ref[k].size], ref[k]), f"precision {prec}: {k} differs"
+        for k in ("Avals", "Dvals"):
+            err = np.abs(out[k][: ref[k].size] - ref[k]) / np.maximum(mag[k], 1e-300)
+            assert not err.size or err.max() <= tol, f"precision {prec}: {k} error {err.max():.3e} > {tol:g}"
+    ctx.check(L.slgpu_matrix_destroy(ctx.h, h))
