@@ -2060,70 +2060,110 @@ static GroupDev::Fp64Mt& ensure_fmt(Ctx* ctx, GroupDev& g, int form)
     return *f;
 }
 
+// One FP64 contraction of a launch: its group, coefficients, element matrices
+// and, for a transposed pair, the partner's.
+struct MmaJob {
+    GroupDev* g;
+    const double* C;
+    double* out;
+    double* out2;
+};
+
+static int mma_form(const MmaJob& j)
+{
+    return j.out2 != nullptr ? 2 : (fp64_mirrored(*j.g) && symmetric_form(*j.g)) ? 1 : 0;
+}
+
 template <int BP>
-static void launch_f64mma(Ctx* ctx, const GroupDev& g, MmaParams mp)
+static void launch_f64mma(Ctx* ctx, const MmaParams& mp, int64_t nblocks)
 {
     static std::once_flag attr;
     std::call_once(attr, [] {
         cudaFuncSetAttribute(k_contract_f64mma<BP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MmaShape<BP>::Smem);
     });
-    mp.nrt = mp.rpad / BP;
-    const int64_t nblocks = (int64_t)g.tiles.size() * mp.nrt;
-    if (nblocks > INT32_MAX)
-        fail(SLGPU_E_UNSUPPORTED, "group too large for one FP64 contraction launch");
     k_contract_f64mma<BP><<<(unsigned)nblocks, 256, MmaShape<BP>::Smem, ctx->x->stream>>>(mp);
     cuda_check(cudaGetLastError(), "k_contract_f64mma");
     ctx->launches++;
 }
 
-// FP64 contraction of one group on the FP64 tensor cores: every entry, the
+// FP64 tensor-core contractions of a set of jobs with BP rows per block, as
+// few launches as their blocks and descriptors allow.
+static void run_mma_jobs(Ctx* ctx, const std::vector<MmaJob>& jobs, int BP)
+{
+    size_t k = 0;
+    while (k < jobs.size()) {
+        MmaParams mp{};
+        int64_t nblocks = 0;
+        double flops = 0;
+        for (; k < jobs.size() && mp.ngroups < kMmaBatch; k++) {
+            const MmaJob& j = jobs[k];
+            GroupDev& g = *j.g;
+            const int form = mma_form(j);
+            GroupDev::Fp64Mt& f = ensure_fmt(ctx, g, form);
+            const int64_t n = (int64_t)g.tiles.size() * (f.rpad / BP);
+            if (n > INT32_MAX)
+                fail(SLGPU_E_UNSUPPORTED, "group too large for one FP64 contraction launch");
+            if (nblocks + n > INT32_MAX)
+                break;
+            MmaGroup& G = mp.g[mp.ngroups++];
+            G.Mt = f.Mt.as<double>();
+            G.C = j.C;
+            G.tiles = g.tiles_d.as<Tile>();
+            G.ops = f.plan.as<StoreOp>();
+            G.opstart = f.plan.as<int32_t>() + sizeof(StoreOp) / 4 * f.nops;
+            G.sectors = f.sectors ? 1 : 0;
+            G.Q = g.nterms * g.ngp;
+            G.Qpad = f.Qpad;
+            G.rpad = f.rpad;
+            G.es = g.ntf * g.ld;
+            G.es2 = form == 2 ? g.ndof * row_stride(g.ndof, g.ntf) : G.es;
+            G.nrt = f.rpad / BP;
+            G.w0 = (int)nblocks;
+            G.nelem = g.nelem;
+            G.out = j.out;
+            G.out2 = form == 2 ? j.out2 : j.out;
+            nblocks += n;
+            flops += 2.0 * needed_rows(g, form) * G.Q * g.nelem;
+        }
+        const int kt = kstat_start(ctx, "contract_fp64", flops);
+        if (BP == 64)
+            launch_f64mma<64>(ctx, mp, nblocks);
+        else
+            launch_f64mma<128>(ctx, mp, nblocks);
+        kstat_stop(ctx, kt);
+    }
+}
+
+// FP64 contractions of a step on the FP64 tensor cores: every entry, the
 // upper triangle of a symmetric group (mirrored into the lower), or every
 // entry with the transposed partner's element matrices written into out2.
 // Rows per block (128 or 64) are picked per group shape by timing on first
 // use (SLGPU_F64_TILE=128 or 64 forces one).
-static void contract_fp64_mma(Ctx* ctx, GroupDev& g, const double* C, double* out, double* out2)
+static void contract_fp64_all(Ctx* ctx, const std::vector<MmaJob>& jobs)
 {
-    const int form = out2 != nullptr ? 2 : (fp64_mirrored(g) && symmetric_form(g)) ? 1 : 0;
-    GroupDev::Fp64Mt& f = ensure_fmt(ctx, g, form);
-    MmaParams mp{};
-    mp.Mt = f.Mt.as<double>();
-    mp.C = C;
-    mp.tiles = g.tiles_d.as<Tile>();
-    mp.ops = f.plan.as<StoreOp>();
-    mp.opstart = f.plan.as<int32_t>() + sizeof(StoreOp) / 4 * f.nops;
-    mp.sectors = f.sectors ? 1 : 0;
-    mp.Q = g.nterms * g.ngp;
-    mp.Qpad = f.Qpad;
-    mp.rpad = f.rpad;
-    mp.es = g.ntf * g.ld;
-    mp.es2 = form == 2 ? g.ndof * row_stride(g.ndof, g.ntf) : mp.es;
-    mp.nelem = g.nelem;
-    mp.out = out;
-    mp.out2 = form == 2 ? out2 : out;
+    if (jobs.empty())
+        return;
     static const int forced = [] {
         const char* v = std::getenv("SLGPU_F64_TILE");
         return v == nullptr ? 0 : std::strcmp(v, "64") == 0 ? 64 : std::strcmp(v, "128") == 0 ? 128 : 0;
     }();
-    auto run = [&](int bp) {
-        if (bp == 64)
-            launch_f64mma<64>(ctx, g, mp);
-        else
-            launch_f64mma<128>(ctx, g, mp);
-    };
-    const std::array<int, 5> key{1, 0, g.ntf, g.ndof, g.ngp};
-    int bp = forced;
-    if (bp == 0) {
-        auto it = ctx->tile_choice.find(key);
-        if (it != ctx->tile_choice.end())
-            bp = it->second;
-        else if (!ctx->x->capturing && ctx->x == &ctx->main)
-            bp = ctx->tile_choice[key] = pick_by_timing(ctx, {128, 64}, run);
-        else
-            bp = 128;
+    std::vector<MmaJob> by[2];
+    for (const MmaJob& j : jobs) {
+        const std::array<int, 5> key{1, 0, j.g->ntf, j.g->ndof, j.g->ngp};
+        int bp = forced;
+        if (bp == 0) {
+            auto it = ctx->tile_choice.find(key);
+            if (it != ctx->tile_choice.end())
+                bp = it->second;
+            else if (!ctx->x->capturing && ctx->x == &ctx->main)
+                bp = ctx->tile_choice[key] = pick_by_timing(ctx, {128, 64}, [&](int b) { run_mma_jobs(ctx, {j}, b); });
+            else
+                bp = 128;
+        }
+        by[bp == 64 ? 1 : 0].push_back(j);
     }
-    const int kt = kstat_start(ctx, "contract_fp64", 2.0 * needed_rows(g, form) * mp.Q * g.nelem);
-    run(bp);
-    kstat_stop(ctx, kt);
+    run_mma_jobs(ctx, by[0], 128);
+    run_mma_jobs(ctx, by[1], 64);
 }
 
 // Transposed pairs among a matrix's split-precision groups: group j is the
@@ -2371,6 +2411,7 @@ void launch_contractions(Ctx* ctx, const Matrix& M, int precision, const std::ve
     phase_event(ctx, ctx->x->evpool[1]);
     size_t gi = 0;
     std::vector<SplitJob> split_jobs;  // every split-precision group of the step, contracted together
+    std::vector<MmaJob> mma_jobs;      // every FP64 group that the small kernel does not take, likewise
     for (auto& g : M.groups) {
         if (g->nelem > 0) {
             double* Cg = C.as<double>() + coff[gi];
@@ -2417,11 +2458,12 @@ void launch_contractions(Ctx* ctx, const Matrix& M, int precision, const std::ve
                 cuda_check(cudaGetLastError(), "k_contract_small");
                 ctx->launches++;
             } else {
-                contract_fp64_mma(ctx, *g, Cg, vals + gvb[gi], pair[gi] > (int)gi ? vals + gvb[pair[gi]] : nullptr);
+                mma_jobs.push_back(MmaJob{g.get(), Cg, vals + gvb[gi], pair[gi] > (int)gi ? vals + gvb[pair[gi]] : nullptr});
             }
         }
         gi++;
     }
+    contract_fp64_all(ctx, mma_jobs);
     contract_split_all(ctx, split_jobs);
     phase_event(ctx, ctx->x->evpool[2]);
     C.release();
