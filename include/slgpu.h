@@ -74,8 +74,8 @@ int slgpu_transfer_bytes(const slgpu_ctx* ctx, int64_t* h2d, int64_t* d2h);
  * be called before the memory is freed.  No counterpart in the reference. */
 int slgpu_host_register(slgpu_ctx* ctx, void* ptr, size_t bytes);
 int slgpu_host_unregister(slgpu_ctx* ctx, void* ptr);
-/* The tile shapes the first-use tuner picked (one line each: kind, choice,
- * group shape ntf/ndof/ngp) and the CSR value kernel of each resident
+/* The rows per block the first-use tuner picked for FP64 contractions (one
+ * line each: choice, group shape ntf/ndof/ngp) and the CSR value kernel of each resident
  * pattern, as text.  No counterpart in the reference (a single fixed BLAS
  * switch, src/densemat.cpp:264-306, picks between dgemm and a loop). */
 int slgpu_tuned_tiles(slgpu_ctx* ctx, char* buf, size_t len);
@@ -301,7 +301,8 @@ int slgpu_check_coefficient_kernels(slgpu_ctx* ctx, int handle, char* log, size_
  * algorithmic work of those launches.  Families and work units:
  *   "coefficients"        bytes of coefficients written (8 per term, point, element)
  *   "contract_fp64"       FLOPs, 2*ntf*ndof*nterms*ngp per element
- *   "slice_cols"          bytes: coefficients read, slices and exponents written
+ *   "slice_cols"          bytes: slices and scales written (and coefficients read,
+ *                         where they went through memory)
  *   "contract_split"      INT8 tensor operations, 2*pairs*ntf*ndof*nterms*ngp per
  *   "contract_split_fp32" element (pairs = 21 for the split tier, 15 for FP32)
  *   "row_values"          bytes: kept element values + slots, incidences, row

@@ -1658,49 +1658,37 @@ static bool split_supported(const GroupDev& g)
     return Q > 0 && Q <= 16384;
 }
 
-template <int B, int S, int L, int NE>
+template <int B, int S, int L>
 static void launch_split(Ctx* ctx, const SplitParams& p)
 {
     static bool attr = false;
-    constexpr size_t smem = split_smem_bytes<NE>();
+    constexpr size_t smem = split_smem_bytes();
     if (!attr) {
-        cuda_check(cudaFuncSetAttribute(k_contract_split<B, S, L, NE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+        cuda_check(cudaFuncSetAttribute(k_contract_split<B, S, L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                    "smem attribute");
         attr = true;
     }
     const int64_t grid = std::min<int64_t>(p.nwork, std::max(ctx->nsm, 1));
     cuda_check(cudaMemsetAsync(p.next, 0, sizeof(unsigned long long), ctx->x->stream), "memset");
-    k_contract_split<B, S, L, NE><<<(unsigned)grid, kSplitThreads, smem, ctx->x->stream>>>(p);
+    k_contract_split<B, S, L><<<(unsigned)grid, kSplitThreads, smem, ctx->x->stream>>>(p);
 }
 
-// Element-tile width of the split kernel forced by SLGPU_SPLIT_TILE=32 or 64;
-// 0: picked per group shape by timing (tile_choice).
-static int split_tile_forced()
-{
-    static const int ne = [] {
-        const char* v = std::getenv("SLGPU_SPLIT_TILE");
-        if (v == nullptr)
-            return 0;
-        return std::strcmp(v, "32") == 0 ? 32 : std::strcmp(v, "64") == 0 ? 64 : 0;
-    }();
-    return ne;
-}
-
-// One split-precision contraction of a launch: group, tier, form and where
-// its coefficients, their largest magnitudes and element matrices (and, for a transposed
-// pair, the partner's) are.
+// One split-precision contraction of a step: group, tier and form; its column
+// slices and scales; its coefficients and their largest magnitudes, where they
+// are in memory and still to be sliced (null: sliced already); and its element
+// matrices (for a transposed pair, the partner's too).
 struct SplitJob {
     GroupDev* g;
     int tier;
     bool paired;
+    int8_t* slices;
+    double* colscale;
     const double* C;
     const int32_t* elemtop;
     double* out;
     double* out2;
     bool f32;  // out and out2 hold floats
 };
-
-static std::array<int, 5> split_shape_key(const GroupDev& g, int tier) { return {0, tier, g.ntf, g.ndof, g.ngp}; }
 
 // Column-slice bytes of one group in the scratch (256-byte aligned blocks).
 static size_t split_col_bytes(const GroupDev& g, const GroupDev::Split& sp)
@@ -1709,59 +1697,91 @@ static size_t split_col_bytes(const GroupDev& g, const GroupDev::Split& sp)
 }
 static size_t split_scale_bytes(const GroupDev& g) { return (g.tiles.size() * 64 * 8 + 255) & ~size_t(255); }
 
-template <int B, int S, int NE>
-static void launch_slices(Ctx* ctx, const ColSliceParams& cs)
-{
-    k_slice_cols<B, S, NE><<<grid_for(cs.ntiles * 64, 128), 128, 0, ctx->x->stream>>>(cs);
-}
+static int job_slot(const SplitJob& j) { return j.tier + 2 * (j.paired ? 2 : symmetric_form(*j.g) ? 1 : 0); }
 
-// Column slicing and the tcgen05 contraction of a set of jobs of one tier
-// with element-tile width NE: one slicing launch and one persistent
-// contraction launch per kSplitBatch jobs.  Every job's column slices and
-// scales get their own block of the execution state's scratch.
-static void run_split_jobs(Ctx* ctx, const std::vector<SplitJob>& jobs, int NE)
+// Row operands of the jobs, and a block of the execution state's scratch for
+// the column slices and scales of each.
+static void place_split_jobs(Ctx* ctx, std::vector<SplitJob>& jobs)
 {
-    if (jobs.empty())
-        return;
-    const int tier = jobs[0].tier;
-    size_t colb = 0, expb = 0;
+    size_t colb = 0, scaleb = 0;
     for (const SplitJob& j : jobs) {
-        const GroupDev::Split& sp = ensure_split(ctx, *j.g, tier, j.paired);
+        const GroupDev::Split& sp = ensure_split(ctx, *j.g, j.tier, j.paired);
         colb += split_col_bytes(*j.g, sp);
-        expb += split_scale_bytes(*j.g);
+        scaleb += split_scale_bytes(*j.g);
     }
     {
         ArenaPause keep(*ctx->x);  // per-state scratch, kept between requests
         if (ctx->x->split_cols.bytes() < colb)
             ctx->x->split_cols.alloc(ctx, colb);
-        if (ctx->x->split_colscale.bytes() < expb)
-            ctx->x->split_colscale.alloc(ctx, expb);
+        if (ctx->x->split_colscale.bytes() < scaleb)
+            ctx->x->split_colscale.alloc(ctx, scaleb);
     }
     int8_t* cols = ctx->x->split_cols.as<int8_t>();
-    double* cscale = ctx->x->split_colscale.as<double>();
-    for (size_t b0 = 0; b0 < jobs.size(); b0 += kSplitBatch) {
-        const size_t b1 = std::min(jobs.size(), b0 + kSplitBatch);
+    char* scales = ctx->x->split_colscale.as<char>();
+    for (SplitJob& j : jobs) {
+        j.slices = cols;
+        j.colscale = reinterpret_cast<double*>(scales);
+        cols += split_col_bytes(*j.g, *j.g->split[job_slot(j)]);
+        scales += split_scale_bytes(*j.g);
+    }
+}
+
+// Slices of the jobs whose coefficients are in memory.
+static void slice_split_jobs(Ctx* ctx, const std::vector<SplitJob>& jobs)
+{
+    size_t k = 0;
+    while (k < jobs.size()) {
         ColSliceParams cs{};
-        SplitParams sp{};
-        double slice_bytes = 0, ops = 0;
-        for (size_t k = b0; k < b1; k++) {
+        double bytes = 0;
+        int tier = 0;
+        for (; k < jobs.size() && cs.ngroups < kSplitBatch; k++) {
             const SplitJob& j = jobs[k];
+            if (j.C == nullptr)
+                continue;
             const GroupDev& g = *j.g;
-            const GroupDev::Split& s = *g.split[tier + 2 * (j.paired ? 2 : symmetric_form(g) ? 1 : 0)];
-            const int64_t ntiles = (int64_t)g.tiles.size();
-            const int Q = g.nterms * g.ngp;
+            const GroupDev::Split& s = *g.split[job_slot(j)];
+            tier = j.tier;
             ColSliceGroup& c = cs.g[cs.ngroups++];
             c.C = j.C;
             c.elemtop = j.elemtop;
             c.tiles = g.tiles_d.as<Tile>();
-            c.Q = Q;
+            c.nterms = g.nterms;
+            c.ngp = g.ngp;
             c.Qpad = s.Qpad;
             c.nelem = g.nelem;
-            c.ntiles = ntiles;
-            c.slices = cols;
-            c.colscale = cscale;
+            c.ntiles = (int64_t)g.tiles.size();
+            c.slices = j.slices;
+            c.colscale = j.colscale;
             c.t0 = cs.ntiles;
-            cs.ntiles += ntiles;
+            cs.ntiles += c.ntiles;
+            bytes += 8.0 * g.nterms * g.ngp * g.nelem + 4.0 * g.nelem + (double)split_col_bytes(g, s) + 8.0 * c.ntiles * 64;
+        }
+        if (cs.ngroups == 0)
+            break;
+        const int kt = kstat_start(ctx, "slice_cols", bytes);
+        const unsigned grid = grid_for(cs.ntiles * 64, 128);
+        if (tier == 0)
+            k_slice_cols<8, 6><<<grid, 128, 0, ctx->x->stream>>>(cs);
+        else
+            k_slice_cols<7, 5><<<grid, 128, 0, ctx->x->stream>>>(cs);
+        kstat_stop(ctx, kt);
+        cuda_check(cudaGetLastError(), "k_slice_cols");
+        ctx->launches++;
+    }
+}
+
+// The tcgen05 contraction of a step's jobs (one tier): one persistent launch
+// per kSplitBatch jobs.
+static void contract_split_all(Ctx* ctx, const std::vector<SplitJob>& jobs)
+{
+    for (size_t b0 = 0; b0 < jobs.size(); b0 += kSplitBatch) {
+        const size_t b1 = std::min(jobs.size(), b0 + kSplitBatch);
+        SplitParams sp{};
+        double ops = 0;
+        for (size_t k = b0; k < b1; k++) {
+            const SplitJob& j = jobs[k];
+            const GroupDev& g = *j.g;
+            const GroupDev::Split& s = *g.split[job_slot(j)];
             SplitGroup& G = sp.g[sp.ngroups++];
             G.es = g.ntf * g.ld;
             G.es2 = g.ndof * row_stride(g.ndof, g.ntf);
@@ -1773,47 +1793,28 @@ static void run_split_jobs(Ctx* ctx, const std::vector<SplitJob>& jobs, int NE)
             G.out2 = j.out2;
             G.tiles = g.tiles_d.as<Tile>();
             G.A = s.slices.as<int8_t>();
-            G.B = cols;
+            G.B = j.slices;
             G.rowscale = s.rowscale.as<double>();
-            G.colscale = cscale;
+            G.colscale = j.colscale;
             G.out = j.out;
             G.w0 = sp.nwork;
-            G.nwork = (int64_t)G.ntp * ntiles * (64 / NE);
+            G.nwork = (int64_t)G.ntp * (int64_t)g.tiles.size();
             sp.nwork += G.nwork;
-            const size_t cb = split_col_bytes(g, s);
-            slice_bytes += 8.0 * Q * g.nelem + 4.0 * g.nelem + (double)cb + 8.0 * ntiles * 64;
             // Algorithmic INT8 operations: 2 per product, pairs (a, b) with a + b <= L.
             int pairs = 0;
             for (int a = 1; a <= s.S; a++)
                 for (int bb = 1; bb <= s.S; bb++) pairs += (a + bb <= s.L);
-            ops += 2.0 * pairs * needed_rows(g, j.paired ? 2 : symmetric_form(g) ? 1 : 0) * Q * g.nelem;
-            cols += cb;
-            cscale += split_scale_bytes(g) / 8;
+            ops += 2.0 * pairs * needed_rows(g, job_slot(j) >> 1) * g.nterms * g.ngp * g.nelem;
         }
+        const int tier = jobs[b0].tier;
         sp.error = ctx->x->split_error.as<unsigned int>();
         sp.f32 = jobs[b0].f32 ? 1 : 0;
         sp.next = reinterpret_cast<unsigned long long*>(ctx->x->split_error.as<char>() + 16);
-        const int kt = kstat_start(ctx, "slice_cols", slice_bytes);
-        if (tier == 0 && NE == 64)
-            launch_slices<8, 6, 64>(ctx, cs);
-        else if (tier == 0)
-            launch_slices<8, 6, 32>(ctx, cs);
-        else if (NE == 64)
-            launch_slices<7, 5, 64>(ctx, cs);
-        else
-            launch_slices<7, 5, 32>(ctx, cs);
-        kstat_stop(ctx, kt);
-        cuda_check(cudaGetLastError(), "k_slice_cols");
-        ctx->launches++;
         const int kc = kstat_start(ctx, tier == 0 ? "contract_split" : "contract_split_fp32", ops);
-        if (tier == 0 && NE == 64)
-            launch_split<8, 6, 7, 64>(ctx, sp);
-        else if (tier == 0)
-            launch_split<8, 6, 7, 32>(ctx, sp);
-        else if (NE == 64)
-            launch_split<7, 5, 6, 64>(ctx, sp);
+        if (tier == 0)
+            launch_split<8, 6, 7>(ctx, sp);
         else
-            launch_split<7, 5, 6, 32>(ctx, sp);
+            launch_split<7, 5, 6>(ctx, sp);
         kstat_stop(ctx, kc);
         cuda_check(cudaGetLastError(), "k_contract_split");
         ctx->launches++;
@@ -1853,36 +1854,6 @@ static int pick_by_timing(Ctx* ctx, const std::vector<int>& cand, Run run)
         if (best[c] < 0.97f * best[pick])
             pick = c;
     return cand[pick];
-}
-
-// Element-tile width for a group shape: forced, tuned, or (while graph
-// capture or a request stream prevents timing) 64.
-static int split_ne_of(Ctx* ctx, const GroupDev& g, int tier)
-{
-    if (split_tile_forced() != 0)
-        return split_tile_forced();
-    auto it = ctx->tile_choice.find(split_shape_key(g, tier));
-    return it == ctx->tile_choice.end() ? 64 : it->second;
-}
-
-// All split jobs of one process: shapes without a tuned width are timed
-// first (their jobs at each width), then one launch pair per width.
-static void contract_split_all(Ctx* ctx, const std::vector<SplitJob>& jobs)
-{
-    if (jobs.empty())
-        return;
-    if (split_tile_forced() == 0 && !ctx->x->capturing && ctx->x == &ctx->main) {
-        std::map<std::array<int, 5>, std::vector<SplitJob>> untuned;
-        for (const SplitJob& j : jobs)
-            if (!ctx->tile_choice.count(split_shape_key(*j.g, j.tier)))
-                untuned[split_shape_key(*j.g, j.tier)].push_back(j);
-        for (auto& kv : untuned)
-            ctx->tile_choice[kv.first] = pick_by_timing(ctx, {64, 32}, [&](int ne) { run_split_jobs(ctx, kv.second, ne); });
-    }
-    std::vector<SplitJob> by[2];
-    for (const SplitJob& j : jobs) by[split_ne_of(ctx, *j.g, j.tier) == 32 ? 1 : 0].push_back(j);
-    run_split_jobs(ctx, by[0], 64);
-    run_split_jobs(ctx, by[1], 32);
 }
 
 // Whether a group's contraction runs in split precision: element matrices
@@ -2149,7 +2120,7 @@ static void contract_fp64_all(Ctx* ctx, const std::vector<MmaJob>& jobs)
     }();
     std::vector<MmaJob> by[2];
     for (const MmaJob& j : jobs) {
-        const std::array<int, 5> key{1, 0, j.g->ntf, j.g->ndof, j.g->ngp};
+        const std::array<int, 3> key{j.g->ntf, j.g->ndof, j.g->ngp};
         int bp = forced;
         if (bp == 0) {
             auto it = ctx->tile_choice.find(key);
@@ -2250,106 +2221,213 @@ struct JitGroup {
     double* C;
     int32_t* elemtop;  // nullptr, or per element: atomicMax of the high words of |C|
 };
+struct JitSlice {
+    const double* tables;
+    const double* elemdata;
+    const double* fielddata;
+    const double* term_scale;
+    int8_t* slices;    // nullptr: the group has none in this launch
+    double* colscale;
+};
 
-// Geometry + coefficients of every group into C (offsets coff).  Consecutive
-// groups with the same geometry key run as one runtime-compiled kernel; the
-// interpreter kernel is used when SLGPU_COEF_INTERPRETER=1 or when a kernel
-// cannot be compiled.
-// Groups per runtime-compiled coefficient kernel: their descriptors (48 bytes
-// each) are one by-value kernel parameter.
+// Groups per runtime-compiled kernel: their descriptors (48 bytes each) are
+// one by-value kernel parameter.
 constexpr int kJitBatch = 64;
 
-static void launch_coefficients(Ctx* ctx, const Matrix& M, double* C, const std::vector<int64_t>& coff, int32_t* elemtop,
-                                const std::vector<int64_t>& eoff, const std::vector<GroupData>* ov, const std::vector<int>& pair)
+// The kernel of a batch, remembered by its first group (the source depends
+// only on the batch's groups).
+template <class Source>
+static cudaKernel_t batch_kernel(Ctx* ctx, GroupDev::Jit& jit, const std::vector<const GroupDev*>& batch, const char* name, int smem,
+                                 Source source)
 {
-    // The second group of a transposed pair needs no coefficients.
-    auto skip = [&](size_t j) { return pair[j] >= 0 && pair[j] < (int)j; };
+    std::vector<uint64_t> ids;
+    for (const GroupDev* b : batch) ids.push_back(b->serial);
+    if (jit.kernel == nullptr || jit.members != ids) {
+        jit.kernel = jit_kernel(ctx, source(), name, smem);
+        jit.members = ids;
+    }
+    return jit.kernel;
+}
+
+// How the coefficients of a step are evaluated.  Consecutive groups with the
+// same geometry key run as one runtime-compiled kernel: to slices where the
+// group goes through the split contraction, else to memory.  The interpreter
+// kernel is used when SLGPU_COEF_INTERPRETER=1, when a kernel cannot be
+// compiled, and for elements of lower dimension than the mesh (boundary
+// projections).
+struct CoefPlan {
+    struct Batch {
+        size_t first;                // group whose geometry the kernel takes
+        std::vector<size_t> groups;  // in the order of the kernel's descriptors
+        cudaKernel_t kernel;
+        SliceShape shape;            // slices
+    };
+    std::vector<Batch> slices, coefs;
+    std::vector<char> sliced;       // per group: its slices come from `slices`
+    std::vector<char> interpreted;  // per group: needs the interpreter
+};
+
+// Groups per slicing kernel (20 bytes of static shared memory per group and
+// element), its most dynamic shared memory, and whether a group's values fit
+// it with the fewest elements per block.
+constexpr size_t kSliceBatch = 16;
+constexpr size_t kSliceSmemMax = 190 * 1024;
+static bool slice_fits(const GroupDev& g)
+{
+    const SliceShape sh = slice_shape({&g});
+    return sh.smem <= kSliceSmemMax && (size_t)sh.E * (24 * (size_t)g.ncn + 20 * kSliceBatch) <= 30 * 1024;
+}
+
+// `skip`: groups without coefficients of their own (the second of a
+// transposed pair); they stay in their batch, whose kernel then serves both.
+static CoefPlan coef_plan(Ctx* ctx, const Matrix& M, int precision, const std::vector<char>& skip)
+{
     static const bool interp_only = [] {
         const char* v = std::getenv("SLGPU_COEF_INTERPRETER");
         return v != nullptr && std::strcmp(v, "1") == 0;
     }();
     const size_t ng = M.groups.size();
-    size_t k = 0;
-    while (k < ng) {
+    const int tier = precision == SLGPU_PREC_FP32 ? 1 : 0;
+    CoefPlan P;
+    P.sliced.assign(ng, 0);
+    P.interpreted.assign(ng, 0);
+    for (size_t k = 0, k1; k < ng; k = k1) {
         const GroupDev& g0 = *M.groups[k];
-        size_t k1 = k + 1;
-        while (k1 < ng && k1 - k < kJitBatch && M.groups[k1]->geom_hash == g0.geom_hash) k1++;
-        if (g0.nelem == 0) {
-            k = k1;
+        for (k1 = k + 1; k1 < ng && k1 - k < kJitBatch && M.groups[k1]->geom_hash == g0.geom_hash;) k1++;
+        if (g0.nelem == 0)
             continue;
-        }
+        const size_t ns = P.slices.size(), nc = P.coefs.size();
         bool done = false;
-        // The runtime-compiled kernel covers elements of the mesh dimension;
-        // lower-dimensional ones (boundary projections) use the interpreter.
         if (!interp_only && !ctx->jit_broken && g0.elemdim == g0.problemdim) {
             try {
-                std::vector<const GroupDev*> batch;
-                for (size_t j = k; j < k1; j++) batch.push_back(M.groups[j].get());
-                // The kernel of a batch is remembered by its first group (the
-                // source depends only on the batch's groups).
-                std::vector<uint64_t> ids;
-                for (const GroupDev* b : batch) ids.push_back(b->serial);
-                cudaKernel_t kern = nullptr;
-                if (g0.jit_members == ids)
-                    kern = g0.jit_kernel;
-                else {
-                    kern = jit_coef_kernel(ctx, jit_coef_source(batch));
-                    g0.jit_members = ids;
-                    g0.jit_kernel = kern;
+                std::vector<char> taken(k1 - k, 0);
+                for (size_t a = k; a < k1;) {
+                    CoefPlan::Batch b{k, {}, nullptr, {}};
+                    std::vector<const GroupDev*> list;
+                    bool wanted = false;
+                    for (; a < k1 && list.size() < kSliceBatch; a++) {
+                        const GroupDev& ga = *M.groups[a];
+                        if (!uses_split(ga, precision) || !slice_fits(ga))
+                            continue;
+                        taken[a - k] = 1;
+                        b.groups.push_back(a);
+                        list.push_back(&ga);
+                        wanted = wanted || !skip[a];
+                    }
+                    if (!wanted)
+                        continue;
+                    b.shape = slice_shape(list);
+                    b.kernel = batch_kernel(ctx, list[0]->jit_slice[tier], list, "slgpu_slices", (int)kSliceSmemMax,
+                                            [&] { return jit_slice_source(list, tier); });
+                    P.slices.push_back(std::move(b));
                 }
-                std::vector<JitGroup> jg;
-                for (size_t j = k; j < k1; j++) {
-                    GroupDev& G = *M.groups[j];
-                    const double* ed = ov != nullptr && (*ov)[j].elemdata != nullptr ? (*ov)[j].elemdata : G.elemdata.as<double>();
-                    const double* fd = ov != nullptr && (*ov)[j].fielddata != nullptr ? (*ov)[j].fielddata : G.fielddata.as<double>();
-                    const double* ts = ov != nullptr && (*ov)[j].term_scale != nullptr ? (*ov)[j].term_scale : G.term_scale_d.as<double>();
-                    jg.push_back(JitGroup{G.tables.as<double>(), ed, fd, ts, skip(j) ? nullptr : C + coff[j],
-                                          eoff[j] >= 0 && !skip(j) ? elemtop + eoff[j] : nullptr});
+                bool rest = false;
+                for (size_t a = k; a < k1; a++) rest = rest || (!taken[a - k] && !skip[a]);
+                if (rest) {
+                    CoefPlan::Batch b{k, {}, nullptr, {}};
+                    std::vector<const GroupDev*> list;
+                    for (size_t a = k; a < k1; a++) {
+                        b.groups.push_back(a);
+                        list.push_back(M.groups[a].get());
+                    }
+                    b.kernel = batch_kernel(ctx, g0.jit_coef, list, "slgpu_coef", 0, [&] { return jit_coef_source(list); });
+                    P.coefs.push_back(std::move(b));
                 }
-                const MeshDev& m = ctx->meshes.at(g0.mesh);
-                JitGeom geom{m.xyz.as<double>(), m.types.at(g0.elemtype).conn.as<int32_t>(), g0.elems.as<int32_t>(), g0.orient.as<int32_t>(),
-                             (long long)g0.nelem, g0.weights.as<double>(), g0.lagrange.as<double>()};
-                void* args[] = {&geom, jg.data()};  // the group array is one by-value parameter
-                const int64_t n = g0.nelem * (int64_t)g0.ngp;
-                double cbytes = 0;
-                for (size_t j = k; j < k1; j++)
-                    if (!skip(j))
-                        cbytes += 8.0 * M.groups[j]->nterms * M.groups[j]->ngp * M.groups[j]->nelem;
-                const int kt = kstat_start(ctx, "coefficients", cbytes);
-                cuda_check(cudaLaunchKernel((const void*)kern, dim3(grid_for(n, 128)), dim3(128), args, 0, ctx->x->stream),
-                           "coefficient kernel launch");
-                kstat_stop(ctx, kt);
-                ctx->launches++;
+                for (size_t a = k; a < k1; a++) P.sliced[a] = taken[a - k];
                 done = true;
             } catch (const SlgpuException&) {
                 throw;
             } catch (const std::exception& e) {
                 ctx->jit_broken = true;
                 ctx->jit_error = e.what();
+                P.slices.resize(ns);
+                P.coefs.resize(nc);
             }
         }
-        if (!done) {
-            for (size_t j = k; j < k1; j++) {
-                if (skip(j))
-                    continue;
-                GroupDev& G = *M.groups[j];
-                CoefParams cp = coef_params(ctx, G, C + coff[j]);
-                cp.elemtop = eoff[j] >= 0 ? elemtop + eoff[j] : nullptr;
-                if (ov != nullptr && (*ov)[j].elemdata != nullptr)
-                    cp.elemdata = (*ov)[j].elemdata;
-                if (ov != nullptr && (*ov)[j].fielddata != nullptr)
-                    cp.fielddata = (*ov)[j].fielddata;
-                if (ov != nullptr && (*ov)[j].term_scale != nullptr)
-                    cp.term_scale = (*ov)[j].term_scale;
-                const int64_t n = G.nelem * (int64_t)G.ngp;
-                const int kt = kstat_start(ctx, "coefficients", 8.0 * G.nterms * G.ngp * G.nelem);
-                k_geometry_coef<<<grid_for(n, 128), 128, 0, ctx->x->stream>>>(cp);
-                kstat_stop(ctx, kt);
-                cuda_check(cudaGetLastError(), "k_geometry_coef");
-                ctx->launches++;
+        if (!done)
+            for (size_t a = k; a < k1; a++) P.interpreted[a] = skip[a] ? 0 : 1;
+    }
+    return P;
+}
+
+// Coefficients of the planned groups: to the slices of their jobs (job[j],
+// null: none), or into C at coff[j] (coff[j] < 0: not needed there), with the
+// largest magnitudes of split groups in elemtop at eoff[j] (eoff[j] >= 0).
+static void launch_coefficients(Ctx* ctx, const Matrix& M, const CoefPlan& plan, const std::vector<const SplitJob*>& job, double* C,
+                                const std::vector<int64_t>& coff, int32_t* elemtop, const std::vector<int64_t>& eoff,
+                                const std::vector<GroupData>* ov)
+{
+    auto elemdata = [&](size_t j) {
+        return ov != nullptr && (*ov)[j].elemdata != nullptr ? (*ov)[j].elemdata : M.groups[j]->elemdata.as<double>();
+    };
+    auto fielddata = [&](size_t j) {
+        return ov != nullptr && (*ov)[j].fielddata != nullptr ? (*ov)[j].fielddata : M.groups[j]->fielddata.as<double>();
+    };
+    auto scales = [&](size_t j) {
+        return ov != nullptr && (*ov)[j].term_scale != nullptr ? (*ov)[j].term_scale : M.groups[j]->term_scale_d.as<double>();
+    };
+    auto geometry = [&](const GroupDev& g) {
+        const MeshDev& m = ctx->meshes.at(g.mesh);
+        return JitGeom{m.xyz.as<double>(), m.types.at(g.elemtype).conn.as<int32_t>(), g.elems.as<int32_t>(), g.orient.as<int32_t>(),
+                       (long long)g.nelem, g.weights.as<double>(), g.lagrange.as<double>()};
+    };
+    for (const CoefPlan::Batch& b : plan.slices) {
+        const GroupDev& g0 = *M.groups[b.first];
+        JitGeom geom = geometry(g0);
+        const void* tiles = g0.tiles_d.as<void>();
+        std::vector<JitSlice> js;
+        double bytes = 0;
+        for (size_t j : b.groups) {
+            const SplitJob* sj = job[j];
+            if (sj == nullptr) {
+                js.push_back(JitSlice{});
+                continue;
             }
+            js.push_back(JitSlice{M.groups[j]->tables.as<double>(), elemdata(j), fielddata(j), scales(j), sj->slices, sj->colscale});
+            bytes += (double)split_col_bytes(*sj->g, *sj->g->split[job_slot(*sj)]) + 8.0 * sj->g->tiles.size() * 64;
         }
-        k = k1;
+        void* args[] = {&geom, js.data(), &tiles};  // the group array is one by-value parameter
+        const int kt = kstat_start(ctx, "slice_cols", bytes);
+        cuda_check(cudaLaunchKernel((const void*)b.kernel, dim3((unsigned)(g0.tiles.size() * (64 / b.shape.E))),
+                                    dim3((unsigned)b.shape.threads), args, b.shape.smem, ctx->x->stream),
+                   "slicing kernel launch");
+        kstat_stop(ctx, kt);
+        ctx->launches++;
+    }
+    for (const CoefPlan::Batch& b : plan.coefs) {
+        const GroupDev& g0 = *M.groups[b.first];
+        std::vector<JitGroup> jg;
+        double bytes = 0;
+        for (size_t j : b.groups) {
+            const GroupDev& G = *M.groups[j];
+            jg.push_back(JitGroup{G.tables.as<double>(), elemdata(j), fielddata(j), scales(j), coff[j] >= 0 ? C + coff[j] : nullptr,
+                                  eoff[j] >= 0 ? elemtop + eoff[j] : nullptr});
+            if (coff[j] >= 0)
+                bytes += 8.0 * G.nterms * G.ngp * G.nelem;
+        }
+        JitGeom geom = geometry(g0);
+        void* args[] = {&geom, jg.data()};  // the group array is one by-value parameter
+        const int kt = kstat_start(ctx, "coefficients", bytes);
+        cuda_check(cudaLaunchKernel((const void*)b.kernel, dim3(grid_for(g0.nelem * (int64_t)g0.ngp, 128)), dim3(128), args, 0, ctx->x->stream),
+                   "coefficient kernel launch");
+        kstat_stop(ctx, kt);
+        ctx->launches++;
+    }
+    for (size_t j = 0; j < M.groups.size(); j++) {
+        if (!plan.interpreted[j])
+            continue;
+        GroupDev& G = *M.groups[j];
+        CoefParams cp = coef_params(ctx, G, C + coff[j]);
+        cp.elemtop = eoff[j] >= 0 ? elemtop + eoff[j] : nullptr;
+        cp.elemdata = elemdata(j);
+        cp.fielddata = fielddata(j);
+        cp.term_scale = scales(j);
+        const int64_t n = G.nelem * (int64_t)G.ngp;
+        const int kt = kstat_start(ctx, "coefficients", 8.0 * G.nterms * G.ngp * G.nelem);
+        k_geometry_coef<<<grid_for(n, 128), 128, 0, ctx->x->stream>>>(cp);
+        kstat_stop(ctx, kt);
+        cuda_check(cudaGetLastError(), "k_geometry_coef");
+        ctx->launches++;
     }
 }
 
@@ -2369,16 +2447,6 @@ bool float_values(const Matrix& M, int precision)
 void launch_contractions(Ctx* ctx, const Matrix& M, int precision, const std::vector<int64_t>& gvb, double* vals,
                          const std::vector<GroupData>* ov, bool f32)
 {
-    // Coefficients of every group coexist ([term][gp][element] per group) so
-    // that groups sharing geometry are evaluated by one kernel.
-    std::vector<int64_t> coff(M.groups.size());
-    int64_t ctot = 0;
-    for (size_t k = 0; k < M.groups.size(); k++) {
-        coff[k] = ctot;
-        ctot += (int64_t)M.groups[k]->nterms * M.groups[k]->ngp * M.groups[k]->nelem;
-    }
-    DevBuf C;
-    C.alloc(ctx, std::max<int64_t>(ctot, 1) * 8);
     if (precision != SLGPU_PREC_FP64) {
         if (ctx->x->split_error.empty()) {
             ArenaPause keep(*ctx->x);
@@ -2391,46 +2459,67 @@ void launch_contractions(Ctx* ctx, const Matrix& M, int precision, const std::ve
         cuda_check(cudaEventCreate(&e), "cudaEventCreate");
         ctx->x->evpool.push_back(e);
     }
-    // Split-precision groups: the high word of each element's largest
-    // coefficient, gathered by the coefficient kernels (atomicMax from 0).
-    std::vector<int64_t> eoff(M.groups.size(), -1);
-    int64_t etot = 0;
-    for (size_t k = 0; k < M.groups.size(); k++)
-        if (uses_split(*M.groups[k], precision)) {
+    const std::vector<int> pair = cross_pairs(M, precision, ov);
+    const size_t ng = M.groups.size();
+    // The second group of a transposed pair is written by the first's
+    // contraction and needs no coefficients.
+    std::vector<char> skip(ng);
+    for (size_t k = 0; k < ng; k++) skip[k] = M.groups[k]->nelem == 0 || (pair[k] >= 0 && pair[k] < (int)k) ? 1 : 0;
+    const CoefPlan plan = coef_plan(ctx, M, precision, skip);
+    // Split precision for the larger element matrices (order >= 2);
+    // right-hand sides and small matrices stay in FP64.
+    std::vector<SplitJob> split_jobs;  // every split-precision group of the step, contracted together
+    std::vector<const SplitJob*> job(ng, nullptr);
+    split_jobs.reserve(ng);
+    for (size_t k = 0; k < ng; k++)
+        if (!skip[k] && uses_split(*M.groups[k], precision)) {
+            split_jobs.push_back(SplitJob{M.groups[k].get(), precision == SLGPU_PREC_SPLIT ? 0 : 1, pair[k] >= 0, nullptr, nullptr, nullptr,
+                                          nullptr, vals + gvb[k], pair[k] >= 0 ? vals + gvb[pair[k]] : nullptr, f32});
+            job[k] = &split_jobs.back();
+        }
+    place_split_jobs(ctx, split_jobs);
+    // Coefficients that go through memory ([term][gp][element] per group,
+    // all groups side by side), and the high words of the largest ones of
+    // each element (atomicMax from 0) where they are still to be sliced.
+    std::vector<int64_t> coff(ng, -1), eoff(ng, -1);
+    int64_t ctot = 0, etot = 0;
+    for (size_t k = 0; k < ng; k++) {
+        if (skip[k] || plan.sliced[k])
+            continue;
+        coff[k] = ctot;
+        ctot += (int64_t)M.groups[k]->nterms * M.groups[k]->ngp * M.groups[k]->nelem;
+        if (job[k] != nullptr) {
             eoff[k] = etot;
             etot += M.groups[k]->nelem;
         }
-    DevBuf E;
+    }
+    DevBuf C, E;
+    if (ctot > 0)
+        C.alloc(ctx, (size_t)ctot * 8);
     if (etot > 0) {
         E.alloc(ctx, (size_t)etot * 4);
         cuda_check(cudaMemsetAsync(E.as<void>(), 0, (size_t)etot * 4, ctx->x->stream), "memset");
     }
-    const std::vector<int> pair = cross_pairs(M, precision, ov);
+    for (size_t k = 0, n = 0; k < ng; k++)
+        if (job[k] != nullptr) {
+            SplitJob& j = split_jobs[n++];
+            if (coff[k] >= 0) {
+                j.C = C.as<double>() + coff[k];
+                j.elemtop = E.as<int32_t>() + eoff[k];
+            }
+        }
     phase_event(ctx, ctx->x->evpool[0]);
-    launch_coefficients(ctx, M, C.as<double>(), coff, E.as<int32_t>(), eoff, ov, pair);
+    launch_coefficients(ctx, M, plan, job, C.as<double>(), coff, E.as<int32_t>(), eoff, ov);
     phase_event(ctx, ctx->x->evpool[1]);
     size_t gi = 0;
-    std::vector<SplitJob> split_jobs;  // every split-precision group of the step, contracted together
     std::vector<MmaJob> mma_jobs;      // every FP64 group that the small kernel does not take, likewise
     for (auto& g : M.groups) {
         if (g->nelem > 0) {
-            double* Cg = C.as<double>() + coff[gi];
-            // Split precision for the larger element matrices (order >= 2);
-            // right-hand sides and small matrices stay in FP64.  The second
-            // group of a transposed pair is written by the first's contraction.
-            if (uses_split(*g, precision)) {
-                if (pair[gi] < 0 || pair[gi] > (int)gi)
-                    split_jobs.push_back(SplitJob{g.get(), precision == SLGPU_PREC_SPLIT ? 0 : 1, pair[gi] > (int)gi, Cg,
-                                                  E.as<int32_t>() + eoff[gi], vals + gvb[gi],
-                                                  pair[gi] > (int)gi ? vals + gvb[pair[gi]] : nullptr, f32});
+            if (skip[gi] || job[gi] != nullptr) {
                 gi++;
                 continue;
             }
-            // The second group of a transposed pair is written by the first's contraction.
-            if (pair[gi] >= 0 && pair[gi] < (int)gi) {
-                gi++;
-                continue;
-            }
+            const double* Cg = C.as<double>() + coff[gi];
             if (f32)
                 fail(SLGPU_E_STATE, "float element values need every group contracted by the split kernels");
             const int64_t P = (int64_t)g->ntf * g->ndof;
@@ -2464,6 +2553,7 @@ void launch_contractions(Ctx* ctx, const Matrix& M, int precision, const std::ve
         gi++;
     }
     contract_fp64_all(ctx, mma_jobs);
+    slice_split_jobs(ctx, split_jobs);
     contract_split_all(ctx, split_jobs);
     phase_event(ctx, ctx->x->evpool[2]);
     C.release();
@@ -2743,6 +2833,13 @@ void prepare_value_path(Ctx* ctx, const Matrix& M, int precision)
         x.split_error.alloc(ctx, 32);
 }
 
+void compile_value_path(Ctx* ctx, const Matrix& M, int precision)
+{
+    std::vector<char> none(M.groups.size());
+    for (size_t gi = 0; gi < M.groups.size(); gi++) none[gi] = M.groups[gi]->nelem == 0 ? 1 : 0;
+    coef_plan(ctx, M, precision, none);
+}
+
 ValueGraph::~ValueGraph()
 {
     if (exec != nullptr)
@@ -2774,7 +2871,6 @@ static std::vector<uint64_t> value_signature(Ctx* ctx, const Matrix& M, int prec
     p(M.Avals.as<void>());
     p(M.Dvals.as<void>());
     p(M.rsegs_dev.as<void>());
-    u((uint64_t)split_tile_forced());
     u((uint64_t)ctx->nsm);
     u(ctx->timers ? 1 : 0);
     u(ctx->jit_broken ? 1 : 0);
@@ -2786,13 +2882,15 @@ static std::vector<uint64_t> value_signature(Ctx* ctx, const Matrix& M, int prec
     for (auto& gp : M.groups) {
         const GroupDev& g = *gp;
         u(g.serial);
-        p(g.jit_kernel);
-        u(g.jit_members.size());
-        for (uint64_t id : g.jit_members) u(id);
+        for (const GroupDev::Jit* jit : {&g.jit_coef, &g.jit_slice[0], &g.jit_slice[1]}) {
+            p(jit->kernel);
+            u(jit->members.size());
+            for (uint64_t id : jit->members) u(id);
+        }
         u(symmetric_form(g) ? 1 : 0);
         u((uint64_t)(pair[gi++] + 1));
-        for (int t = 0; t < 2; t++) {
-            auto it = ctx->tile_choice.find(split_shape_key(g, t));
+        {
+            auto it = ctx->tile_choice.find({g.ntf, g.ndof, g.ngp});
             u(it == ctx->tile_choice.end() ? 0 : (uint64_t)it->second);
         }
         for (int t = 0; t < 6; t++) {
@@ -3177,9 +3275,8 @@ int slgpu_tuned_tiles(slgpu_ctx* ctx, char* buf, size_t len)
         std::string t;
         for (const auto& kv : ctx->tile_choice) {
             const auto& k = kv.first;
-            t += (k[0] == 0 ? std::string("split tier ") + std::to_string(k[1]) + " NE=" : std::string("fp64 rows/block="));
-            t += std::to_string(kv.second) + " for ntf " + std::to_string(k[2]) + " ndof " + std::to_string(k[3]) + " ngp " +
-                 std::to_string(k[4]) + "\n";
+            t += "fp64 rows/block=" + std::to_string(kv.second) + " for ntf " + std::to_string(k[0]) + " ndof " + std::to_string(k[1]) +
+                 " ngp " + std::to_string(k[2]) + "\n";
         }
         for (const auto& p : ctx->patterns)
             if (p)
@@ -3467,8 +3564,14 @@ int slgpu_check_coefficient_kernels(slgpu_ctx* ctx, int handle, char* log, size_
             std::vector<const GroupDev*> batch;
             for (size_t j = k; j < k1; j++) batch.push_back(M.groups[j].get());
             try {
-                if (M.groups[k]->elemdim == M.groups[k]->problemdim)
+                if (M.groups[k]->elemdim == M.groups[k]->problemdim) {
                     jit_compile(jit_coef_source(batch));
+                    std::vector<const GroupDev*> sliced;
+                    for (const GroupDev* g : batch)
+                        if (sliced.size() < kSliceBatch && uses_split(*g, SLGPU_PREC_SPLIT) && slice_fits(*g))
+                            sliced.push_back(g);
+                    for (int tier = 0; tier < 2 && !sliced.empty(); tier++) jit_compile(jit_slice_source(sliced, tier));
+                }
             } catch (const std::exception& e) {
                 fail(SLGPU_E_CUDA, e.what());
             }

@@ -102,10 +102,13 @@ struct GroupDev {
     std::vector<double> hconsts;
     uint64_t geom_hash = 0;
     uint64_t serial = 0;  // unique per group created by the context
-    // Runtime-compiled coefficient kernel of the batch this group leads
-    // (batch members by serial).
-    mutable std::vector<uint64_t> jit_members;
-    mutable cudaKernel_t jit_kernel = nullptr;
+    // Runtime-compiled kernels of the batch this group leads (batch members
+    // by serial).
+    struct Jit {
+        std::vector<uint64_t> members;
+        cudaKernel_t kernel = nullptr;
+    };
+    mutable Jit jit_coef, jit_slice[2];  // coefficients; slices per tier
 
     DevBuf elems, orient, weights, lagrange, tables, consts, prog_d, elemdata, fielddata, field_off_d, field_rows_d,
         tab_off_d, tab_rows_d, term_scale_d, term_tf_d, term_dof_d, tiles_d;
@@ -320,10 +323,9 @@ struct Ctx {
     std::recursive_mutex mu;  // one thread at a time inside the context
     std::string last_error;
     int64_t bytes_h2d = 0, bytes_d2h = 0;  // host <-> device bytes copied by the context's calls
-    // Tile shapes picked by timing on first use, per contraction kind and
-    // group shape {kind (0 split, 1 FP64), tier, ntf, ndof, ngp}: the split
-    // kernel's element-tile width NE, the FP64 kernel's rows per block.
-    std::map<std::array<int, 5>, int> tile_choice;
+    // Rows per block of the FP64 contraction, picked by timing on first use
+    // per group shape {ntf, ndof, ngp}.
+    std::map<std::array<int, 3>, int> tile_choice;
     std::map<int, MeshDev> meshes;
     std::map<int, std::unique_ptr<Matrix>> matrices;
     int next_handle = 1;
@@ -413,12 +415,22 @@ void htrace_mark(Ctx* ctx, const char* label);
 // current execution state's split scratch grown to fit them, so that the
 // value path allocates nothing for them.
 void prepare_value_path(Ctx* ctx, const Matrix& M, int precision);
+// Compiles the runtime kernels that the value path takes at this precision.
+void compile_value_path(Ctx* ctx, const Matrix& M, int precision);
 void kstat_stop(Ctx* ctx, int i);
 void kstat_collect(Ctx* ctx);
 
 // Runtime-compiled coefficient kernels (coef_jit.cu).
 std::string jit_coef_source(const std::vector<const GroupDev*>& batch);
-cudaKernel_t jit_coef_kernel(Ctx* ctx, const std::string& src);
+struct SliceShape {
+    int E = 0, round = 0, threads = 0;  // elements per block, groups per round, threads
+    bool single = false;                // one point of one element per thread
+    size_t smem = 0;                    // dynamic shared memory
+};
+SliceShape slice_shape(const std::vector<const GroupDev*>& batch);
+std::string jit_slice_source(const std::vector<const GroupDev*>& batch, int tier);
+// Cached by source; `smem`: most dynamic shared memory of a launch.
+cudaKernel_t jit_kernel(Ctx* ctx, const std::string& src, const char* name, int smem = 0);
 std::vector<char> jit_compile(const std::string& src);  // NVRTC only, no device needed
 
 }  // namespace slgpu

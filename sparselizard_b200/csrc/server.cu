@@ -797,6 +797,7 @@ int slgpu_server_prepare(slgpu_server* S, int handle, int precision)
         const size_t est = (size_t)estimate_bytes(M, precision, nullptr);
         for (Slot& s : S->slots) {
             ctx->x = &s.ex;
+            compile_value_path(ctx, M, precision);
             prepare_value_path(ctx, M, precision);
             const size_t want = std::max(s.arena_need, est);
             if (s.ex.arena.bytes() < want)

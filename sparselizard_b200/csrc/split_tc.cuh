@@ -24,22 +24,23 @@
 // the products bound: 1725 -> 1451 us.
 //
 // Level accumulators sit side by side in TMEM (level l at columns
-// NE(l-2) .. NE(l-2)+NE-1 for an element tile of NE columns), and the column
+// NE(l-2) .. NE(l-2)+NE-1, NE = 64 elements), and the column
 // slices of one K step sit side by side in shared memory, so A slice a times
 // the concatenation [c_1 | ... | c_k] (N = NE k <= 256) writes every pair
 // (a, b) straight into level a+b's columns: for S = 6, 8 MMAs per K step
-// (NE = 64) or 6 (NE = 32) instead of 21.
+// instead of 21.
 //
 // Operands live in global memory already in the interleaved K-major layout
 // that the UMMA "no swizzle" canonical form expects, blocked so that one K
 // step of one tile is a single contiguous range (one bulk copy per operand):
 //   A (rows of M):    [orient][ptile][kstep][slice][2][128][16 bytes]
-//   B (columns of C): [unit][kstep][2][slice][NE][16 bytes]
+//   B (columns of C): [tile][kstep][2][slice][NE][16 bytes]
 // A core matrix (8 rows x 16 bytes) is 128 contiguous bytes; 8-row groups are
 // SBO = 128 bytes apart, the two 16-byte K chunks of a step LBO bytes apart.
 #pragma once
 
 #include "engine_internal.h"
+#include "split_digits.cuh"
 
 #include <cstdint>
 
@@ -52,23 +53,20 @@ constexpr int kSplitEpiWarps = 16;  // 4 per TMEM lane quarter, 16 columns each
 constexpr int kSplitThreads = 64 + 32 * kSplitEpiWarps;
 constexpr int kSplitABytes = 2 * kSplitM * 16;  // one slice of one K step of A
 
-// Element-tile width NE (columns of one accumulator level) and what follows
-// from it.  NE = 64: one accumulator (6 levels x 64 = 384 TMEM columns), the
-// epilogue of a tile runs between its MMAs and the next tile's.  NE = 32: two
-// accumulators (2 x 192 columns), the epilogue of one tile overlaps the MMAs
-// of the next; A (the rows of M) is read twice as often per element.
-template <int NE>
-struct SplitShape {
-    static constexpr int kUnits = 64 / NE;               // element tiles per 64-element tile
-    static constexpr int kBufs = NE == 32 ? 2 : 1;       // TMEM accumulators
-    static constexpr int kStages = NE == 32 ? 7 : 6;     // shared-memory pipeline depth
-    static constexpr int kBBytes = 2 * NE * 16;          // one slice of one K step of B
-    static constexpr int kGroup = 256 / NE;              // B slices per MMA (N <= 256)
-};
+// Elements per tile: the columns of one accumulator level.  Six levels of 64
+// fill 384 of the 512 TMEM columns, so there is one accumulator, and a tile's
+// MMAs wait until the one before has been read.  Two accumulators of 32
+// columns need no such wait, but A (the rows of M) is read twice as often and
+// the MMAs are half as wide: 1.4 times slower with long K, no faster with
+// short.
+constexpr int kSplitNE = 64;
+constexpr int kSplitStages = 6;                // shared-memory pipeline depth
+constexpr int kSplitBBytes = 2 * kSplitNE * 16;  // one slice of one K step of B
+constexpr int kSplitGroupB = 256 / kSplitNE;   // B slices per MMA (N <= 256)
 
 // One group of a batched contraction launch.  Its work items are
 // [w0, w0 + nwork) of the launch: item w0 + v is row tile v % ntp of element
-// unit v / ntp.
+// tile v / ntp.
 struct SplitGroup {
     int Ppad, ntp, nk;      // padded rows, row tiles, K steps
     int nrows;              // rows of A computed
@@ -77,7 +75,7 @@ struct SplitGroup {
                             // out, and its mirror in out2, or out (-1: nowhere); null:
                             // row r is value r, without a mirror
     double* out2;           // null, or the transposed partner group's element matrices
-    const Tile* tiles;      // 64-element tiles; unit u = tile u / kUnits, part u % kUnits
+    const Tile* tiles;      // [nwork / ntp]
     const int8_t* A;        // row slices
     const int8_t* B;        // column slices
     const double* rowscale;  // [norient][Ppad]: R_p 2^-(B L)
@@ -110,18 +108,10 @@ __device__ __forceinline__ int split_group_of(const SplitParams& p, int gi, int6
     return gi;
 }
 
-// Elements [e0, e0 + ne) and orientation of element unit u (ne <= 0: empty).
-template <int NE>
-__device__ __forceinline__ Tile split_unit(const Tile* tiles, int64_t u)
-{
-    Tile t = tiles[u / SplitShape<NE>::kUnits];
-    const int part = (int)(u % SplitShape<NE>::kUnits) * NE;
-    t.e0 += part;
-    t.ne = min(t.ne - part, NE);
-    return t;
-}
-
 // ---------------------------------------------------------------- slicing
+
+// Order of K: q = g nterms + t, the terms of a Gauss point side by side (the
+// slicing kernel has them in one thread).
 
 // Row slices of M for one orientation: block per row p, threads over q.
 // M[p][q] = T_t[o][i][g] * D_t[o][j][g] as in the FP64 contraction.
@@ -139,79 +129,16 @@ struct RowSliceParams {
     double* rowscale; // [norient][Ppad]
 };
 
-// Scale of a row or column from the high word h of the largest magnitude in
-// it: *q, the value that 2^(B S) units stand for (R and Q above), and the
-// factor that turns a value into those units.
-//   B = 8: |x| < the double of high word h + 1, so |x| / Q < 0.498 and its S
-//   balanced digits represent it (the largest such number is 0.49804);
-//   B = 7: the power of two above |x|.
-// Magnitudes below 2^-900 take a power of two and a factor below the
-// overflow: *pre, by which values are multiplied first (1 otherwise).
-// Nothing set (h = 0): digits and scale are zero.  Infinities and NaN (h from
-// 0x7ff00000): the scale is NaN, so that the results are.
-template <int B, int S>
-__device__ __forceinline__ double split_scale(int h, double* q, double* pre)
-{
-    const double unit = __longlong_as_double((long long)(1023 + B * S) << 52);  // 2^(B S)
-    *pre = 1.0;
-    if (h <= 0) {
-        *q = 0.0;
-        return 0.0;
-    }
-    if (h >= 0x7ff00000) {
-        *q = __longlong_as_double(0x7ff8000000000000ll);
-        return 0.0;
-    }
-    const bool tiny = h < (1023 - 900) << 20;
-    if (tiny || B == 7) {
-        int ex;
-        frexp(__hiloint2double(h, -1), &ex);  // |x| < 2^ex
-        ex += B == 7 ? 0 : 2;
-        *q = ldexp(1.0, ex);
-        *pre = tiny ? 0x1p512 : 1.0;
-        return ldexp(unit, -ex - (tiny ? 512 : 0));
-    }
-    const double top = h >= 0x7fefffff ? __longlong_as_double(0x7fefffffffffffffll) : __hiloint2double(h + 1, 0);
-    *q = top * (1.0 / 0.498);
-    return 0.498 * unit / top;
-}
-
-// The S digits of x in units of 1 / f, byte k the digit S - 1 - k.
-// B = 8, each plus 128: 1.5 2^52 + rint(x f) holds the integer in its low
-// bits, and adding 128 to every digit makes them all non-negative.
-// B = 7, two's complement: the 7-bit fields of |x| f truncated, with x's sign.
-template <int B, int S>
-__device__ __forceinline__ unsigned long long split_digits(double x, double f)
-{
-    if constexpr (B == 8) {
-        constexpr unsigned long long kBias = 0x8080808080808080ull >> (8 * (8 - S));
-        return (unsigned long long)__double_as_longlong(fma(x, f, 0x1.8p52)) + kBias;
-    } else {
-        const unsigned long long mag = __double2ull_rz(fabs(x) * f);
-        unsigned long long u = 0;
-#pragma unroll
-        for (int k = 0; k < S; k++) {
-            const int d = (int)((mag >> (7 * k)) & 127);
-            u |= (unsigned long long)(uint8_t)(int8_t)(x < 0 ? -d : d) << (8 * k);
-        }
-        return u;
-    }
-}
-// What turns a byte of split_digits into the signed digit.
-template <int B>
-__host__ __device__ constexpr uint32_t split_flip() { return B == 8 ? 0x80808080u : 0u; }
-
 // M[pe][q] (pe < 0: zero).
 __device__ __forceinline__ double m_entry(const RowSliceParams& p, int o, int pe, int q)
 {
-    const int Q = p.nterms * p.ngp;
-    if (q >= Q || pe < 0)
+    const int g = q / p.nterms, t = q - g * p.nterms, ngp = p.ngp;
+    if (pe < 0 || g >= ngp)
         return 0.0;
-    const int t = q / p.ngp, g = q - t * p.ngp;
     const int i = pe / p.ndof, j = pe - i * p.ndof;
-    const double tv = p.tables[p.tab_off[p.term_tf[t]] + ((int64_t)o * p.ntf + i) * p.ngp + g];
+    const double tv = p.tables[p.tab_off[p.term_tf[t]] + ((int64_t)o * p.ntf + i) * ngp + g];
     const int dt = p.term_dof[t];
-    const double dv = dt >= 0 ? p.tables[p.tab_off[dt] + ((int64_t)o * p.ndof + j) * p.ngp + g] : 1.0;
+    const double dv = dt >= 0 ? p.tables[p.tab_off[dt] + ((int64_t)o * p.ndof + j) * ngp + g] : 1.0;
     return tv * dv;
 }
 
@@ -244,19 +171,19 @@ __global__ void k_slice_rows(RowSliceParams p)
     }
 }
 
-// Column slices of C: thread per (64-element tile, slot); C[q][e] is read
+// Column slices of coefficients in memory: thread per (64-element tile, slot); C[q][e] is read
 // once, coalesced over the tile's consecutive elements, and 16-byte chunks
 // are written coalesced over slots.  The high word of each element's largest
 // |C[q][e]| comes from the coefficient kernel.  Empty slots get zero slices.
-// About 8 instructions per coefficient (one fma, the bias, byte permutes):
-// HBM-bound.
+// For groups whose coefficients the runtime-compiled slicing kernel
+// (jit_slice_source) cannot evaluate.
 struct ColSliceGroup {
     const double* C;  // [Q][nelem]
     const int32_t* elemtop;  // [nelem]; 0: the column is zero
     const Tile* tiles;
-    int Q, Qpad;
+    int nterms, ngp, Qpad;
     int64_t nelem, ntiles;
-    int8_t* slices;   // [unit][kstep][2][S][NE][16]
+    int8_t* slices;   // [tile][kstep][2][S][64][16]
     double* colscale; // [ntiles][64]
     int64_t t0;       // first tile of the group in the launch
 };
@@ -267,22 +194,7 @@ struct ColSliceParams {
     int64_t ntiles;   // sum over the groups
 };
 
-// Word k4 of each slice: digit s of four values as signed bytes.
 template <int B, int S>
-__device__ __forceinline__ void split_words(const unsigned long long (&u)[4], uint32_t (&w)[S][4], int k4)
-{
-#pragma unroll
-    for (int s = 0; s < S; s++) {
-        const int b = S - 1 - s;  // byte of the digit
-        const uint32_t sel = (uint32_t)((b & 3) | ((b & 3) + 4) << 4);
-        uint32_t v[4];
-#pragma unroll
-        for (int k = 0; k < 4; k++) v[k] = b < 4 ? (uint32_t)u[k] : (uint32_t)(u[k] >> 32);
-        w[s][k4] = __byte_perm(__byte_perm(v[0], v[1], sel), __byte_perm(v[2], v[3], sel), 0x5410) ^ split_flip<B>();
-    }
-}
-
-template <int B, int S, int NE>
 __global__ void k_slice_cols(const __grid_constant__ ColSliceParams pb)
 {
     const int64_t gt = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -301,15 +213,14 @@ __global__ void k_slice_cols(const __grid_constant__ ColSliceParams pb)
     const double f = split_scale<B, S>(valid ? p.elemtop[e] : 0, &unit, &pre);
     p.colscale[t * 64 + slot] = unit;
     const int nchunk = p.Qpad / 16;
-    const int64_t u0 = t * SplitShape<NE>::kUnits + slot / NE;
-    uint4* out = reinterpret_cast<uint4*>(p.slices) + u0 * (int64_t)nchunk * S * NE + slot % NE;
+    uint4* out = reinterpret_cast<uint4*>(p.slices) + t * (int64_t)nchunk * S * kSplitNE + slot;
     const double* col = p.C + e;
     for (int c = 0; c < nchunk; c++) {
         double x[16];
 #pragma unroll
         for (int k = 0; k < 16; k++) {
-            const int q = c * 16 + k;
-            x[k] = (valid && q < p.Q) ? col[(int64_t)q * p.nelem] : 0.0;
+            const int q = c * 16 + k, g = q / p.nterms, t = q - g * p.nterms;
+            x[k] = valid && g < p.ngp ? col[((int64_t)t * p.ngp + g) * p.nelem] : 0.0;
         }
         uint32_t w[S][4];
 #pragma unroll
@@ -321,7 +232,7 @@ __global__ void k_slice_cols(const __grid_constant__ ColSliceParams pb)
         }
         // chunk c of K step c/2 lands at [kstep][c&1][s][slot]: (c*S + s) * NE.
 #pragma unroll
-        for (int s = 0; s < S; s++) out[((int64_t)c * S + s) * NE] = make_uint4(w[s][0], w[s][1], w[s][2], w[s][3]);
+        for (int s = 0; s < S; s++) out[((int64_t)c * S + s) * kSplitNE] = make_uint4(w[s][0], w[s][1], w[s][2], w[s][3]);
     }
 }
 
@@ -466,53 +377,49 @@ __device__ __forceinline__ void split_store(const double (&d)[16], V* out, int e
 // ---------------------------------------------------------------- contraction
 
 // Shared memory: pipeline stages, each one K step (32 bytes) of every A slice
-// (128 rows) and every B slice (NE rows), plus barriers.
-template <int NE>
+// (128 rows) and every B slice (64 rows), plus barriers.
 struct SplitSmem {
-    static constexpr int kSt = SplitShape<NE>::kStages;
-    alignas(1024) int8_t A[kSt][kSplitMaxS * kSplitABytes];
-    alignas(1024) int8_t B[kSt][kSplitMaxS * SplitShape<NE>::kBBytes];
-    alignas(8) uint64_t full[kSt];
-    uint64_t empty[kSt];
-    uint64_t tmem_full[2], tmem_empty[2], drain;
+    alignas(1024) int8_t A[kSplitStages][kSplitMaxS * kSplitABytes];
+    alignas(1024) int8_t B[kSplitStages][kSplitMaxS * kSplitBBytes];
+    alignas(8) uint64_t full[kSplitStages];
+    uint64_t empty[kSplitStages];
+    uint64_t tmem_full, tmem_empty, drain;
     uint64_t item_full[kSplitItems], item_empty[kSplitItems];
     int64_t items[kSplitItems];
-    double colscale[kSplitEpiWarps][16];  // each epilogue warp's columns of the unit at hand
+    double colscale[kSplitEpiWarps][16];  // each epilogue warp's columns of the tile at hand
     uint32_t tmem;
     int failed;
 };
-template <int NE>
-constexpr size_t split_smem_bytes() { return sizeof(SplitSmem<NE>) + 1024; }
+constexpr size_t split_smem_bytes() { return sizeof(SplitSmem) + 1024; }
 
 // Persistent, warp-specialised kernel; one CTA per SM holds all 512 TMEM
-// columns.  Work item w = (row tile w % ntp, element unit w / ntp).  Each
+// columns.  Work item w = (row tile w % ntp, element tile w / ntp).  Each
 // CTA's first item is its index; later ones come from a global counter, so
 // the items are taken in order and the CTAs working at the same time always
-// hold neighbouring items: they share element units (B is read from L2 once
-// per unit), and the 32-byte sectors that neighbouring row tiles' mirrored
+// hold neighbouring items: they share element tiles (B is read from L2 once
+// per tile), and the 32-byte sectors that neighbouring row tiles' mirrored
 // stores share are completed while they are still in L2.  (Handed out
-// round-robin, the CTAs drift apart over a long launch.)  The producer skips
-// empty units (past the end of a short tile) and passes each item to the MMA
+// round-robin, the CTAs drift apart over a long launch.)  The producer
+// passes each item to the MMA
 // and epilogue roles through a ring of kSplitItems slots; -1 ends the CTA.
 //   warp 0 (one thread): bulk copies of each K step into the stage ring;
 //   warp 1 (one thread): MMAs; owns the TMEM allocation;
 //   warps 2-17: epilogue; warp w reads TMEM lanes 32(w%4) .. 32(w%4)+31 and
-//              16 of the NE columns.
-// Barriers: full/empty per stage (copies -> MMA -> copies), tmem_full[b] (MMAs
-// of a tile done -> epilogue) and tmem_empty[b] (epilogue has read
-// accumulator b -> MMAs of the next tile using it).  Every wait is bounded: on
+//              16 of the 64 columns.
+// Barriers: full/empty per stage (copies -> MMA -> copies), tmem_full (MMAs of a
+// tile done -> epilogue) and tmem_empty (epilogue has read the accumulator ->
+// MMAs of the next tile).  Every wait is bounded: on
 // timeout the CTA records the failure, the roles stop, outstanding copies and
 // MMAs are waited for (bounded), the TMEM is freed and the CTA returns.
-template <int B, int S, int L, int NE>
+template <int B, int S, int L>
 __global__ void __launch_bounds__(kSplitThreads, 1) k_contract_split(const __grid_constant__ SplitParams p)
 {
     constexpr int NL = L - 1;  // levels 2 .. L
     static_assert(S <= kSplitMaxS && NL <= S && NL >= 5 && NL <= 6, "level layout");
-    using Sh = SplitShape<NE>;
-    static_assert(Sh::kBufs == 1 ? NL * NE <= 512 : NL * NE <= 256, "accumulators fit the 512 TMEM columns");
-    constexpr int kSt = Sh::kStages;
+    constexpr int NE = kSplitNE, kSt = kSplitStages;
+    static_assert(NL * NE <= 512, "the accumulator fits the 512 TMEM columns");
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    SplitSmem<NE>& sm = *reinterpret_cast<SplitSmem<NE>*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    SplitSmem& sm = *reinterpret_cast<SplitSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     constexpr uint32_t kCols = 512;
     volatile int* failed = &sm.failed;
@@ -527,13 +434,11 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_contract_split(const __gri
             mbar_init(&sm.full[s], 1);
             mbar_init(&sm.empty[s], 1);
         }
-        for (int b = 0; b < 2; b++) {
-            mbar_init(&sm.tmem_full[b], 1);
-            mbar_init(&sm.tmem_empty[b], NE / 4);  // epilogue warps with columns
-        }
+        mbar_init(&sm.tmem_full, 1);
+        mbar_init(&sm.tmem_empty, kSplitEpiWarps);
         for (int k = 0; k < kSplitItems; k++) {
             mbar_init(&sm.item_full[k], 1);
-            mbar_init(&sm.item_empty[k], 1 + NE / 4);  // MMA issuer and epilogue warps
+            mbar_init(&sm.item_empty[k], 1 + kSplitEpiWarps);  // MMA issuer and epilogue warps
         }
         mbar_init(&sm.drain, 1);
         sm.failed = 0;
@@ -543,7 +448,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_contract_split(const __gri
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = sm.tmem;
-    constexpr uint32_t kABytes = S * kSplitABytes, kBBytes = S * Sh::kBBytes;
+    constexpr uint32_t kABytes = S * kSplitABytes, kBBytes = S * kSplitBBytes;
 
     if (warp == 0 && lane == 0) {
         // ------------------------------------------------ producer
@@ -554,15 +459,11 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_contract_split(const __gri
         int gi = 0;
         int64_t w = blockIdx.x;
         for (uint32_t k = 0; ok; k++) {
-            // The next non-empty work item, or -1 at the end.
+            // The next work item, or -1 at the end.
             int64_t item = -1;
-            while (w < p.nwork) {
+            if (w < p.nwork) {
                 gi = split_group_of(p, gi, w);
-                if (split_unit<NE>(p.g[gi].tiles, (w - p.g[gi].w0) / p.g[gi].ntp).ne > 0) {
-                    item = w;
-                    break;
-                }
-                w = (int64_t)atomicAdd(p.next, 1ull) + gridDim.x;
+                item = w;
             }
             const int slot = (int)(k % kSplitItems);
             if (!mbar_wait(&sm.item_empty[slot], ((k / kSplitItems) & 1) ^ 1, failed)) {
@@ -578,7 +479,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_contract_split(const __gri
             const int64_t v = item - G.w0;
             const int pt = (int)(v % G.ntp);
             const int64_t u = v / G.ntp;
-            const Tile unit = split_unit<NE>(G.tiles, u);
+            const Tile unit = G.tiles[u];
             const int8_t* srcA = G.A + ((int64_t)unit.orient * G.ntp + pt) * G.nk * kABytes;
             const int8_t* srcB = G.B + u * G.nk * kBBytes;
             const int nk = G.nk;
@@ -613,7 +514,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_contract_split(const __gri
         int stage = 0;
         uint32_t phase = 0;
         bool ok = true;
-        int64_t i = 0;  // units processed by this CTA
+        int64_t i = 0;  // tiles processed by this CTA
         int gi = 0;
         for (uint32_t k = 0; ok; k++) {
             const int slot = (int)(k % kSplitItems);
@@ -628,14 +529,11 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_contract_split(const __gri
             gi = split_group_of(p, gi, w);
             const SplitGroup& G = p.g[gi];
             const int nk = G.nk;
-            const int buf = (int)(i % Sh::kBufs);
-            const int64_t use = i / Sh::kBufs;
-            if (use > 0 && !mbar_wait(&sm.tmem_empty[buf], (uint32_t)((use - 1) & 1), failed)) {
+            if (i > 0 && !mbar_wait(&sm.tmem_empty, (uint32_t)((i - 1) & 1), failed)) {
                 ok = false;
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t dbase = tmem + (uint32_t)(buf * 256);
             for (int ks = 0; ks < nk; ks++) {
                 if (!mbar_wait(&sm.full[stage], phase, failed)) {
                     ok = false;
@@ -648,10 +546,10 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_contract_split(const __gri
                     const int nbt = (S < L - 1 - a0) ? S : L - 1 - a0;  // b = 1 .. min(S, L - a)
                     const uint64_t ad = umma_desc(a_base + a0 * kSplitABytes, kSplitM * 16, 128);
 #pragma unroll
-                    for (int b0 = 0; b0 < nbt; b0 += Sh::kGroup) {
-                        const int nb = (nbt - b0) < Sh::kGroup ? (nbt - b0) : Sh::kGroup;
+                    for (int b0 = 0; b0 < nbt; b0 += kSplitGroupB) {
+                        const int nb = (nbt - b0) < kSplitGroupB ? (nbt - b0) : kSplitGroupB;
                         const uint64_t bd = umma_desc(b_base + b0 * NE * 16, S * NE * 16, 128);
-                        umma_i8(dbase + (uint32_t)(NE * (a0 + b0)), ad, bd, umma_idesc_i8(kSplitM, NE * nb),
+                        umma_i8(tmem + (uint32_t)(NE * (a0 + b0)), ad, bd, umma_idesc_i8(kSplitM, NE * nb),
                                 (ks > 0 || a0 > 0) ? 1u : 0u);
                     }
                 }
@@ -663,7 +561,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_contract_split(const __gri
             }
             if (!ok)
                 break;
-            umma_commit(&sm.tmem_full[buf]);
+            umma_commit(&sm.tmem_full);
             i++;
         }
         if (!ok) {
@@ -686,7 +584,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_contract_split(const __gri
         const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16);
         int64_t i = 0;
         int gi = 0;
-        for (uint32_t k = 0; c0 < NE; k++) {
+        for (uint32_t k = 0;; k++) {
             const int slot = (int)(k % kSplitItems);
             if (!mbar_wait(&sm.item_full[slot], (k / kSplitItems) & 1, failed)) {
                 *failed = 1;
@@ -704,8 +602,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_contract_split(const __gri
             const int64_t v = w - G.w0;
             const int pt = (int)(v % G.ntp);
             const int64_t u = v / G.ntp;
-            const Tile unit = split_unit<NE>(G.tiles, u);
-            const int buf = (int)(i % Sh::kBufs);
+            const Tile unit = G.tiles[u];
             // What the stores need from global memory is requested before the
             // accumulator is complete: a load issued after stores waits
             // behind them.
@@ -716,13 +613,13 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_contract_split(const __gri
             if (lane < 16)
                 sm.colscale[warp - 2][lane] = __ldg(G.colscale + u * NE + c0 + lane);
             __syncwarp();
-            if (!mbar_wait(&sm.tmem_full[buf], (uint32_t)((i / Sh::kBufs) & 1), failed)) {
+            if (!mbar_wait(&sm.tmem_full, (uint32_t)(i & 1), failed)) {
                 *failed = 1;
                 atomicOr(p.error, 1u);
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t col = lane_base + (uint32_t)(buf * 256 + c0);
+            const uint32_t col = lane_base + (uint32_t)c0;
             // V = R_p Q_e 2^-(B L) T.
             double d[16];
 #pragma unroll
@@ -736,7 +633,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_contract_split(const __gri
                     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                     __syncwarp();
                     if (lane == 0)
-                        mbar_arrive(&sm.tmem_empty[buf]);
+                        mbar_arrive(&sm.tmem_empty);
                 }
 #pragma unroll
                 for (int j = 0; j < 8; j++) {
@@ -746,7 +643,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_contract_split(const __gri
                     d[h + j] = split_combine<B, NL>(x) * rsc * sm.colscale[warp - 2][h + j];
                 }
             }
-            __syncwarp();  // every lane has read the scales before the next unit's
+            __syncwarp();  // every lane has read the scales before the next tile's
             const int64_t e = unit.e0 + c0;
             const int nj = min(16, unit.ne - c0);
             const int em = G.out2 != nullptr ? G.es2 : G.es;

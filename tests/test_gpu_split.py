@@ -296,3 +296,39 @@ def test_element_matrix_shapes(ctx, ntf, ndof, form):
             err = np.abs(out[k][: ref[k].size] - ref[k]) / np.maximum(mag[k], 1e-300)
             assert not err.size or err.max() <= tol, f"precision {prec}: {k} error {err.max():.3e} > {tol:g}"
     ctx.check(L.slgpu_matrix_destroy(ctx.h, h))
+
+
+def test_slicing_kernel_matches_interpreter(tmp_path):
+    """The runtime-compiled slicing kernel against the interpreter and the
+    slicing of coefficients in memory (SLGPU_COEF_INTERPRETER=1, its own
+    process): one and several points per thread, elements per block from 4 to
+    32, K that is and is not a multiple of 16 and 32, short tiles.  Both round
+    the coefficients within a few units in the last place and the digits alike
+    or to the neighbouring integer: equal within 1e-12 of the largest value."""
+    import subprocess
+
+    code = """
+import os, sys
+import numpy as np
+sys.path.insert(0, {tests!r}); sys.path.insert(0, {root!r})
+from sparselizard_b200 import abi
+import test_gpu_graphs as T
+ctx, out = abi.Context(0), {{}}
+for k, (grid, ntf, ndof, nterms, ngp1, ndofs) in enumerate([(9, 9, 9, 4, 2, 400), (20, 9, 9, 4, 3, 3000), (13, 10, 8, 9, 4, 900),
+                                                            (11, 8, 8, 5, 8, 500), (11, 12, 9, 3, 9, 600), (7, 9, 9, 1, 7, 300),
+                                                            (6, 9, 9, 10, 11, 300)]):
+    t = T._setup(ctx, np.random.Generator(np.random.PCG64(60 + k)), 20 + k, grid, ntf, ndof, nterms, ngp1, ndofs)
+    for prec in (abi.PREC_SPLIT, abi.PREC_FP32):
+        out["%d_%d_A" % (k, prec)], out["%d_%d_D" % (k, prec)] = T._process(ctx, t, prec)
+ctx.close()
+np.savez(sys.argv[1], **out)
+""".format(tests=os.path.dirname(os.path.abspath(__file__)), root=P.ROOT)
+    res = {}
+    for interp in ("0", "1"):
+        out = str(tmp_path / f"{interp}.npz")
+        subprocess.run([sys.executable, "-c", code, out], env=dict(os.environ, SLGPU_COEF_INTERPRETER=interp), check=True, timeout=600)
+        res[interp] = np.load(out)
+    for key in res["0"].files:
+        a, b = res["0"][key], res["1"][key]
+        tol = 1e-12 if f"_{abi.PREC_SPLIT}_" in key else 2e-7  # float storage rounds to the neighbouring float
+        assert np.all(np.isfinite(a)) and np.abs(a - b).max() <= tol * np.abs(b).max(), key
