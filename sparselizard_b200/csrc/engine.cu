@@ -1076,6 +1076,188 @@ static int bits_for(int64_t n)
     return b;
 }
 
+// Longest row, in COO entries, that k_row_pattern takes (its table has 1.5
+// times as many slots, at most 8192).
+constexpr int64_t kPatternRowMax = 5461;
+
+// Builds the CSR structure, slot map and incidence lists of P row by row.
+// False, with P untouched, when a row has too many COO entries; the caller
+// then sorts all of them.
+static bool pattern_by_rows(Ctx* ctx, Matrix& M, Pattern& P, const std::vector<Segment>& segs, const uint8_t* dconstr, bool rhs, DevBuf& renum)
+{
+    const int64_t ncoo = P.ncoo, nA = P.nA;
+    std::vector<IncSeg> isegs;
+    int64_t ninc_total = 0;
+    size_t si = 0;
+    DevBuf counter;
+    counter.alloc(ctx, 5 * 8);  // bad addresses, incidences, most COO entries of a row, kept COO entries, longest row
+    unsigned long long* cnt = counter.as<unsigned long long>();
+    cuda_check(cudaMemsetAsync(cnt, 0, 5 * 8, ctx->x->stream), "memset");
+    // Dof addresses element by element, once per address array.
+    std::map<const void*, std::shared_ptr<DevBuf>> turned;
+    for (auto& g : M.groups) {
+        for (int d = 0; d < g->ndests; d++, si++) {
+            IncSeg s{};
+            s.inc_base = ninc_total;
+            s.count = g->nelem * (int64_t)g->ntf;
+            s.coo_base = segs[si].coo_base;
+            s.width = g->ndof;
+            s.ntf = g->ntf;
+            s.kind = 0;
+            s.nelem = g->nelem;
+            s.rows = g->tfaddr[d]->as<int32_t>();
+            if (!rhs && g->nelem > 0) {
+                std::shared_ptr<DevBuf>& t = turned[g->dofaddr[d]->as<void>()];
+                if (!t) {
+                    t = std::make_shared<DevBuf>();
+                    t->alloc(ctx, (size_t)g->ndof * g->nelem * 4);
+                    if ((g->ndof + 31) / 32 > 65535)
+                        return false;
+                    k_transpose_addr<<<dim3((unsigned)((g->nelem + 31) / 32), (unsigned)((g->ndof + 31) / 32)), dim3(32, 8), 0, ctx->x->stream>>>(
+                        g->dofaddr[d]->as<int32_t>(), g->ndof, g->nelem, M.ndofs, t->as<int32_t>(), cnt);
+                    cuda_check(cudaGetLastError(), "k_transpose_addr");
+                }
+                s.dofs = t->as<int32_t>();
+            }
+            isegs.push_back(s);
+            ninc_total += s.count;
+        }
+    }
+    for (auto& f : M.frags) {
+        IncSeg s{};
+        s.inc_base = ninc_total;
+        s.count = (int64_t)f->nr * f->nc;
+        s.coo_base = segs[si].coo_base;
+        s.width = 1;
+        s.kind = 1;
+        s.ntr = f->ntr;
+        s.ndr = f->ndr;
+        s.nr = f->nr;
+        s.nc = f->nc;
+        s.rows = f->rows.as<int32_t>();
+        s.cols = f->cols.as<int32_t>();
+        isegs.push_back(s);
+        ninc_total += s.count;
+        si++;
+    }
+    // Limits of the incidence words, reported by the general path.
+    if (ninc_total == 0 || ninc_total >= (int64_t)0xFFFFFFFFll || isegs.size() >= (size_t(1) << 23))
+        return false;
+    const uint32_t invalid = (uint32_t)M.ndofs;  // above every kept row
+    DevBuf dsegs, ikeys, ikeys_alt, iids, iids_alt, rowinc, rowcoo, inc_ptr, coo_ptr, tmp;
+    upload_staged(ctx, dsegs, isegs.data(), isegs.size() * sizeof(IncSeg));
+    ikeys.alloc(ctx, ninc_total * 4);
+    ikeys_alt.alloc(ctx, ninc_total * 4);
+    iids.alloc(ctx, ninc_total * 4);
+    iids_alt.alloc(ctx, ninc_total * 4);
+    k_inc_row_keys<<<grid_for(ninc_total, 256), 256, 0, ctx->x->stream>>>(dsegs.as<IncSeg>(), (int)isegs.size(), ninc_total, dconstr, M.ndofs,
+                                                                      ikeys.as<uint32_t>(), iids.as<uint32_t>(), cnt + 1, invalid, cnt);
+    cuda_check(cudaGetLastError(), "k_inc_row_keys");
+    cub::DoubleBuffer<uint32_t> ik(ikeys.as<uint32_t>(), ikeys_alt.as<uint32_t>());
+    cub::DoubleBuffer<uint32_t> iv(iids.as<uint32_t>(), iids_alt.as<uint32_t>());
+    size_t temp = 0, temp2 = 0;
+    cuda_check(cub::DeviceRadixSort::SortPairs(nullptr, temp, ik, iv, ninc_total, 0, bits_for(M.ndofs), ctx->x->stream), "SortPairs size");
+    cuda_check(cub::DeviceScan::ExclusiveSum(nullptr, temp2, (uint32_t*)nullptr, (uint32_t*)nullptr, nA + 1, ctx->x->stream), "scan size");
+    tmp.alloc(ctx, std::max(temp, temp2));
+    temp = temp2 = std::max(temp, temp2);
+    cuda_check(cub::DeviceRadixSort::SortPairs(tmp.as<void>(), temp, ik, iv, ninc_total, 0, bits_for(M.ndofs), ctx->x->stream), "SortPairs");
+    rowinc.alloc(ctx, (nA + 1) * 4);
+    rowcoo.alloc(ctx, (nA + 1) * 4);
+    inc_ptr.alloc(ctx, (nA + 1) * 4);
+    coo_ptr.alloc(ctx, (nA + 1) * 4);
+    cuda_check(cudaMemsetAsync(rowinc.as<void>(), 0, (nA + 1) * 4, ctx->x->stream), "memset");
+    cuda_check(cudaMemsetAsync(rowcoo.as<void>(), 0, (nA + 1) * 4, ctx->x->stream), "memset");
+    k_inc_rows<<<grid_for(ninc_total, 256), 256, 0, ctx->x->stream>>>(ik.Current(), iv.Current(), ninc_total, invalid, dsegs.as<IncSeg>(),
+                                                                  (int)isegs.size(), renum.as<int32_t>(), rowinc.as<uint32_t>(),
+                                                                  rowcoo.as<uint32_t>());
+    cuda_check(cudaGetLastError(), "k_inc_rows");
+    k_max_u32<<<grid_for(nA, 256), 256, 0, ctx->x->stream>>>(rowcoo.as<uint32_t>(), nA, cnt + 2);
+    cuda_check(cudaGetLastError(), "k_max_u32");
+    cuda_check(cub::DeviceScan::ExclusiveSum(tmp.as<void>(), temp, rowinc.as<uint32_t>(), inc_ptr.as<uint32_t>(), nA + 1, ctx->x->stream), "scan");
+    cuda_check(cub::DeviceScan::ExclusiveSum(tmp.as<void>(), temp, rowcoo.as<uint32_t>(), coo_ptr.as<uint32_t>(), nA + 1, ctx->x->stream), "scan");
+    unsigned long long h[5] = {};
+    uint32_t kept_coo = 0;
+    cuda_check(cudaMemcpyAsync(h, cnt, 5 * 8, cudaMemcpyDeviceToHost, ctx->x->stream), "D2H");
+    cuda_check(cudaMemcpyAsync(&kept_coo, coo_ptr.as<uint32_t>() + nA, 4, cudaMemcpyDeviceToHost, ctx->x->stream), "D2H");
+    cuda_check(cudaStreamSynchronize(ctx->x->stream), "sync");
+    if (h[0] != 0) {  // how many COO entries
+        cuda_check(cudaMemsetAsync(cnt, 0, 8, ctx->x->stream), "memset");
+        for (size_t s = 0; s < isegs.size(); s++)
+            if (isegs[s].count > 0)
+                k_check_addr<<<grid_for(isegs[s].kind == 0 ? isegs[s].nelem : isegs[s].count, 256), 256, 0, ctx->x->stream>>>(
+                    dsegs.as<IncSeg>(), (int)s, M.ndofs, cnt);
+        cuda_check(cudaGetLastError(), "k_check_addr");
+        cuda_check(cudaMemcpyAsync(h, cnt, 8, cudaMemcpyDeviceToHost, ctx->x->stream), "D2H");
+        cuda_check(cudaStreamSynchronize(ctx->x->stream), "sync");
+        fail(SLGPU_E_ARG, std::to_string(h[0]) + " COO addresses are >= the DOF count");
+    }
+    if ((int64_t)h[2] > kPatternRowMax)
+        return false;
+    ikeys.release();
+    const int64_t ninc = (int64_t)h[1];
+    int hmax = 32;
+    while (hmax < (int)h[2] + (int)h[2] / 2) hmax *= 2;
+    P.ninc = ninc;
+    P.inc.alloc(ctx, std::max<int64_t>(ninc, 1) * 8);
+    P.slotmap.alloc(ctx, std::max<int64_t>(ncoo, 1) * 2);
+    DevBuf cols;
+    cols.alloc(ctx, std::max<size_t>(kept_coo, 1) * 4);
+    RowPatternParams rp{};
+    rp.sids = iv.Current();
+    rp.inc_ptr = inc_ptr.as<uint32_t>();
+    rp.coo_ptr = coo_ptr.as<uint32_t>();
+    rp.segs = dsegs.as<IncSeg>();
+    rp.nsegs = (int)isegs.size();
+    rp.nrows = nA;
+    rp.constrained = dconstr;
+    rp.slotmap = P.slotmap.as<uint16_t>();
+    rp.inc = P.inc.as<unsigned long long>();
+    rp.cols = cols.as<uint32_t>();
+    rp.rowcA = rowinc.as<uint32_t>();
+    rp.rowcD = rowcoo.as<uint32_t>();
+    rp.counters = cnt + 3;
+    static std::once_flag attr;
+    std::call_once(attr, [] { cudaFuncSetAttribute(k_row_pattern, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024); });
+    // Counts of rows without kept rows beyond nA stay zero (the scans' last entry).
+    cuda_check(cudaMemsetAsync(rowinc.as<void>(), 0, (nA + 1) * 4, ctx->x->stream), "memset");
+    cuda_check(cudaMemsetAsync(rowcoo.as<void>(), 0, (nA + 1) * 4, ctx->x->stream), "memset");
+    for (int H = 256; nA > 0; H *= 2) {
+        rp.hmin = H == 256 ? 0 : H / 2;
+        rp.hmax = H;
+        const size_t per_warp = (size_t)12 * H;
+        const int wpb = (int)std::max<size_t>(1, std::min<size_t>(4, (96 * 1024) / per_warp));
+        k_row_pattern<<<grid_for(nA, wpb), 32 * wpb, per_warp * wpb, ctx->x->stream>>>(rp);
+        cuda_check(cudaGetLastError(), "k_row_pattern");
+        if (H >= hmax)
+            break;
+    }
+    P.Arows.alloc(ctx, (nA + 1) * 4);
+    P.Drows.alloc(ctx, (nA + 1) * 4);
+    cuda_check(cub::DeviceScan::ExclusiveSum(tmp.as<void>(), temp, rowinc.as<uint32_t>(), P.Arows.as<uint32_t>(), nA + 1, ctx->x->stream), "scan");
+    cuda_check(cub::DeviceScan::ExclusiveSum(tmp.as<void>(), temp, rowcoo.as<uint32_t>(), P.Drows.as<uint32_t>(), nA + 1, ctx->x->stream), "scan");
+    uint32_t tot[2];
+    cuda_check(cudaMemcpyAsync(h, cnt, 5 * 8, cudaMemcpyDeviceToHost, ctx->x->stream), "D2H");
+    cuda_check(cudaMemcpyAsync(&tot[0], P.Arows.as<uint32_t>() + nA, 4, cudaMemcpyDeviceToHost, ctx->x->stream), "D2H");
+    cuda_check(cudaMemcpyAsync(&tot[1], P.Drows.as<uint32_t>() + nA, 4, cudaMemcpyDeviceToHost, ctx->x->stream), "D2H");
+    cuda_check(cudaStreamSynchronize(ctx->x->stream), "sync");
+    P.nvalid = (int64_t)h[3];
+    P.lmax = (int)h[4];
+    P.nnzA = tot[0];
+    P.nnzD = tot[1];
+    if (P.nnzA >= (int64_t(1) << 31) || P.nnzD >= (int64_t(1) << 31))
+        fail(SLGPU_E_UNSUPPORTED, "more than 2^31-1 nonzeros in a CSR block (32-bit PETSc row pointers)");
+    P.Acols.alloc(ctx, std::max<int64_t>(P.nnzA, 1) * 4);
+    P.Dcols.alloc(ctx, std::max<int64_t>(P.nnzD, 1) * 4);
+    if (nA > 0) {
+        k_row_cols<<<grid_for(nA * 32, 256), 256, 0, ctx->x->stream>>>(cols.as<uint32_t>(), coo_ptr.as<uint32_t>(), P.Arows.as<uint32_t>(),
+                                                                   P.Drows.as<uint32_t>(), nA, renum.as<int32_t>(), P.Acols.as<int32_t>(),
+                                                                   P.Dcols.as<int32_t>());
+        cuda_check(cudaGetLastError(), "k_row_cols");
+    }
+    P.inc_ptr = std::move(inc_ptr);
+    return true;
+}
+
 // Builds (or fetches) the pattern for matrix M with the given constraints
 // (all-zero constraints for a right-hand side, which has one column).
 static std::shared_ptr<Pattern> get_pattern(Ctx* ctx, Matrix& M, const std::vector<Segment>& segs, const uint8_t* dconstr,
@@ -1106,6 +1288,52 @@ static std::shared_ptr<Pattern> get_pattern(Ctx* ctx, Matrix& M, const std::vect
     size_t temp = 0;
     DevBuf tmp;
 
+    // ---- local renumbering of constrained / unconstrained DOFs.
+    DevBuf renum;
+    renum.alloc(ctx, std::max<int64_t>(M.ndofs, 1) * 4);
+    int64_t nA = 0, nD = 0;
+    {
+        DevBuf flagsA, scanA, flagsD, scanD;
+        flagsA.alloc(ctx, (M.ndofs + 1) * 4);
+        flagsD.alloc(ctx, (M.ndofs + 1) * 4);
+        scanA.alloc(ctx, (M.ndofs + 1) * 4);
+        scanD.alloc(ctx, (M.ndofs + 1) * 4);
+        k_constraint_flags<<<grid_for(M.ndofs + 1, 256), 256, 0, ctx->x->stream>>>(dconstr, M.ndofs, flagsA.as<uint32_t>(),
+                                                                                 flagsD.as<uint32_t>());
+        cuda_check(cudaGetLastError(), "k_constraint_flags");
+        temp = 0;
+        cuda_check(cub::DeviceScan::ExclusiveSum(nullptr, temp, flagsA.as<uint32_t>(), scanA.as<uint32_t>(), (int64_t)M.ndofs + 1,
+                                                 ctx->x->stream),
+                   "scan size");
+        tmp.alloc(ctx, temp);
+        cuda_check(cub::DeviceScan::ExclusiveSum(tmp.as<void>(), temp, flagsA.as<uint32_t>(), scanA.as<uint32_t>(), (int64_t)M.ndofs + 1,
+                                                 ctx->x->stream),
+                   "scan");
+        cuda_check(cub::DeviceScan::ExclusiveSum(tmp.as<void>(), temp, flagsD.as<uint32_t>(), scanD.as<uint32_t>(), (int64_t)M.ndofs + 1,
+                                                 ctx->x->stream),
+                   "scan");
+        tmp.release();
+        uint32_t tot[2];
+        cuda_check(cudaMemcpyAsync(&tot[0], scanA.as<uint32_t>() + M.ndofs, 4, cudaMemcpyDeviceToHost, ctx->x->stream), "D2H");
+        cuda_check(cudaMemcpyAsync(&tot[1], scanD.as<uint32_t>() + M.ndofs, 4, cudaMemcpyDeviceToHost, ctx->x->stream), "D2H");
+        k_renumber<<<grid_for(M.ndofs, 256), 256, 0, ctx->x->stream>>>(dconstr, M.ndofs, scanA.as<uint32_t>(), scanD.as<uint32_t>(),
+                                                                     renum.as<int32_t>());
+        cuda_check(cudaGetLastError(), "k_renumber");
+        cuda_check(cudaStreamSynchronize(ctx->x->stream), "sync");
+        nA = tot[0];
+        nD = tot[1];
+        P->ainds.alloc(ctx, std::max<int64_t>(nA, 1) * 4);
+        P->dinds.alloc(ctx, std::max<int64_t>(nD, 1) * 4);
+        if (M.ndofs > 0) {
+            k_dof_split<<<grid_for(M.ndofs, 256), 256, 0, ctx->x->stream>>>(dconstr, M.ndofs, scanA.as<uint32_t>(), scanD.as<uint32_t>(),
+                                                                          P->ainds.as<int32_t>(), P->dinds.as<int32_t>());
+            cuda_check(cudaGetLastError(), "k_dof_split");
+        }
+    }
+    P->nA = nA;
+    P->nD = nD;
+    const bool by_rows = pattern_by_rows(ctx, M, *P, segs, dconstr, rhs, renum);
+    if (!by_rows) {
     // ---- COO keys in COO order, stable radix sort on the used bits.
     DevBuf keys, keys_alt, idx, idx_alt, counter;
     keys.alloc(ctx, std::max<int64_t>(ncoo, 1) * 8);
@@ -1206,51 +1434,6 @@ static std::shared_ptr<Pattern> get_pattern(Ctx* ctx, Matrix& M, const std::vect
                                                                      run_start.as<uint32_t>());
         cuda_check(cudaGetLastError(), "k_run_starts");
     }
-
-    // ---- local renumbering of constrained / unconstrained DOFs.
-    DevBuf renum;
-    renum.alloc(ctx, std::max<int64_t>(M.ndofs, 1) * 4);
-    int64_t nA = 0, nD = 0;
-    {
-        DevBuf flagsA, scanA, flagsD, scanD;
-        flagsA.alloc(ctx, (M.ndofs + 1) * 4);
-        flagsD.alloc(ctx, (M.ndofs + 1) * 4);
-        scanA.alloc(ctx, (M.ndofs + 1) * 4);
-        scanD.alloc(ctx, (M.ndofs + 1) * 4);
-        k_constraint_flags<<<grid_for(M.ndofs + 1, 256), 256, 0, ctx->x->stream>>>(dconstr, M.ndofs, flagsA.as<uint32_t>(),
-                                                                                 flagsD.as<uint32_t>());
-        cuda_check(cudaGetLastError(), "k_constraint_flags");
-        temp = 0;
-        cuda_check(cub::DeviceScan::ExclusiveSum(nullptr, temp, flagsA.as<uint32_t>(), scanA.as<uint32_t>(), (int64_t)M.ndofs + 1,
-                                                 ctx->x->stream),
-                   "scan size");
-        tmp.alloc(ctx, temp);
-        cuda_check(cub::DeviceScan::ExclusiveSum(tmp.as<void>(), temp, flagsA.as<uint32_t>(), scanA.as<uint32_t>(), (int64_t)M.ndofs + 1,
-                                                 ctx->x->stream),
-                   "scan");
-        cuda_check(cub::DeviceScan::ExclusiveSum(tmp.as<void>(), temp, flagsD.as<uint32_t>(), scanD.as<uint32_t>(), (int64_t)M.ndofs + 1,
-                                                 ctx->x->stream),
-                   "scan");
-        tmp.release();
-        uint32_t tot[2];
-        cuda_check(cudaMemcpyAsync(&tot[0], scanA.as<uint32_t>() + M.ndofs, 4, cudaMemcpyDeviceToHost, ctx->x->stream), "D2H");
-        cuda_check(cudaMemcpyAsync(&tot[1], scanD.as<uint32_t>() + M.ndofs, 4, cudaMemcpyDeviceToHost, ctx->x->stream), "D2H");
-        k_renumber<<<grid_for(M.ndofs, 256), 256, 0, ctx->x->stream>>>(dconstr, M.ndofs, scanA.as<uint32_t>(), scanD.as<uint32_t>(),
-                                                                     renum.as<int32_t>());
-        cuda_check(cudaGetLastError(), "k_renumber");
-        cuda_check(cudaStreamSynchronize(ctx->x->stream), "sync");
-        nA = tot[0];
-        nD = tot[1];
-        P->ainds.alloc(ctx, std::max<int64_t>(nA, 1) * 4);
-        P->dinds.alloc(ctx, std::max<int64_t>(nD, 1) * 4);
-        if (M.ndofs > 0) {
-            k_dof_split<<<grid_for(M.ndofs, 256), 256, 0, ctx->x->stream>>>(dconstr, M.ndofs, scanA.as<uint32_t>(), scanD.as<uint32_t>(),
-                                                                          P->ainds.as<int32_t>(), P->dinds.as<int32_t>());
-            cuda_check(cudaGetLastError(), "k_dof_split");
-        }
-    }
-    P->nA = nA;
-    P->nD = nD;
 
     // ---- A / D classification, CSR structure, slot of every run.
     DevBuf run_target;
@@ -1445,6 +1628,7 @@ static std::shared_ptr<Pattern> get_pattern(Ctx* ctx, Matrix& M, const std::vect
     cuda_check(cudaMemcpyAsync(counts_h, counter.as<void>(), 16, cudaMemcpyDeviceToHost, ctx->x->stream), "D2H");
     cuda_check(cudaStreamSynchronize(ctx->x->stream), "sync");
     P->lmax = (int)counts_h[0];
+    }
 
     P->last_use = ++ctx->use_clock;
     ctx->patterns.push_back(P);
@@ -1821,31 +2005,36 @@ static void contract_split_all(Ctx* ctx, const std::vector<SplitJob>& jobs)
     }
 }
 
-// Times the candidates on the jobs' own data and returns the fastest.  The
-// first candidate is the default: it runs once untimed first (clocks ramp up
-// on a GPU that was idle), then every candidate runs three times in turn and
-// its best run counts; another candidate replaces the default only when its
-// best run is at least 3 % faster.  The candidates give identical results.
+// Times the candidates on the call's own data and returns the fastest.  The
+// first candidate is the default: it runs once first (clocks ramp up on a GPU
+// that was idle), then every candidate runs in turn, once where that first run
+// took 50 us or more, else three times, and its best run counts; another
+// candidate replaces the default only when its best run is at least 3 %
+// faster.  The candidates give identical results.
 template <class Run>
 static int pick_by_timing(Ctx* ctx, const std::vector<int>& cand, Run run)
 {
-    constexpr int kRounds = 3;
     const size_t nc = cand.size();
-    std::vector<cudaEvent_t> ev(kRounds * nc + 1);
+    if (nc == 1) {
+        run(cand[0]);
+        return cand[0];
+    }
+    cudaEvent_t ev[2];
     for (auto& e : ev) cuda_check(cudaEventCreate(&e), "cudaEventCreate");
-    run(cand[0]);
-    cuda_check(cudaEventRecord(ev[0], ctx->x->stream), "cudaEventRecord");
-    for (size_t r = 0; r < kRounds; r++)
-        for (size_t c = 0; c < nc; c++) {
-            run(cand[c]);
-            cuda_check(cudaEventRecord(ev[1 + r * nc + c], ctx->x->stream), "cudaEventRecord");
-        }
-    cuda_check(cudaEventSynchronize(ev[kRounds * nc]), "sync");
+    auto timed = [&](int c) {
+        cuda_check(cudaEventRecord(ev[0], ctx->x->stream), "cudaEventRecord");
+        run(c);
+        cuda_check(cudaEventRecord(ev[1], ctx->x->stream), "cudaEventRecord");
+        cuda_check(cudaEventSynchronize(ev[1]), "sync");
+        float t = 0;
+        cudaEventElapsedTime(&t, ev[0], ev[1]);
+        return t;
+    };
+    const int rounds = timed(cand[0]) >= 0.05f ? 1 : 3;
     std::vector<float> best(nc, 0.0f);
-    for (size_t c = 0; c < nc; c++)
-        for (size_t r = 0; r < kRounds; r++) {
-            float t = 0;
-            cudaEventElapsedTime(&t, ev[r * nc + c], ev[r * nc + c + 1]);
+    for (int r = 0; r < rounds; r++)
+        for (size_t c = 0; c < nc; c++) {
+            const float t = timed(cand[c]);
             best[c] = r == 0 ? t : std::min(best[c], t);
         }
     for (auto& e : ev) cudaEventDestroy(e);
@@ -2776,9 +2965,15 @@ void launch_row_values(Ctx* ctx, const Matrix& M, Pattern& P, const std::vector<
     if (choice < 0 && !ctx->x->capturing && ctx->x == &ctx->main) {
         // Every candidate timed on this call's data (their outputs are
         // identical), warp per row being the default.
-        const int kt = kstat_start(ctx, "row_values", (1.0 + 3.0 * cand.size()) * rbytes);
-        P.row_kernel = pick_by_timing(ctx, cand, launch);
+        const int kt = kstat_start(ctx, "row_values", 0.0);
+        int runs = 0;
+        P.row_kernel = pick_by_timing(ctx, cand, [&](int c) {
+            launch(c);
+            runs++;
+        });
         kstat_stop(ctx, kt);
+        if (kt >= 0)
+            ctx->x->kev_tag[kt].second = runs * rbytes;
         return;
     }
     if (choice < 0)

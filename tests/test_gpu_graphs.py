@@ -284,3 +284,49 @@ def test_shared_address_arrays(ctx):
         ctx.check(L.slgpu_matrix_destroy(ctx.h, h))
     assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
     assert out[0][2] == out[1][2]
+
+
+@pytest.mark.parametrize("per_row,ndof,ndofs", [(1, 1, 50), (21, 1, 400), (22, 2, 400), (43, 3, 300), (5461, 1, 9000), (5462, 1, 9000),
+                                                (700, 7, 60), (150, 33, 6000)])
+def test_pattern_row_sizes(ctx, per_row, ndof, ndofs):
+    """Rows with few to many COO entries, up to and beyond the most that the
+    row-by-row pattern takes, with repeated columns, dropped and constrained
+    ones, and two destinations: CSR structure equal to the oracle's, values
+    within 1e-12 of the sums of magnitudes."""
+    import os
+    import sys
+
+    sys.path.insert(0, os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "oracle"))
+    import slref
+
+    rng = np.random.Generator(np.random.PCG64(per_row + 7 * ndof))
+    grid = int(np.ceil(np.sqrt(per_row))) + 1
+    gb, xyz, conn = S.group(rng, nelem_grid=grid, ntf=2, ndof=ndof, nterms=2, ngp1=2, norient=1, ndests=2, ndofs=ndofs)
+    g = gb.g
+    # Test function 0 of the first per_row elements meets row 3; the others spread.
+    tf = np.ctypeslib.as_array(g.dests[0].tfaddr, (2, g.nelem))
+    tf[0, :] = -1
+    tf[0, :per_row] = 3
+    con = (rng.random(ndofs) < 0.1).astype(np.uint8)
+    con[3] = 0
+    ref = slref.matrix([g], xyz, [conn], ndofs, con)
+    mag = slref.matrix([g], xyz, [conn], ndofs, con, absmode=True)
+    L = ctx.lib
+    ctx.check(L.slgpu_mesh_set_nodes(ctx.h, 41, xyz.size // 3, abi.f64p(xyz)))
+    ctx.check(L.slgpu_mesh_set_elements(ctx.h, 41, 3, 4, conn.size // 4, abi.i32p(conn)))
+    g.mesh = 41
+    h = ctypes.c_int()
+    ctx.check(L.slgpu_matrix_create(ctx.h, ndofs, ctypes.byref(h)))
+    ctx.check(L.slgpu_matrix_add_group(ctx.h, h, ctypes.byref(g), None))
+    info = abi.CsrInfo()
+    ctx.check(L.slgpu_matrix_process(ctx.h, h, con.ctypes.data_as(ctypes.POINTER(ctypes.c_uint8)), abi.PREC_FP64, ctypes.byref(info)))
+    out = {k: np.zeros(max(1, n), t) for k, n, t in (("Arows", info.nA + 1, np.int32), ("Acols", info.nnzA, np.int32),
+                                                     ("Avals", info.nnzA, np.float64), ("Drows", info.nA + 1, np.int32),
+                                                     ("Dcols", info.nnzD, np.int32), ("Dvals", info.nnzD, np.float64))}
+    ctx.check(L.slgpu_matrix_download(ctx.h, h, *[abi.i32p(v) if v.dtype == np.int32 else abi.f64p(v) for v in out.values()]))
+    ctx.check(L.slgpu_matrix_destroy(ctx.h, h))
+    for k in ("Arows", "Acols", "Drows", "Dcols"):
+        assert np.array_equal(out[k][: ref[k].size], ref[k]), f"{k} differs"
+    for k in ("Avals", "Dvals"):
+        err = np.abs(out[k][: ref[k].size] - ref[k]) / np.maximum(mag[k], 1e-300)
+        assert not err.size or err.max() <= 1e-12, f"{k}: {err.max():.3e}"
