@@ -164,25 +164,115 @@ static void h2d_pageable(Ctx* ctx, void* dst, const void* src, size_t n)
         fail(SLGPU_E_CUDA, err);
 }
 
+// From this size on a pageable array goes through the page-locked ring: its
+// threads cost about 0.2 ms, the driver's own staging copies about 6 GB/s.
+constexpr size_t kRingBytes = size_t(2) << 20;
+
+static void copy_h2d(Ctx* ctx, void* dst, const void* src, size_t bytes)
+{
+    if (bytes == 0)
+        return;
+    if (bytes >= kRingBytes && !ctx->x->capturing) {
+        cudaPointerAttributes a{};
+        const bool pinned = cudaPointerGetAttributes(&a, src) == cudaSuccess && a.type == cudaMemoryTypeHost;
+        cudaGetLastError();
+        if (!pinned) {
+            h2d_pageable(ctx, dst, src, bytes);
+            return;
+        }
+    }
+    cuda_check(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->x->stream), "cudaMemcpyAsync H2D");
+}
+
 template <class T>
 static void upload(Ctx* ctx, DevBuf& buf, const T* src, size_t count)
 {
     buf.alloc(ctx, count * sizeof(T));
     const size_t bytes = count * sizeof(T);
     ctx->bytes_h2d += (int64_t)bytes;
-    if (count == 0)
-        return;
-    if (bytes >= (size_t(8) << 20) && !ctx->x->capturing) {
-        cudaPointerAttributes a{};
-        const bool pinned = cudaPointerGetAttributes(&a, src) == cudaSuccess && a.type == cudaMemoryTypeHost;
-        cudaGetLastError();
-        if (!pinned) {
-            h2d_pageable(ctx, buf.as<void>(), src, bytes);
+    copy_h2d(ctx, buf.as<void>(), src, bytes);
+}
+
+// The arrays of one group: those of up to kMost bytes are gathered in one
+// page-locked block and copied at once into one device buffer, of which each
+// becomes a part; larger ones are uploaded by themselves, from kRingBytes on
+// through the ring, data arrays too.  (A group has about 20 arrays, most of a
+// few hundred bytes, and each took an allocation and a pageable copy.  A
+// right-hand side of 512 P3 quadrangles: 165 -> 69..93 us; the source of
+// 68921 27-node hexahedra, 22 MB of addresses and field values: 5.4 -> 2.4 ms;
+// nine groups of 4096 hexahedra and their assembly and download: 4.58 -> 4.23 ms.)
+class GroupUpload {
+public:
+    GroupUpload(Ctx* ctx, DevBuf& pack) : ctx_(ctx), pack_(pack) {}
+    // `src` in pieces that follow one another in the buffer.
+    void add(DevBuf& buf, std::vector<std::pair<const void*, size_t>> pieces)
+    {
+        size_t bytes = 0;
+        for (auto& p : pieces) bytes += p.second;
+        ctx_->bytes_h2d += (int64_t)bytes;
+        if (bytes > kMost) {
+            buf.alloc(ctx_, bytes);
+            size_t off = 0;
+            for (auto& p : pieces) {
+                copy_h2d(ctx_, buf.as<char>() + off, p.first, p.second);
+                off += p.second;
+            }
             return;
         }
+        items_.push_back(Item{&buf, std::move(pieces), total_, bytes});
+        total_ += (std::max<size_t>(bytes, 16) + 255) & ~size_t(255);
     }
-    cuda_check(cudaMemcpyAsync(buf.as<void>(), src, bytes, cudaMemcpyHostToDevice, ctx->x->stream), "cudaMemcpyAsync H2D");
-}
+    template <class T>
+    void add(DevBuf& buf, const T* src, size_t count)
+    {
+        add(buf, {{src, count * sizeof(T)}});
+    }
+    template <class T>
+    void add(DevBuf& buf, const std::vector<T>& v)
+    {
+        add(buf, v.data(), v.size());
+    }
+    void finish()
+    {
+        pack_.alloc(ctx_, total_);
+        const int b = ctx_->pack_turn ^= 1;
+        if (ctx_->pack_ev[b] == nullptr)
+            cuda_check(cudaEventCreateWithFlags(&ctx_->pack_ev[b], cudaEventDisableTiming), "cudaEventCreate");
+        cuda_check(cudaEventSynchronize(ctx_->pack_ev[b]), "group upload");  // the block's previous copy
+        if (ctx_->pack_bytes[b] < total_) {
+            if (ctx_->pack_stage[b] != nullptr)
+                cudaFreeHost(ctx_->pack_stage[b]);
+            ctx_->pack_stage[b] = nullptr;
+            ctx_->pack_bytes[b] = 0;
+            const size_t want = std::max<size_t>(total_, size_t(1) << 18);
+            cuda_check(cudaHostAlloc(reinterpret_cast<void**>(&ctx_->pack_stage[b]), want, cudaHostAllocDefault), "cudaHostAlloc");
+            ctx_->pack_bytes[b] = want;
+        }
+        for (const Item& it : items_) {
+            char* dst = ctx_->pack_stage[b] + it.off;
+            for (auto& p : it.pieces) {
+                if (p.second > 0)
+                    std::memcpy(dst, p.first, p.second);
+                dst += p.second;
+            }
+            it.buf->view(pack_.as<char>() + it.off, it.bytes);
+        }
+        cuda_check(cudaMemcpyAsync(pack_.as<void>(), ctx_->pack_stage[b], total_, cudaMemcpyHostToDevice, ctx_->x->stream), "group upload");
+        cuda_check(cudaEventRecord(ctx_->pack_ev[b], ctx_->x->stream), "cudaEventRecord");
+    }
+
+private:
+    static constexpr size_t kMost = size_t(512) << 10;
+    struct Item {
+        DevBuf* buf;
+        std::vector<std::pair<const void*, size_t>> pieces;
+        size_t off, bytes;
+    };
+    Ctx* ctx_;
+    DevBuf& pack_;
+    std::vector<Item> items_;
+    size_t total_ = 0;
+};
 
 template <class T>
 static void upload(Ctx* ctx, DevBuf& buf, const std::vector<T>& v)
@@ -558,11 +648,11 @@ static void content_keys(const slgpu_group& g, GroupDev& gd)
 {
     gd.term_keys.clear();
     gd.data_keys.clear();
+    if (g.terms[0].dof_table < 0)
+        return;  // right-hand sides are never paired
     for (int k = 0; k < g.nelemdata; k++) gd.data_keys.push_back(key_of(g.elemdata[k], (size_t)g.nelem, 1));
     for (int k = 0; k < g.nfielddata; k++)
         gd.data_keys.push_back(key_of(g.fielddata[k], (size_t)g.fieldrows[k] * g.nelem, 2));
-    if (g.terms[0].dof_table < 0)
-        return;
     std::vector<GroupDev::Key> tk(g.ntables);
     for (int k = 0; k < g.ntables; k++)
         tk[k] = key_mix(key_of(g.tables[k].vals, (size_t)g.norient * g.tables[k].rows * g.ngp, 3), (uint64_t)g.tables[k].rows);
@@ -689,7 +779,6 @@ static std::shared_ptr<GroupDev> make_group(Ctx* ctx, const slgpu_group& g,
         gd->tab_rows.push_back(g.tables[k].rows);
         off += (int64_t)g.norient * g.tables[k].rows * g.ngp;
     }
-    const int64_t tables_total = off;
     for (int k = 0; k < g.nelemdata; k++) gd->elemdata_off.push_back((int64_t)k * g.nelem);
     off = 0;
     for (int k = 0; k < g.nfielddata; k++) {
@@ -697,7 +786,6 @@ static std::shared_ptr<GroupDev> make_group(Ctx* ctx, const slgpu_group& g,
         gd->field_rows.push_back(g.fieldrows[k]);
         off += (int64_t)g.fieldrows[k] * g.nelem;
     }
-    const int64_t field_total = off;
     for (int t = 0; t < g.nterms; t++) {
         gd->term_scale.push_back(g.terms[t].scale);
         gd->term_tf.push_back(g.terms[t].tf_table);
@@ -771,37 +859,32 @@ static std::shared_ptr<GroupDev> make_group(Ctx* ctx, const slgpu_group& g,
         if (g.elems[e] < 0 || g.elems[e] >= mt.nelem)
             fail(SLGPU_E_ARG, "element number out of range of the uploaded mesh");
 
-    upload(ctx, gd->elems, g.elems, (size_t)g.nelem);
-    upload(ctx, gd->orient, g.orient, (size_t)g.nelem);
-    upload(ctx, gd->weights, g.weights, (size_t)g.ngp);
-    upload(ctx, gd->lagrange, g.lagrange, (size_t)(1 + g.elemdim) * g.ncurvednodes * g.ngp);
-    gd->tables.alloc(ctx, (size_t)tables_total * sizeof(double));
-    ctx->bytes_h2d += (int64_t)tables_total * 8 + (int64_t)g.nelemdata * g.nelem * 8 + field_total * 8;
+    GroupUpload up(ctx, gd->pack);
+    up.add(gd->elems, g.elems, (size_t)g.nelem);
+    up.add(gd->orient, g.orient, (size_t)g.nelem);
+    up.add(gd->weights, g.weights, (size_t)g.ngp);
+    up.add(gd->lagrange, g.lagrange, (size_t)(1 + g.elemdim) * g.ncurvednodes * g.ngp);
+    std::vector<std::pair<const void*, size_t>> pieces;
     for (int k = 0; k < g.ntables; k++)
-        cuda_check(cudaMemcpyAsync(gd->tables.as<double>() + gd->tab_off[k], g.tables[k].vals,
-                                   (size_t)g.norient * g.tables[k].rows * g.ngp * sizeof(double), cudaMemcpyHostToDevice,
-                                   ctx->x->stream),
-                   "upload tables");
-    upload(ctx, gd->consts, g.consts, (size_t)g.nconsts);
-    upload(ctx, gd->prog_d, gd->prog);
-    gd->elemdata.alloc(ctx, (size_t)g.nelemdata * g.nelem * sizeof(double));
-    for (int k = 0; k < g.nelemdata; k++)
-        cuda_check(cudaMemcpyAsync(gd->elemdata.as<double>() + gd->elemdata_off[k], g.elemdata[k],
-                                   (size_t)g.nelem * sizeof(double), cudaMemcpyHostToDevice, ctx->x->stream),
-                   "upload elemdata");
-    gd->fielddata.alloc(ctx, (size_t)field_total * sizeof(double));
-    for (int k = 0; k < g.nfielddata; k++)
-        cuda_check(cudaMemcpyAsync(gd->fielddata.as<double>() + gd->field_off[k], g.fielddata[k],
-                                   (size_t)g.fieldrows[k] * g.nelem * sizeof(double), cudaMemcpyHostToDevice, ctx->x->stream),
-                   "upload fielddata");
-    upload(ctx, gd->field_off_d, gd->field_off);
-    upload(ctx, gd->field_rows_d, gd->field_rows);
-    upload(ctx, gd->tab_off_d, gd->tab_off);
-    upload(ctx, gd->tab_rows_d, gd->tab_rows);
-    upload(ctx, gd->term_scale_d, gd->term_scale);
-    upload(ctx, gd->term_tf_d, gd->term_tf);
-    upload(ctx, gd->term_dof_d, gd->term_dof);
-    upload(ctx, gd->tiles_d, gd->tiles);
+        pieces.emplace_back(g.tables[k].vals, (size_t)g.norient * g.tables[k].rows * g.ngp * sizeof(double));
+    up.add(gd->tables, pieces);
+    up.add(gd->consts, g.consts, (size_t)g.nconsts);
+    up.add(gd->prog_d, gd->prog);
+    pieces.clear();
+    for (int k = 0; k < g.nelemdata; k++) pieces.emplace_back(g.elemdata[k], (size_t)g.nelem * sizeof(double));
+    up.add(gd->elemdata, pieces);
+    pieces.clear();
+    for (int k = 0; k < g.nfielddata; k++) pieces.emplace_back(g.fielddata[k], (size_t)g.fieldrows[k] * g.nelem * sizeof(double));
+    up.add(gd->fielddata, pieces);
+    up.add(gd->field_off_d, gd->field_off);
+    up.add(gd->field_rows_d, gd->field_rows);
+    up.add(gd->tab_off_d, gd->tab_off);
+    up.add(gd->tab_rows_d, gd->tab_rows);
+    up.add(gd->term_scale_d, gd->term_scale);
+    up.add(gd->term_tf_d, gd->term_tf);
+    up.add(gd->term_dof_d, gd->term_dof);
+    up.add(gd->tiles_d, gd->tiles);
+    up.finish();
     // Address arrays: uploaded and hashed by content, or, where the caller
     // allows it, taken from an earlier group of the same matrix given the same
     // host array.  The destination's place (salt) is mixed in on the host.
@@ -3441,6 +3524,12 @@ void slgpu_ctx_destroy(slgpu_ctx* ctx)
                 cudaFreeHost(ctx->dl_stage[b]);
             if (ctx->dl_ev[b] != nullptr)
                 cudaEventDestroy(ctx->dl_ev[b]);
+        }
+        for (int b = 0; b < 2; b++) {
+            if (ctx->pack_stage[b] != nullptr)
+                cudaFreeHost(ctx->pack_stage[b]);
+            if (ctx->pack_ev[b] != nullptr)
+                cudaEventDestroy(ctx->pack_ev[b]);
         }
         for (int b = 0; b < Ctx::kUlStages; b++) {
             if (ctx->ul_stage[b] != nullptr)

@@ -29,6 +29,13 @@ public:
     ~DevBuf() { release(); }
     void alloc(Ctx* ctx, size_t bytes);  // throws on failure / budget
     void release();
+    // A part of another buffer, which stays its owner.
+    void view(void* p, size_t bytes)
+    {
+        release();
+        p_ = p;
+        n_ = bytes;
+    }
     template <class T> T* as() const { return static_cast<T*>(p_); }
     size_t bytes() const { return n_; }
     bool empty() const { return p_ == nullptr; }
@@ -110,6 +117,7 @@ struct GroupDev {
     };
     mutable Jit jit_coef, jit_slice[2];  // coefficients; slices per tier
 
+    DevBuf pack;  // holds the arrays below that are small
     DevBuf elems, orient, weights, lagrange, tables, consts, prog_d, elemdata, fielddata, field_off_d, field_rows_d,
         tab_off_d, tab_rows_d, term_scale_d, term_tf_d, term_dof_d, tiles_d;
     std::vector<std::shared_ptr<DevBuf>> tfaddr, dofaddr;  // per destination; shared by groups of one matrix when allowed
@@ -358,6 +366,12 @@ struct Ctx {
     char* ul_stage[kUlStages] = {};
     cudaEvent_t ul_ev[kUlStages] = {};
     std::mutex ul_mu;
+    // Page-locked blocks that group uploads are packed in, taken in turn, and
+    // the events of their copies.
+    char* pack_stage[2] = {};
+    size_t pack_bytes[2] = {};
+    cudaEvent_t pack_ev[2] = {};
+    int pack_turn = 0;
     // Record-only contexts: right-hand-side groups and their DOF counts.
     std::vector<std::shared_ptr<GroupDev>> rhs_record;
     std::vector<int64_t> rhs_record_ndofs;
