@@ -2136,15 +2136,34 @@ static bool uses_split(const GroupDev& g, int precision)
     return precision != SLGPU_PREC_FP64 && !g.rhs && (int64_t)g.ntf * g.ndof >= 64 && split_supported(g);
 }
 
-// Shared memory of k_contract_small for a group (M of every orientation and
-// the block's staged outputs), and whether its FP64 contraction uses it:
-// element matrices of at most 32 entries whose tables fit.
-static size_t small_kernel_smem(const GroupDev& g)
+// Whether a group's FP64 contraction uses k_contract_small: element matrices
+// of at most 32 entries whose tables (M of every orientation, and 128 matrices)
+// take at most 96 KB.
+static bool uses_small_kernel(const GroupDev& g)
 {
     const int64_t P = (int64_t)g.ntf * g.ndof;
-    return ((size_t)g.norient * g.nterms * g.ngp * P + (size_t)kSmallE * (P + 1)) * 8;
+    return P <= kSmallP && ((size_t)g.norient * g.nterms * g.ngp * P + 128 * (size_t)(P + 1)) * 8 <= 96 * 1024;
 }
-static bool uses_small_kernel(const GroupDev& g) { return (int64_t)g.ntf * g.ndof <= kSmallP && small_kernel_smem(g) <= kSmallSmem; }
+
+// Entries per warp: 2, 4 or 8, whichever spreads a matrix over up to 4 warps.
+// Padded to whole parts, M takes at most twice the bound above.
+constexpr size_t kSmallSmem = 200 * 1024;
+
+template <int PP>
+static void launch_small(Ctx* ctx, const GroupDev& g, const ContractParams& kp)
+{
+    static std::once_flag attr;
+    std::call_once(attr, [] { cudaFuncSetAttribute(k_contract_small<PP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallSmem); });
+    const int P = g.ntf * g.ndof, parts = (P + PP - 1) / PP;
+    const size_t smem = ((size_t)g.norient * g.nterms * g.ngp * parts * PP + (size_t)kSmallE * (P + 1)) * 8;
+    // As many blocks as are resident at once, each taking equally many chunks.
+    const int64_t nchunk = (g.nelem + kSmallE - 1) / kSmallE;
+    const int64_t resident = (int64_t)std::max(ctx->nsm, 1) * std::max<int64_t>(1, std::min<int64_t>(kSmallBlocks, (int64_t)(kSmallSmem / smem)));
+    const int64_t each = (nchunk + resident - 1) / resident;
+    k_contract_small<PP><<<(unsigned)((nchunk + each - 1) / each), kSmallE * parts, smem, ctx->x->stream>>>(kp, g.orient.as<int32_t>(), g.norient);
+    cuda_check(cudaGetLastError(), "k_contract_small");
+    ctx->launches++;
+}
 
 // Whether an FP64 contraction of a group may use the mirrored forms (upper
 // triangle of a symmetric group, transposed pairs): matrix groups with at
@@ -2795,7 +2814,6 @@ void launch_contractions(Ctx* ctx, const Matrix& M, int precision, const std::ve
             if (f32)
                 fail(SLGPU_E_STATE, "float element values need every group contracted by the split kernels");
             const int64_t P = (int64_t)g->ntf * g->ndof;
-            const size_t small_smem = small_kernel_smem(*g);
             if (uses_small_kernel(*g)) {
                 ContractParams kp{};
                 kp.tables = g->tables.as<double>();
@@ -2810,14 +2828,14 @@ void launch_contractions(Ctx* ctx, const Matrix& M, int precision, const std::ve
                 kp.C = Cg;
                 kp.tiles = g->tiles_d.as<Tile>();
                 kp.out = vals + gvb[gi];
-                static std::once_flag attr;
-                std::call_once(attr, [] { cudaFuncSetAttribute(k_contract_small, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmem); });
                 const int kt = kstat_start(ctx, "contract_fp64", 2.0 * P * g->nterms * g->ngp * g->nelem);
-                k_contract_small<<<(unsigned)((g->nelem + kSmallE - 1) / kSmallE), kSmallE, small_smem, ctx->x->stream>>>(
-                    kp, g->orient.as<int32_t>(), g->norient);
+                if (P <= 8)
+                    launch_small<2>(ctx, *g, kp);
+                else if (P <= 16)
+                    launch_small<4>(ctx, *g, kp);
+                else
+                    launch_small<8>(ctx, *g, kp);
                 kstat_stop(ctx, kt);
-                cuda_check(cudaGetLastError(), "k_contract_small");
-                ctx->launches++;
             } else {
                 mma_jobs.push_back(MmaJob{g.get(), Cg, vals + gvb[gi], pair[gi] > (int)gi ? vals + gvb[pair[gi]] : nullptr});
             }
