@@ -2074,9 +2074,9 @@ static void contract_split_all(Ctx* ctx, const std::vector<SplitJob>& jobs)
             ops += 2.0 * pairs * needed_rows(g, job_slot(j) >> 1) * g.nterms * g.ngp * g.nelem;
         }
         const int tier = jobs[b0].tier;
-        sp.error = ctx->x->split_error.as<unsigned int>();
+        sp.error = ctx->x->split_flag;
         sp.f32 = jobs[b0].f32 ? 1 : 0;
-        sp.next = reinterpret_cast<unsigned long long*>(ctx->x->split_error.as<char>() + 16);
+        sp.next = ctx->x->split_next.as<unsigned long long>();
         const int kc = kstat_start(ctx, tier == 0 ? "contract_split" : "contract_split_fp32", ops);
         if (tier == 0)
             launch_split<8, 6, 7>(ctx, sp);
@@ -2722,6 +2722,30 @@ static void launch_coefficients(Ctx* ctx, const Matrix& M, const CoefPlan& plan,
     }
 }
 
+// (A flag in device memory, cleared by a memset and read back by a copy each
+// step, took 10 us of it.)
+void ensure_split_state(Ctx* ctx)
+{
+    Exec& x = *ctx->x;
+    if (x.split_flag == nullptr) {
+        cuda_check(cudaHostAlloc(reinterpret_cast<void**>(&x.split_flag), 16, cudaHostAllocMapped), "cudaHostAlloc");
+        *x.split_flag = 0;
+    }
+    if (x.split_next.empty()) {
+        ArenaPause keep(x);
+        x.split_next.alloc(ctx, 16);
+    }
+}
+
+bool split_timed_out(Ctx* ctx)
+{
+    Exec& x = *ctx->x;
+    if (x.split_flag == nullptr || *const_cast<volatile unsigned int*>(x.split_flag) == 0)
+        return false;
+    *x.split_flag = 0;
+    return true;
+}
+
 // Steps 1 and 2 on the current execution state's stream: coefficients of
 // every group (with per-group data overrides, if given), contraction of each
 // group into `vals` at the group's value base, fragment values after them.
@@ -2738,13 +2762,6 @@ bool float_values(const Matrix& M, int precision)
 void launch_contractions(Ctx* ctx, const Matrix& M, int precision, const std::vector<int64_t>& gvb, double* vals,
                          const std::vector<GroupData>* ov, bool f32)
 {
-    if (precision != SLGPU_PREC_FP64) {
-        if (ctx->x->split_error.empty()) {
-            ArenaPause keep(*ctx->x);
-            ctx->x->split_error.alloc(ctx, 32);
-        }
-        cuda_check(cudaMemsetAsync(ctx->x->split_error.as<void>(), 0, 16, ctx->x->stream), "memset");
-    }
     while (ctx->x->evpool.size() < 3) {
         cudaEvent_t e;
         cuda_check(cudaEventCreate(&e), "cudaEventCreate");
@@ -2768,6 +2785,8 @@ void launch_contractions(Ctx* ctx, const Matrix& M, int precision, const std::ve
                                           nullptr, vals + gvb[k], pair[k] >= 0 ? vals + gvb[pair[k]] : nullptr, f32});
             job[k] = &split_jobs.back();
         }
+    if (!split_jobs.empty())
+        ensure_split_state(ctx);
     place_split_jobs(ctx, split_jobs);
     // Coefficients that go through memory ([term][gp][element] per group,
     // all groups side by side), and the high words of the largest ones of
@@ -3125,8 +3144,7 @@ void prepare_value_path(Ctx* ctx, const Matrix& M, int precision)
         x.split_cols.alloc(ctx, colbytes);
     if (x.split_colscale.bytes() < expbytes)
         x.split_colscale.alloc(ctx, expbytes);
-    if (x.split_error.empty())
-        x.split_error.alloc(ctx, 32);
+    ensure_split_state(ctx);
 }
 
 void compile_value_path(Ctx* ctx, const Matrix& M, int precision)
@@ -3172,7 +3190,8 @@ static std::vector<uint64_t> value_signature(Ctx* ctx, const Matrix& M, int prec
     u(ctx->jit_broken ? 1 : 0);
     p(x.split_cols.as<void>());
     p(x.split_colscale.as<void>());
-    p(x.split_error.as<void>());
+    p(x.split_flag);
+    p(x.split_next.as<void>());
     const std::vector<int> pair = cross_pairs(M, precision, nullptr);
     size_t gi = 0;
     for (auto& gp : M.groups) {
@@ -3402,12 +3421,8 @@ static void process_matrix(Ctx* ctx, Matrix& M, const uint8_t* isconstrained, in
     ev_record(ctx, 3);
     cuda_check(cudaEventSynchronize(ctx->x->ev[3]), "sync");
     kstat_collect(ctx);
-    if (precision != SLGPU_PREC_FP64) {
-        unsigned int err = 0;
-        cuda_check(cudaMemcpy(&err, ctx->x->split_error.as<void>(), 4, cudaMemcpyDeviceToHost), "D2H split error");
-        if (err != 0)
-            fail(SLGPU_E_TIMEOUT, "a split-precision contraction tile timed out waiting for its data");
-    }
+    if (split_timed_out(ctx))
+        fail(SLGPU_E_TIMEOUT, "a split-precision contraction tile timed out waiting for its data");
     float coef_ms = 0, contract_ms = 0;
     if (ctx->timers) {
         cudaEventElapsedTime(&coef_ms, ctx->x->evpool[0], ctx->x->evpool[1]);
@@ -3527,7 +3542,9 @@ void slgpu_ctx_destroy(slgpu_ctx* ctx)
     // them must go before the stream does.
     ctx->x->split_cols.release();
     ctx->x->split_colscale.release();
-    ctx->x->split_error.release();
+    ctx->x->split_next.release();
+    if (ctx->x->split_flag != nullptr)
+        cudaFreeHost(ctx->x->split_flag);
     ctx->rhs_record.clear();
     for (cudaLibrary_t lib : ctx->jit_libs) cudaLibraryUnload(lib);
     ctx->jit_libs.clear();

@@ -300,7 +300,11 @@ struct Exec {
     std::vector<std::pair<std::string, double>> kev_tag;   // family, work of each pair
     std::map<std::string, KernelStat> kstats;
     DevBuf split_cols, split_colscale;   // split precision: column slices of the current group
-    DevBuf split_error;                // bytes 0-15: flags set by a timed-out wait; 16-23: split work counter
+    // Split contractions: the flag that a timed-out wait sets (page-locked host
+    // memory that the kernel writes to, so that a step reads it without a
+    // copy), and the work counter.
+    unsigned int* split_flag = nullptr;
+    DevBuf split_next;
     // Page-locked staging for the small uploads of one call (kernel argument
     // arrays), so that they never wait for the stream: reset at the start of
     // each call on this execution state (the previous call has completed).
@@ -429,6 +433,10 @@ void htrace_mark(Ctx* ctx, const char* label);
 // current execution state's split scratch grown to fit them, so that the
 // value path allocates nothing for them.
 void prepare_value_path(Ctx* ctx, const Matrix& M, int precision);
+// The flag and counter of split contractions on the current execution state;
+// whether a wait timed out since the last call (the stream has been synchronised).
+void ensure_split_state(Ctx* ctx);
+bool split_timed_out(Ctx* ctx);
 // Compiles the runtime kernels that the value path takes at this precision.
 void compile_value_path(Ctx* ctx, const Matrix& M, int precision);
 void kstat_stop(Ctx* ctx, int i);

@@ -90,7 +90,6 @@ struct Slot {
     std::shared_ptr<Request> req;
     void* pinned = nullptr;  // staging for inputs and pageable outputs
     size_t pinned_bytes = 0;
-    unsigned int* err_host = nullptr;  // page-locked copy of the split-precision error flag
 };
 
 }  // namespace
@@ -272,9 +271,6 @@ void launch(Server& S, Slot& s, Request& r)
         cuda_check_srv(cudaMemcpyAsync(hA, r.Avals.as<void>(), (size_t)r.nnzA * 8, cudaMemcpyDeviceToHost, st), "D2H Avals");
     if (r.nnzD > 0 && hD != nullptr)
         cuda_check_srv(cudaMemcpyAsync(hD, r.Dvals.as<void>(), (size_t)r.nnzD * 8, cudaMemcpyDeviceToHost, st), "D2H Dvals");
-    *s.err_host = 0;
-    if (r.precision != SLGPU_PREC_FP64 && !s.ex.split_error.empty())
-        cuda_check_srv(cudaMemcpyAsync(s.err_host, s.ex.split_error.as<void>(), 4, cudaMemcpyDeviceToHost, st), "D2H split error");
     cuda_check_srv(cudaEventRecord(s.done, st), "cudaEventRecord");
     htrace_mark(ctx, "request: outputs");
     s.ex.arena_on = false;
@@ -301,7 +297,10 @@ void finish(Server& S, Slot& s)
         float ms = 0;
         cudaEventElapsedTime(&ms, s.start, s.done);
         r.dev_ms = ms;
-        if (*s.err_host != 0) {
+        ctx->x = &s.ex;
+        const bool timed_out = split_timed_out(ctx);
+        ctx->x = &ctx->main;
+        if (timed_out) {
             status = SLGPU_E_TIMEOUT;
             msg = "a split-precision contraction tile timed out waiting for its data";
         }
@@ -486,12 +485,12 @@ int slgpu_server_create(slgpu_ctx* ctx, int nslots, slgpu_server** out)
             return SLGPU_E_CUDA;
         }
         for (auto& e : s.ex.ev) cudaEventCreate(&e);
-        if (cudaHostAlloc(reinterpret_cast<void**>(&s.err_host), 16, cudaHostAllocDefault) != cudaSuccess) {
+        if (cudaHostAlloc(reinterpret_cast<void**>(&s.ex.split_flag), 16, cudaHostAllocMapped) != cudaSuccess) {
             ctx->last_error = "cannot allocate page-locked memory";
             slgpu_server_destroy(S);
             return SLGPU_E_CUDA;
         }
-        *s.err_host = 0;
+        *s.ex.split_flag = 0;
     }
     S->th = std::thread([S] { server_loop(*S); });
     *out = S;
@@ -834,7 +833,7 @@ void slgpu_server_destroy(slgpu_server* S)
         // Slot buffers go before their stream.
         s.ex.split_cols.release();
         s.ex.split_colscale.release();
-        s.ex.split_error.release();
+        s.ex.split_next.release();
         s.ex.arena.release();
         if (s.ex.stream != nullptr)
             cudaStreamSynchronize(s.ex.stream);
@@ -849,8 +848,8 @@ void slgpu_server_destroy(slgpu_server* S)
             cudaEventDestroy(s.done);
         if (s.pinned != nullptr)
             cudaFreeHost(s.pinned);
-        if (s.err_host != nullptr)
-            cudaFreeHost(s.err_host);
+        if (s.ex.split_flag != nullptr)
+            cudaFreeHost(s.ex.split_flag);
         stage_free(s.ex);
         if (s.ex.stream != nullptr)
             cudaStreamDestroy(s.ex.stream);

@@ -92,7 +92,7 @@ struct SplitParams {
     SplitGroup g[kSplitBatch];
     int ngroups;
     int64_t nwork;          // sum of the groups' work items
-    unsigned int* error;    // set on a timed-out wait
+    unsigned int* error;    // set on a timed-out wait (host memory, written only then)
     unsigned long long* next;  // work items handed out after each CTA's first; zero at launch
     int f32;                // out and out2 hold floats (FP32-level steps): same entry order
 };
@@ -501,14 +501,14 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_contract_split(const __gri
         }
         if (!ok) {
             *failed = 1;
-            atomicOr(p.error, 1u);
+            *(volatile unsigned int*)p.error = 1u;
         }
         // No copy may still be in flight when the CTA leaves.
         const int zero = 0;
         for (int s = 0; s < kSt; s++)
             if (used & (1u << s))
                 if (!mbar_wait(&sm.full[s], (last_parity >> s) & 1, &zero))
-                    atomicOr(p.error, 2u);
+                    *(volatile unsigned int*)p.error = 2u;
     } else if (warp == 1 && lane == 0) {
         // ------------------------------------------------ MMA issuer
         int stage = 0;
@@ -566,13 +566,13 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_contract_split(const __gri
         }
         if (!ok) {
             *failed = 1;
-            atomicOr(p.error, 1u);
+            *(volatile unsigned int*)p.error = 1u;
         }
         // Every MMA issued by this thread completes before the TMEM is freed.
         const int zero = 0;
         umma_commit(&sm.drain);
         if (!mbar_wait(&sm.drain, 0, &zero))
-            atomicOr(p.error, 2u);
+            *(volatile unsigned int*)p.error = 2u;
     } else if (warp >= 2) {
         // ------------------------------------------------ epilogue
         // Warp w reads TMEM lane quarter w % 4 and columns c0 .. c0+15 of
@@ -588,7 +588,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_contract_split(const __gri
             const int slot = (int)(k % kSplitItems);
             if (!mbar_wait(&sm.item_full[slot], (k / kSplitItems) & 1, failed)) {
                 *failed = 1;
-                atomicOr(p.error, 1u);
+                *(volatile unsigned int*)p.error = 1u;
                 break;
             }
             const int64_t w = sm.items[slot];
@@ -615,7 +615,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_contract_split(const __gri
             __syncwarp();
             if (!mbar_wait(&sm.tmem_full, (uint32_t)(i & 1), failed)) {
                 *failed = 1;
-                atomicOr(p.error, 1u);
+                *(volatile unsigned int*)p.error = 1u;
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
