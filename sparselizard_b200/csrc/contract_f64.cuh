@@ -14,7 +14,11 @@
 //    symmetric group, or every entry of a group whose transposed partner is
 //    written by the same launch).
 //  * A block computes 64 elements x BP rows (BP = 128 or 64, picked per group
-//    shape by timing); 8 warps of 32 x BP/4 (2 x BP/32 MMA tiles of 16 x 8).
+//    shape by timing); 8 warps of 32 elements x up to BP/32 MMA tiles of 8
+//    rows.  The tiles of a row tile go round its four warps, starting at
+//    another one in each block, and those behind the last row are left out:
+//    the last row tile of 136 rows (order-3 quadrangles) has 8 of them, of
+//    378 and 729 (order-2 hexahedra) 122 and 97.
 //    K advances 16 at a time through a 3-stage cp.async ring of C^T and M^T
 //    tiles in shared memory (rows padded to 68 and BP + 4 doubles so that the
 //    fragment loads of a half-warp hit distinct banks).
@@ -101,7 +105,8 @@ struct MmaGroup {
     int sectors;             // stores of 4 values, on sectors
     int Q, Qpad, rpad;
     int es, es2;         // values per element matrix of out, of out2
-    int nrt;             // row tiles (rpad / BP)
+    int nrt;             // row tiles of BP
+    int rows;            // rows up to the last one that holds an entry
     int w0;              // first block of the group in the launch
     int64_t nelem;
     double* out;         // [nelem][es]
@@ -152,7 +157,9 @@ __global__ void __launch_bounds__(256, 2) k_contract_f64mma(const __grid_constan
     const int r0 = rt * BP;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int gid = lane >> 2, tig = lane & 3;
-    const int we = warp >> 2, wr = warp & 3;  // warp's 32 elements and BP/4 rows
+    // The warp's 32 elements, and its MMA tiles: rows 32 n + 8 wr .. + 7 for n < nt.
+    const int we = warp >> 2, wr = (warp + (int)blockIdx.x) & 3;
+    const int live = min(p.rows - r0, BP), nt = max(0, (live - 8 * wr + 31) >> 5);
     const double* Mt = p.Mt + (int64_t)tile.orient * p.Qpad * p.rpad + r0;
     const int nchunks = p.Qpad / kMmaBQ;
 
@@ -174,7 +181,8 @@ __global__ void __launch_bounds__(256, 2) k_contract_f64mma(const __grid_constan
         for (int k = 0; k < (kMmaBQ * BP) / (2 * 256); k++) {
             const int idx = tid + 256 * k;
             const int row = idx / (BP / 2), c2 = idx % (BP / 2);
-            cp_async16(Ms + row * Sh::MS + 2 * c2, Mt + (int64_t)(q0 + row) * p.rpad + 2 * c2);
+            if (2 * c2 < ((live + 7) & ~7))
+                cp_async16(Ms + row * Sh::MS + 2 * c2, Mt + (int64_t)(q0 + row) * p.rpad + 2 * c2);
         }
     };
 
@@ -215,16 +223,29 @@ __global__ void __launch_bounds__(256, 2) k_contract_f64mma(const __grid_constan
                 a[m][2] = Cs[(ks + tig + 4) * kMmaCS + e];
                 a[m][3] = Cs[(ks + tig + 4) * kMmaCS + e + 8];
             }
+            if (nt == NT) {
 #pragma unroll
-            for (int n = 0; n < NT; n++) {
-                const int r = wr * (8 * NT) + n * 8 + gid;
-                b[n][0] = Ms[(ks + tig) * Sh::MS + r];
-                b[n][1] = Ms[(ks + tig + 4) * Sh::MS + r];
+                for (int n = 0; n < NT; n++) {
+                    const int r = n * 32 + wr * 8 + gid;
+                    b[n][0] = Ms[(ks + tig) * Sh::MS + r];
+                    b[n][1] = Ms[(ks + tig + 4) * Sh::MS + r];
+                }
+#pragma unroll
+                for (int m = 0; m < 2; m++)
+#pragma unroll
+                    for (int n = 0; n < NT; n++) dmma_16x8x8(acc[m][n], a[m], b[n]);
+            } else {
+#pragma unroll
+                for (int n = 0; n < NT - 1; n++) {
+                    if (n >= nt)
+                        break;
+                    const int r = n * 32 + wr * 8 + gid;
+                    b[n][0] = Ms[(ks + tig) * Sh::MS + r];
+                    b[n][1] = Ms[(ks + tig + 4) * Sh::MS + r];
+#pragma unroll
+                    for (int m = 0; m < 2; m++) dmma_16x8x8(acc[m][n], a[m], b[n]);
+                }
             }
-#pragma unroll
-            for (int m = 0; m < 2; m++)
-#pragma unroll
-                for (int n = 0; n < NT; n++) dmma_16x8x8(acc[m][n], a[m], b[n]);
         }
     }
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
@@ -238,7 +259,7 @@ __global__ void __launch_bounds__(256, 2) k_contract_f64mma(const __grid_constan
             const int e = we * 32 + m * 16 + gid + 8 * h;
 #pragma unroll
             for (int n = 0; n < NT; n++)
-                *reinterpret_cast<double2*>(sm_mma + e * Sh::OS + wr * (8 * NT) + n * 8 + 2 * tig) =
+                *reinterpret_cast<double2*>(sm_mma + e * Sh::OS + n * 32 + wr * 8 + 2 * tig) =
                     make_double2(acc[m][n][2 * h], acc[m][n][2 * h + 1]);
         }
     __syncthreads();

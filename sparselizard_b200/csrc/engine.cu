@@ -2279,6 +2279,9 @@ static GroupDev::Fp64Mt& ensure_fmt(Ctx* ctx, GroupDev& g, int form)
         const StorePlan plan = store_plan(g, form);
         f->Qpad = (Q + kMmaBQ - 1) / kMmaBQ * kMmaBQ;
         f->rpad = ((int)plan.entry.size() + kMmaBPMax - 1) / kMmaBPMax * kMmaBPMax;
+        for (int r = 0; r < (int)plan.entry.size(); r++)
+            if (plan.entry[r] >= 0)
+                f->rows = r + 1;
         f->sectors = plan.sectors;
         f->nops = (int)plan.ops.size();
         std::vector<int32_t> all(sizeof(StoreOp) / 4 * plan.ops.size());
@@ -2362,7 +2365,8 @@ static void run_mma_jobs(Ctx* ctx, const std::vector<MmaJob>& jobs, int BP)
             GroupDev& g = *j.g;
             const int form = mma_form(j);
             GroupDev::Fp64Mt& f = ensure_fmt(ctx, g, form);
-            const int64_t n = (int64_t)g.tiles.size() * (f.rpad / BP);
+            const int nrt = (f.rows + BP - 1) / BP;
+            const int64_t n = (int64_t)g.tiles.size() * nrt;
             if (n > INT32_MAX)
                 fail(SLGPU_E_UNSUPPORTED, "group too large for one FP64 contraction launch");
             if (nblocks + n > INT32_MAX)
@@ -2379,7 +2383,8 @@ static void run_mma_jobs(Ctx* ctx, const std::vector<MmaJob>& jobs, int BP)
             G.rpad = f.rpad;
             G.es = g.ntf * g.ld;
             G.es2 = form == 2 ? g.ndof * row_stride(g.ndof, g.ntf) : G.es;
-            G.nrt = f.rpad / BP;
+            G.nrt = nrt;
+            G.rows = f.rows;
             G.w0 = (int)nblocks;
             G.nelem = g.nelem;
             G.out = j.out;

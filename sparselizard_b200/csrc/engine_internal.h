@@ -157,6 +157,7 @@ struct GroupDev {
     // of a symmetric group, 2 every entry with its transposed partner's).
     struct Fp64Mt {
         int Qpad = 0, rpad = 0;
+        int rows = 0;          // rows up to the last one that holds an entry
         bool sectors = false;  // stores of 4 values (else single ones)
         DevBuf Mt;
         DevBuf plan;  // StoreOp [nops], then int32 [rpad / kMmaBin + 1] first store of each bin, then int32 [rpad] entries
