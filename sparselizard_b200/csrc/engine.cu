@@ -2992,10 +2992,12 @@ void launch_thread_rows(Ctx* ctx, const RowParams& rp, bool f32)
 
 void launch_warp_rows(Ctx* ctx, RowParams rp, bool f32)
 {
-    // Consecutive rows per warp: up to kRowsPerWarp (the row buffer stays
-    // clean between them), fewer when the rows are too few to fill the
-    // device with about 48 warps per multiprocessor.
-    const int64_t target = (int64_t)std::max(ctx->nsm, 1) * 48;
+    // Consecutive rows per warp: up to kRowsPerWarp, fewer where that leaves
+    // less than six times the warps that are resident: rows differ in length,
+    // and the last warps run alone.  (One, four, eight, 16 times: tetrahedra of
+    // FP32 elasticity 0.29, 0.117, 0.121, 0.120 ms; order-3 quadrangles 53, 43,
+    // 49, 65 us; order-2 edge elements 0.354, 0.346, 0.342, 0.350 ms.)
+    const int64_t target = (int64_t)std::max(ctx->nsm, 1) * kRowBlocks * 8 * 6;
     rp.rows_per_warp = (int)std::min<int64_t>(kRowsPerWarp, std::max<int64_t>(1, rp.nrows / target));
     const size_t per_warp = (size_t)rp.lmax * 8;
     int wpb = (int)std::max<size_t>(1, std::min<size_t>(8, (48 * 1024) / per_warp));

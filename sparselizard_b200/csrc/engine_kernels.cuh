@@ -1121,20 +1121,31 @@ struct RowParams {
     int uniform_width;  // every segment this width (<= 32) with multiplier 1, else 0
 };
 
-// CSR values, one warp per row: the row's incidences are visited in a fixed
-// order and each adds its element-matrix row (contiguous in the element-major
-// value buffer) into a shared-memory copy of the row through the slot map.
-// Within one incidence every lane hits a different slot, so the sum of each
-// CSR entry is formed in incidence order: deterministic, no atomics.
+// CSR values, a warp's rows one after another: the incidences are visited in a
+// fixed order and each adds its element-matrix row (contiguous in the
+// element-major value buffer) into a shared-memory copy of its CSR row through
+// the slot map.  Within one incidence every lane hits a different slot, so the
+// sum of each CSR entry is formed in incidence order: deterministic, no atomics.
 //
-// Lane l decodes incidence l of each group of 32 (segment lookup, value and
-// slot offsets) once; the other lanes receive it by shuffle.  The loads of
-// kRowBatch incidences are issued before any of them is added (lane j holds
-// entry j of each), so a warp keeps that many element-matrix rows in flight;
-// the additions still run in incidence order.  Incidences flagged serial
-// (duplicate addresses) or wider than a warp are added by their own loop at
-// their place in the order.
+// The incidences of consecutive rows follow one another, so the warp takes
+// them 32 at a time whatever rows they belong to: lane l decodes incidence l
+// (segment lookup, value and slot offsets), its word loaded a window ahead, and
+// the other lanes receive it by shuffle.  The loads of kRowBatch incidences are
+// issued before any of them is added (lane j holds entry j of each); the
+// additions run in incidence order, a finished row being written back between
+// them.  Incidences flagged serial (duplicate addresses) or wider than a warp
+// are added by their own loop at their place in the order.
+//
+// Latency bounds the kernel: rows have 2 (order-3 quadrangles) to 10 (order-2
+// elasticity) incidences, and a window per row left most of its lanes and half
+// of its last batch idle.  22,201 order-3 quadrangles 66 -> 44 us, 27^3 order-2
+// hexahedra 0.61 -> 0.52 ms, order-2 edge elements on 48,000 tetrahedra 0.40 ->
+// 0.34 ms, FP32 elasticity on 16,464 tetrahedra 0.21 -> 0.12 ms; 48^3 hexahedra,
+// whose gathers of 216 and 54 bytes keep memory busy at 4 TB/s, 2.8 ms either
+// way.  (Batches of 5 and 6 with 64 registers, four blocks: within 10 %
+// either way, no better on average.)
 constexpr int kRowBatch = 4;
+constexpr int kRowBlocks = 5;  // resident blocks of 8 warps per multiprocessor (48 registers)
 
 template <class V>
 __device__ __forceinline__ void row_add_generic(double* buf, int width, double mult, const V* v, const int16_t* sm, bool serial,
@@ -1207,7 +1218,7 @@ __global__ void __launch_bounds__(kThreadRows) k_row_thread(RowParams p)
 constexpr int kRowsPerWarp = 31;
 
 template <class V, bool U>
-__global__ void __launch_bounds__(256, 6) k_row_values(RowParams p)
+__global__ void __launch_bounds__(256, kRowBlocks) k_row_values(RowParams p)
 {
     const V* vals = reinterpret_cast<const V*>(p.vals);
     constexpr long long kScale = sizeof(double) / sizeof(V);  // values of type V per double of the buffer
@@ -1229,88 +1240,16 @@ __global__ void __launch_bounds__(256, 6) k_row_values(RowParams p)
     }
     __syncwarp();
     constexpr uint32_t kGeneric = 1u << 17, kSerial = 1u << 16;
-    for (int rr = 0; rr < nr; rr++) {
-        // The CSR bounds are fetched after the incidences (only the
-        // write-back needs them): fewer registers live in the loop below.
-        const uint32_t k0 = __shfl_sync(0xffffffffu, i_lo, rr), k1 = __shfl_sync(0xffffffffu, i_lo, rr + 1);
-        for (uint32_t kb = k0; kb < k1; kb += 32) {
-            const int nkb = (int)min(32u, k1 - kb);
-            // Lane l decodes incidence kb + l.  COO offsets fit 32 bits (fewer
-            // than 2^32 COO entries per matrix); value offsets, with their
-            // row strides, 32 bits in the uniform form and 46 otherwise.
-            uint32_t voff = 0, coo = 0;
-            double mult = 0.0;
-            uint32_t info = 0;  // width | kSerial | kGeneric | value offset bits 32 .. 45 from bit 18
-            if (lane < nkb) {
-                const unsigned long long pk = p.inc[kb + lane];
-                const RowSeg sg = p.segs[(pk >> 40) & ((1ull << 23) - 1)];
-                const uint32_t n = (uint32_t)pk;  // fewer than 2^32 incidences
-                coo = (uint32_t)sg.coo_base + n * (uint32_t)sg.width;
-                const uint64_t v = (uint64_t)sg.val_base * kScale + (uint64_t)n * (uint32_t)sg.ld;
-                voff = (uint32_t)v;
-                mult = sg.mult;
-                const bool serial = (pk >> 63) != 0;
-                info = (uint32_t)sg.width | (serial ? kSerial : 0) | ((serial || sg.width > 32) ? kGeneric : 0) |
-                       (uint32_t)(v >> 32) << 18;
-            }
-            if (!__any_sync(0xffffffffu, (info & kGeneric) != 0)) {
-                // Batches of kRowBatch incidences: every load issued before
-                // the ordered additions.
-                for (int u = 0; u < nkb; u += kRowBatch) {
-                    double val[kRowBatch];
-                    int slot[kRowBatch];
-#pragma unroll
-                    for (int x = 0; x < kRowBatch; x++) {
-                        const int src = (u + x) & 31;
-                        uint64_t vo = __shfl_sync(0xffffffffu, voff, src);
-                        const uint32_t co = __shfl_sync(0xffffffffu, coo, src);
-                        int w = p.uniform_width;
-                        if constexpr (!U) {
-                            const uint32_t inf = __shfl_sync(0xffffffffu, info, src);
-                            w = (int)(inf & 0xffff);
-                            vo |= (uint64_t)(inf >> 18) << 32;
-                        }
-                        slot[x] = -1;
-                        val[x] = 0.0;
-                        if (u + x < nkb && lane < w) {
-                            slot[x] = p.slotmap[(uint64_t)co + lane];
-                            val[x] = (double)vals[vo + lane];
-                        }
-                    }
-#pragma unroll
-                    for (int x = 0; x < kRowBatch; x++) {
-                        if (u + x < nkb) {
-                            if constexpr (U) {
-                                // Multiplier 1: val + buf is fma(val, 1, buf) bit for bit.
-                                if (slot[x] >= 0)
-                                    buf[slot[x]] = val[x] + buf[slot[x]];
-                            } else {
-                                const double m = __shfl_sync(0xffffffffu, mult, (u + x) & 31);
-                                if (slot[x] >= 0)
-                                    buf[slot[x]] = fma(val[x], m, buf[slot[x]]);
-                            }
-                            __syncwarp();
-                        }
-                    }
-                }
-            } else {
-                for (int x = 0; x < nkb; x++) {
-                    const uint32_t inf = __shfl_sync(0xffffffffu, info, x);
-                    const uint64_t vo = __shfl_sync(0xffffffffu, voff, x) | (uint64_t)(inf >> 18) << 32;
-                    const uint32_t co = __shfl_sync(0xffffffffu, coo, x);
-                    const double m = __shfl_sync(0xffffffffu, mult, x);
-                    row_add_generic(buf, (int)(inf & 0xffff), m, vals + vo, p.slotmap + co, (inf & kSerial) != 0, lane);
-                    __syncwarp();
-                }
-            }
-        }
+    const uint32_t K0 = __shfl_sync(0xffffffffu, i_lo, 0), K1 = __shfl_sync(0xffffffffu, i_lo, nr);
+    int rr = 0;                                             // the row being summed
+    uint32_t kend = __shfl_sync(0xffffffffu, i_lo, 1);      // its incidences end here
+    auto write_back = [&] {
         const uint32_t a0 = __shfl_sync(0xffffffffu, a_lo, rr), a1 = __shfl_sync(0xffffffffu, a_lo, rr + 1);
         const uint32_t d0 = __shfl_sync(0xffffffffu, d_lo, rr), d1 = __shfl_sync(0xffffffffu, d_lo, rr + 1);
         const int la = (int)(a1 - a0), L = la + (int)(d1 - d0);
-        const int64_t r = r0 + rr;
         if (p.dense != nullptr) {
             if (lane == 0)
-                p.dense[r] = L > 0 ? -buf[0] : 0.0;
+                p.dense[r0 + rr] = L > 0 ? -buf[0] : 0.0;
             __syncwarp();
             for (int s = lane; s < L; s += 32) buf[s] = 0.0;
         } else {
@@ -1324,7 +1263,84 @@ __global__ void __launch_bounds__(256, 6) k_row_values(RowParams p)
             }
         }
         __syncwarp();
+        rr++;
+        kend = __shfl_sync(0xffffffffu, i_lo, (rr + 1) & 31);
+    };
+    unsigned long long pk = K0 + lane < K1 ? p.inc[K0 + lane] : 0;
+    for (uint32_t kb = K0; kb < K1; kb += 32) {
+        const int nkb = (int)min(32u, K1 - kb);
+        // Lane l decodes incidence kb + l.  COO offsets fit 32 bits (fewer
+        // than 2^32 COO entries per matrix); value offsets, with their
+        // row strides, 32 bits in the uniform form and 46 otherwise.
+        uint32_t voff = 0, coo = 0;
+        double mult = 0.0;
+        uint32_t info = 0;  // width | kSerial | kGeneric | value offset bits 32 .. 45 from bit 18
+        if (lane < nkb) {
+            const RowSeg sg = p.segs[(pk >> 40) & ((1ull << 23) - 1)];
+            const uint32_t n = (uint32_t)pk;  // fewer than 2^32 incidences
+            coo = (uint32_t)sg.coo_base + n * (uint32_t)sg.width;
+            const uint64_t v = (uint64_t)sg.val_base * kScale + (uint64_t)n * (uint32_t)sg.ld;
+            voff = (uint32_t)v;
+            mult = sg.mult;
+            const bool serial = (pk >> 63) != 0;
+            info = (uint32_t)sg.width | (serial ? kSerial : 0) | ((serial || sg.width > 32) ? kGeneric : 0) | (uint32_t)(v >> 32) << 18;
+        }
+        if (kb + 32 + lane < K1)
+            pk = p.inc[kb + 32 + lane];
+        if (!__any_sync(0xffffffffu, (info & kGeneric) != 0)) {
+            // Batches of kRowBatch incidences: every load issued before
+            // the ordered additions.
+            for (int u = 0; u < nkb; u += kRowBatch) {
+                double val[kRowBatch];
+                int slot[kRowBatch];
+#pragma unroll
+                for (int x = 0; x < kRowBatch; x++) {
+                    const int src = (u + x) & 31;
+                    uint64_t vo = __shfl_sync(0xffffffffu, voff, src);
+                    const uint32_t co = __shfl_sync(0xffffffffu, coo, src);
+                    int w = p.uniform_width;
+                    if constexpr (!U) {
+                        const uint32_t inf = __shfl_sync(0xffffffffu, info, src);
+                        w = (int)(inf & 0xffff);
+                        vo |= (uint64_t)(inf >> 18) << 32;
+                    }
+                    slot[x] = -1;
+                    val[x] = 0.0;
+                    if (u + x < nkb && lane < w) {
+                        slot[x] = p.slotmap[(uint64_t)co + lane];
+                        val[x] = (double)vals[vo + lane];
+                    }
+                }
+#pragma unroll
+                for (int x = 0; x < kRowBatch; x++) {
+                    if (u + x < nkb) {
+                        while (kb + u + x >= kend) write_back();
+                        if constexpr (U) {
+                            // Multiplier 1: val + buf is fma(val, 1, buf) bit for bit.
+                            if (slot[x] >= 0)
+                                buf[slot[x]] = val[x] + buf[slot[x]];
+                        } else {
+                            const double m = __shfl_sync(0xffffffffu, mult, (u + x) & 31);
+                            if (slot[x] >= 0)
+                                buf[slot[x]] = fma(val[x], m, buf[slot[x]]);
+                        }
+                        __syncwarp();
+                    }
+                }
+            }
+        } else {
+            for (int x = 0; x < nkb; x++) {
+                while (kb + x >= kend) write_back();
+                const uint32_t inf = __shfl_sync(0xffffffffu, info, x);
+                const uint64_t vo = __shfl_sync(0xffffffffu, voff, x) | (uint64_t)(inf >> 18) << 32;
+                const uint32_t co = __shfl_sync(0xffffffffu, coo, x);
+                const double m = __shfl_sync(0xffffffffu, mult, x);
+                row_add_generic(buf, (int)(inf & 0xffff), m, vals + vo, p.slotmap + co, (inf & kSerial) != 0, lane);
+                __syncwarp();
+            }
+        }
     }
+    while (rr < nr) write_back();
 }
 
 }  // namespace slgpu

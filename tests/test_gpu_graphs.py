@@ -144,6 +144,59 @@ def test_value_kernels_agree(tmp_path):
             assert np.array_equal(a, b), f"{key}: {k} and warp-per-row value kernels differ"
 
 
+@pytest.mark.parametrize("grid,ndofs,mult,dup", [(60, 3000, 1.0, False), (200, 30000, 3.0, True), (400, 150000, 1.0, True),
+                                                 (400, 150000, -2.5, False), (600, 1200000, 1.0, False)])
+def test_rows_of_a_warp(tmp_path, grid, ndofs, mult, dup):
+    """1 to 31 rows per warp, rows of one to thousands of incidences that start
+    and end anywhere in a window of 32, with and without serial incidences and
+    multipliers: the warp kernel's values equal the streaming kernel's bit for
+    bit (each forced in its own process)."""
+    import os
+    import subprocess
+    import sys
+
+    code = """
+import ctypes, sys
+import numpy as np
+import _synthetic as S
+from sparselizard_b200 import abi
+rng = np.random.Generator(np.random.PCG64(41))
+grid, ndofs, mult, dup = %d, %d, %r, %r
+gb, xyz, conn = S.group(rng, nelem_grid=grid, ntf=4, ndof=4, nterms=1, ngp1=2, norient=1, ndests=1, ndofs=ndofs)
+g = gb.g
+g.dests[0].multiplier = mult
+t = np.ctypeslib.as_array(g.dests[0].tfaddr, (4, g.nelem))
+d = np.ctypeslib.as_array(g.dests[0].dofaddr, (4, g.nelem))
+d[:] = (t[::-1] // 16 * 16 + rng.integers(0, 16, d.shape)) %% ndofs  # rows stay short
+t[:, ::97] = rng.integers(0, 40, t[:, ::97].shape)  # and some have many incidences
+if dup:
+    d[1, ::13] = d[0, ::13]
+ctx = abi.Context(0)
+L = ctx.lib
+ctx.check(L.slgpu_mesh_set_nodes(ctx.h, 0, xyz.size // 3, abi.f64p(xyz)))
+ctx.check(L.slgpu_mesh_set_elements(ctx.h, 0, 3, 4, conn.size // 4, abi.i32p(conn)))
+h = ctypes.c_int()
+ctx.check(L.slgpu_matrix_create(ctx.h, ndofs, ctypes.byref(h)))
+ctx.check(L.slgpu_matrix_add_group(ctx.h, h, ctypes.byref(g), None))
+con = (rng.random(ndofs) < 0.05).astype(np.uint8)
+info = abi.CsrInfo()
+ctx.check(L.slgpu_matrix_process(ctx.h, h, con.ctypes.data_as(ctypes.POINTER(ctypes.c_uint8)), abi.PREC_FP64, ctypes.byref(info)))
+A, D = np.zeros(max(1, info.nnzA)), np.zeros(max(1, info.nnzD))
+ctx.check(L.slgpu_matrix_download_values(ctx.h, h, abi.f64p(A), abi.f64p(D)))
+np.savez(sys.argv[1], A=A, D=D)
+""" % (grid, ndofs, mult, dup)
+    here = os.path.dirname(os.path.abspath(__file__))
+    res = {}
+    for k in ("stream", "warp"):
+        out = str(tmp_path / f"{k}.npz")
+        env = dict(os.environ, SLGPU_ROW_KERNEL=k, PYTHONPATH=os.pathsep.join([here, os.path.dirname(here)]))
+        subprocess.run([sys.executable, "-c", code, out], env=env, check=True, timeout=300)
+        res[k] = np.load(out)
+    for key in ("A", "D"):
+        assert np.all(np.isfinite(res["warp"][key])) and np.abs(res["warp"][key]).max() > 0
+        assert np.array_equal(res["warp"][key], res["stream"][key]), key
+
+
 def test_graph_replay_with_transposed_pair(ctx):
     """A matrix with two transposed-partner groups, edited so that the pairing
     turns off and on again (a scale of one group; element data of one group,
