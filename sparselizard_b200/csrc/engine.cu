@@ -164,9 +164,11 @@ static void h2d_pageable(Ctx* ctx, void* dst, const void* src, size_t n)
         fail(SLGPU_E_CUDA, err);
 }
 
-// From this size on a pageable array goes through the page-locked ring: its
-// threads cost about 0.2 ms, the driver's own staging copies about 6 GB/s.
-constexpr size_t kRingBytes = size_t(2) << 20;
+// From this size on a pageable array goes through the page-locked ring: below
+// it the ring's few chunks and its threads cost more than the driver's own
+// staging (a group with 5.1 MB of addresses added in 2.2 ms, in 2.7 through the
+// ring, in 2.6 through the ring in eight smaller chunks).
+constexpr size_t kRingBytes = size_t(8) << 20;
 
 static void copy_h2d(Ctx* ctx, void* dst, const void* src, size_t bytes)
 {
