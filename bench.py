@@ -306,9 +306,9 @@ def run_reference(args, spec):
     print(json.dumps(line), flush=True)
 
 
-KERNEL_NAMES = {"coefficients": "slgpu_coef (runtime-compiled)", "contract_fp64": "k_contract_fp64 / k_contract_small",
-                "slice_cols": "k_slice_cols", "contract_split": "k_contract_split<7,8>",
-                "contract_split_fp32": "k_contract_split<5,6>", "row_values": "k_row_values / k_row_stream (chosen per pattern)"}
+KERNEL_NAMES = {"coefficients": "slgpu_coef (runtime-compiled)", "contract_fp64": "k_contract_f64mma / k_contract_small",
+                "slice_cols": "slgpu_slices (runtime-compiled) / k_slice_cols", "contract_split": "k_contract_split<8,6,7>",
+                "contract_split_fp32": "k_contract_split<7,5,6>", "row_values": "k_row_values / k_row_stream (chosen per pattern)"}
 
 
 def int8_peak_tops(sustained_s=2.0):
