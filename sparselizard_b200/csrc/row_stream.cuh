@@ -5,9 +5,8 @@
 // src/formulation/rawmat.cpp:67-125 and 221-299) is a gather of element-matrix
 // rows: every incidence of a CSR row is a contiguous run of `width` element
 // values (element-major buffer) plus the run of their 16-bit row slots.  The
-// one-row-per-warp kernel (k_row_values) issues those gathers a few at a time
-// and waits on each batch, so for short rows of long incidences it is bound
-// by DRAM latency.  Here a warp owns chunks of consecutive rows (chunk c,
+// warp kernel (k_row_values) issues those gathers a batch at a time into
+// registers and waits on each batch.  Here a warp owns chunks of consecutive rows (chunk c,
 // c + W, c + 2W, ... for warp c of W) and keeps R incidences of its stream in
 // flight: entry k % R of the ring receives incidence k's values and slots
 // (16-byte aligned supersets of the two runs, copied 16 bytes per lane with
