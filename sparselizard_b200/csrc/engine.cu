@@ -3176,7 +3176,7 @@ ValueGraph::~ValueGraph()
 // kernel handles and sizes.  Contents that can change in place (per-element
 // data, field data, term scales, the destination multipliers of the resident
 // segment array, node coordinates) are read by the kernels at run time and
-// are not part of it.  A group's own buffers and sizes are fixed at creation,
+// are not part of it, but for whether every multiplier is 1.  A group's own buffers and sizes are fixed at creation,
 // so its serial number stands for them.
 static std::vector<uint64_t> value_signature(Ctx* ctx, const Matrix& M, int precision, bool rhs, const Pattern& P,
                                              const std::vector<Segment>& segs)
@@ -3236,10 +3236,14 @@ static std::vector<uint64_t> value_signature(Ctx* ctx, const Matrix& M, int prec
         u((uint64_t)f->nr);
         u((uint64_t)f->nc);
     }
+    // Multipliers that are all 1 are part of the value kernel's launch.
+    bool unit = true;
     for (const Segment& sg : segs) {
         u((uint64_t)sg.coo_base);
         u((uint64_t)sg.val_base);
+        unit = unit && sg.mult == 1.0;
     }
+    u(unit ? 1 : 0);
     return s;
 }
 

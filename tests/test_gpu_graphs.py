@@ -383,3 +383,37 @@ def test_pattern_row_sizes(ctx, per_row, ndof, ndofs):
     for k in ("Avals", "Dvals"):
         err = np.abs(out[k][: ref[k].size] - ref[k]) / np.maximum(mag[k], 1e-300)
         assert not err.size or err.max() <= 1e-12, f"{k}: {err.max():.3e}"
+
+
+def test_graph_follows_unit_multipliers(tmp_path):
+    """Destination multipliers that are all 1 when the step is captured and
+    then are not: the warp value kernel, which takes multipliers of 1 from the
+    launch, is captured anew.  Doubled multipliers give exactly doubled values,
+    and the first values come back with the first multipliers."""
+    import os
+    import subprocess
+    import sys
+
+    code = """
+import sys
+import numpy as np
+from sparselizard_b200 import abi
+import test_gpu_graphs as T
+ctx = abi.Context(0)
+t = T._setup(ctx, np.random.Generator(np.random.PCG64(51)), 61, 30, 9, 9, 2, 2, 900)
+n, out = t["ndests"], {}
+for k, mult in enumerate([1.0] * 4 + [2.0] * 4 + [1.0] * 2):
+    ctx.check(ctx.lib.slgpu_matrix_set_scales(ctx.h, t["h"], 0, None, abi.f64p(np.full(n, mult))))
+    out["A%d" % k], out["D%d" % k] = T._process(ctx, t, abi.PREC_FP64)
+assert ctx.lib.slgpu_graph_launches(ctx.h) >= 4
+np.savez(sys.argv[1], **out)
+"""
+    here = os.path.dirname(os.path.abspath(__file__))
+    out = str(tmp_path / "m.npz")
+    env = dict(os.environ, SLGPU_ROW_KERNEL="warp", PYTHONPATH=os.pathsep.join([here, os.path.dirname(here)]))
+    subprocess.run([sys.executable, "-c", code, out], env=env, check=True, timeout=300)
+    r = np.load(out)
+    for b in "AD":
+        assert np.abs(r[b + "0"]).max() > 0
+        for k in range(10):
+            assert np.array_equal(r[f"{b}{k}"], r[b + "0"] * (2.0 if 4 <= k < 8 else 1.0)), f"{b}, call {k}"
