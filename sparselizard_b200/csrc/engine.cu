@@ -2079,6 +2079,7 @@ static void contract_split_all(Ctx* ctx, const std::vector<SplitJob>& jobs)
         sp.error = ctx->x->split_flag;
         sp.f32 = jobs[b0].f32 ? 1 : 0;
         sp.next = ctx->x->split_next.as<unsigned long long>();
+        ctx->x->split_queued = true;
         const int kc = kstat_start(ctx, tier == 0 ? "contract_split" : "contract_split_fp32", ops);
         if (tier == 0)
             launch_split<8, 6, 7>(ctx, sp);
@@ -2744,9 +2745,24 @@ void ensure_split_state(Ctx* ctx)
     }
 }
 
+// A call that threw between queueing a contraction and reading the flag leaves
+// both behind: that contraction is waited for first.
+void split_begin(Ctx* ctx)
+{
+    Exec& x = *ctx->x;
+    if (x.split_flag == nullptr)
+        return;
+    if (x.split_queued) {
+        cuda_check(cudaStreamSynchronize(x.stream), "sync");
+        x.split_queued = false;
+    }
+    *const_cast<volatile unsigned int*>(x.split_flag) = 0;
+}
+
 bool split_timed_out(Ctx* ctx)
 {
     Exec& x = *ctx->x;
+    x.split_queued = false;
     if (x.split_flag == nullptr || *const_cast<volatile unsigned int*>(x.split_flag) == 0)
         return false;
     *x.split_flag = 0;
@@ -3308,6 +3324,7 @@ static void process_matrix(Ctx* ctx, Matrix& M, const uint8_t* isconstrained, in
 {
     htrace_begin(ctx);
     ctx->x->kev_tag.clear();
+    split_begin(ctx);
     stage_reset(*ctx->x);
     if (ctx->record_only) {
         if (isconstrained != nullptr)
@@ -3417,6 +3434,7 @@ static void process_matrix(Ctx* ctx, Matrix& M, const uint8_t* isconstrained, in
         }
         if (M.vgraph) {
             cuda_check(cudaGraphLaunch(M.vgraph->exec, ctx->x->stream), "cudaGraphLaunch");
+            ctx->x->split_queued = precision != SLGPU_PREC_FP64;
             ctx->x->kev_tag = M.vgraph->kev_tag;
             ctx->launches += M.vgraph->launches;
             ctx->graph_launches++;

@@ -305,6 +305,7 @@ struct Exec {
     // memory that the kernel writes to, so that a step reads it without a
     // copy), and the work counter.
     unsigned int* split_flag = nullptr;
+    bool split_queued = false;  // contractions queued since the flag was read
     DevBuf split_next;
     // Page-locked staging for the small uploads of one call (kernel argument
     // arrays), so that they never wait for the stream: reset at the start of
@@ -435,8 +436,10 @@ void htrace_mark(Ctx* ctx, const char* label);
 // value path allocates nothing for them.
 void prepare_value_path(Ctx* ctx, const Matrix& M, int precision);
 // The flag and counter of split contractions on the current execution state;
-// whether a wait timed out since the last call (the stream has been synchronised).
+// the flag cleared, before a call queues any; whether a wait of the call timed
+// out (the stream has been synchronised).
 void ensure_split_state(Ctx* ctx);
+void split_begin(Ctx* ctx);
 bool split_timed_out(Ctx* ctx);
 // Compiles the runtime kernels that the value path takes at this precision.
 void compile_value_path(Ctx* ctx, const Matrix& M, int precision);

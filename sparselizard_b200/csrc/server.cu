@@ -167,6 +167,7 @@ void launch(Server& S, Slot& s, Request& r)
     Pattern& P = *M.pattern;
     const double t0 = S.now();
     ctx->x = &s.ex;
+    split_begin(ctx);
     stage_reset(s.ex);
     htrace_begin(ctx);
     cudaStream_t st = s.ex.stream;
