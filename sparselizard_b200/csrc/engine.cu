@@ -186,6 +186,22 @@ static void copy_h2d(Ctx* ctx, void* dst, const void* src, size_t bytes)
     cuda_check(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->x->stream), "cudaMemcpyAsync H2D");
 }
 
+// Most dynamic shared memory of a block.
+constexpr size_t kSmemMax = 227 * 1024;
+
+// Raises a kernel's dynamic shared-memory limit.  The limit belongs to the
+// device, so every context does it once for its own; always to the same number
+// of bytes, so that contexts on one device do not lower it for each other.
+template <class K>
+static void raise_smem(Ctx* ctx, K* kernel, size_t bytes)
+{
+    const void* f = reinterpret_cast<const void*>(kernel);
+    if (ctx->smem_raised.count(f) != 0)
+        return;
+    cuda_check(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes), "shared-memory limit");
+    ctx->smem_raised.insert(f);
+}
+
 template <class T>
 static void upload(Ctx* ctx, DevBuf& buf, const T* src, size_t count)
 {
@@ -1301,8 +1317,7 @@ static bool pattern_by_rows(Ctx* ctx, Matrix& M, Pattern& P, const std::vector<S
     rp.rowcA = rowinc.as<uint32_t>();
     rp.rowcD = rowcoo.as<uint32_t>();
     rp.counters = cnt + 3;
-    static std::once_flag attr;
-    std::call_once(attr, [] { cudaFuncSetAttribute(k_row_pattern, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024); });
+    raise_smem(ctx, k_row_pattern, 96 * 1024);
     // Counts of rows without kept rows beyond nA stay zero (the scans' last entry).
     cuda_check(cudaMemsetAsync(rowinc.as<void>(), 0, (nA + 1) * 4, ctx->x->stream), "memset");
     cuda_check(cudaMemsetAsync(rowcoo.as<void>(), 0, (nA + 1) * 4, ctx->x->stream), "memset");
@@ -1930,13 +1945,8 @@ static bool split_supported(const GroupDev& g)
 template <int B, int S, int L>
 static void launch_split(Ctx* ctx, const SplitParams& p)
 {
-    static bool attr = false;
     constexpr size_t smem = split_smem_bytes();
-    if (!attr) {
-        cuda_check(cudaFuncSetAttribute(k_contract_split<B, S, L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                   "smem attribute");
-        attr = true;
-    }
+    raise_smem(ctx, k_contract_split<B, S, L>, smem);
     const int64_t grid = std::min<int64_t>(p.nwork, std::max(ctx->nsm, 1));
     cuda_check(cudaMemsetAsync(p.next, 0, sizeof(unsigned long long), ctx->x->stream), "memset");
     k_contract_split<B, S, L><<<(unsigned)grid, kSplitThreads, smem, ctx->x->stream>>>(p);
@@ -2155,8 +2165,7 @@ constexpr size_t kSmallSmem = 200 * 1024;
 template <int PP>
 static void launch_small(Ctx* ctx, const GroupDev& g, const ContractParams& kp)
 {
-    static std::once_flag attr;
-    std::call_once(attr, [] { cudaFuncSetAttribute(k_contract_small<PP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallSmem); });
+    raise_smem(ctx, k_contract_small<PP>, kSmallSmem);
     const int P = g.ntf * g.ndof, parts = (P + PP - 1) / PP;
     const size_t smem = ((size_t)g.norient * g.nterms * g.ngp * parts * PP + (size_t)kSmallE * (P + 1)) * 8;
     // As many blocks as are resident at once, each taking equally many chunks.
@@ -2345,10 +2354,7 @@ static int mma_form(const MmaJob& j)
 template <int BP>
 static void launch_f64mma(Ctx* ctx, const MmaParams& mp, int64_t nblocks)
 {
-    static std::once_flag attr;
-    std::call_once(attr, [] {
-        cudaFuncSetAttribute(k_contract_f64mma<BP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MmaShape<BP>::Smem);
-    });
+    raise_smem(ctx, k_contract_f64mma<BP>, MmaShape<BP>::Smem);
     k_contract_f64mma<BP><<<(unsigned)nblocks, 256, MmaShape<BP>::Smem, ctx->x->stream>>>(mp);
     cuda_check(cudaGetLastError(), "k_contract_f64mma");
     ctx->launches++;
@@ -2958,23 +2964,17 @@ StreamLaunch stream_launch(Ctx* ctx, const RowParams& rp, const std::vector<RowS
     L.smem = (narrow ? row_stream_warp_bytes(StreamNarrow::R, StreamNarrow::VSH, StreamNarrow::SSH, sp.lpad)
                      : row_stream_warp_bytes(StreamWide::R, StreamWide::VSH, StreamWide::SSH, sp.lpad)) *
              kStreamWarps;
-    if (wmax > StreamWide::WMAX || L.smem > 227 * 1024)
+    if (wmax > StreamWide::WMAX || L.smem > kSmemMax)
         return L;
     L.kern = narrow ? k_row_stream<StreamNarrow> : k_row_stream<StreamWide>;
-    // Occupancy by ring depth and shared memory size; the kernels' shared
-    // memory limit only ever grows (launches on other streams may use a
-    // larger one).
+    if (L.smem > 48 * 1024)
+        raise_smem(ctx, L.kern, kSmemMax);
+    // Occupancy by ring depth and shared memory size.
     static std::mutex occ_mu;
     static std::map<std::pair<int, size_t>, int> blocks_per_sm;
-    static size_t attr_max = 48 * 1024;
     int nblk = 1;
     {
         std::lock_guard<std::mutex> lk(occ_mu);
-        if (L.smem > attr_max) {
-            for (auto k : {k_row_stream<StreamNarrow>, k_row_stream<StreamWide>})
-                cuda_check(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.smem), "smem attribute");
-            attr_max = L.smem;
-        }
         const auto key = std::make_pair(ring, L.smem);
         auto bi = blocks_per_sm.find(key);
         if (bi == blocks_per_sm.end()) {
@@ -3020,24 +3020,15 @@ void launch_warp_rows(Ctx* ctx, RowParams rp, bool f32)
     const size_t per_warp = (size_t)rp.lmax * 8;
     int wpb = (int)std::max<size_t>(1, std::min<size_t>(8, (48 * 1024) / per_warp));
     size_t smem = per_warp * wpb;
-    if (smem > 48 * 1024) {
-        if (smem > 227 * 1024)
-            fail(SLGPU_E_UNSUPPORTED, "a CSR row is too long for the shared-memory row buffer");
-        cuda_check(cudaFuncSetAttribute(k_row_values<double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem attribute");
-        cuda_check(cudaFuncSetAttribute(k_row_values<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem attribute");
-        cuda_check(cudaFuncSetAttribute(k_row_values<double, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem attribute");
-        cuda_check(cudaFuncSetAttribute(k_row_values<float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem attribute");
-    }
+    if (smem > kSmemMax)
+        fail(SLGPU_E_UNSUPPORTED, "a CSR row is too long for the shared-memory row buffer");
     const unsigned grid = grid_for((rp.nrows + rp.rows_per_warp - 1) / rp.rows_per_warp, wpb);
     const bool U = rp.uniform_width > 0;
-    if (f32 && U)
-        k_row_values<float, true><<<grid, 32 * wpb, smem, ctx->x->stream>>>(rp);
-    else if (f32)
-        k_row_values<float, false><<<grid, 32 * wpb, smem, ctx->x->stream>>>(rp);
-    else if (U)
-        k_row_values<double, true><<<grid, 32 * wpb, smem, ctx->x->stream>>>(rp);
-    else
-        k_row_values<double, false><<<grid, 32 * wpb, smem, ctx->x->stream>>>(rp);
+    void (*kern)(RowParams) = f32 ? (U ? k_row_values<float, true> : k_row_values<float, false>)
+                                  : (U ? k_row_values<double, true> : k_row_values<double, false>);
+    if (smem > 48 * 1024)
+        raise_smem(ctx, kern, kSmemMax);
+    kern<<<grid, 32 * wpb, smem, ctx->x->stream>>>(rp);
     cuda_check(cudaGetLastError(), "k_row_values");
     ctx->launches++;
 }

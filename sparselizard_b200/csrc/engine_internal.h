@@ -9,6 +9,7 @@
 #include <cstdint>
 #include <exception>
 #include <map>
+#include <set>
 #include <memory>
 #include <mutex>
 #include <string>
@@ -340,6 +341,7 @@ struct Ctx {
     // Rows per block of the FP64 contraction, picked by timing on first use
     // per group shape {ntf, ndof, ngp}.
     std::map<std::array<int, 3>, int> tile_choice;
+    std::set<const void*> smem_raised;  // kernels whose shared-memory limit this context has raised (raise_smem)
     std::map<int, MeshDev> meshes;
     std::map<int, std::unique_ptr<Matrix>> matrices;
     int next_handle = 1;

@@ -42,3 +42,43 @@ extern "C" unsigned int* flag(void* ctx) { return static_cast<slgpu::Ctx*>(ctx)-
         A, D = T._process(ctx, t, p)
         assert flag[0] == 0 and np.array_equal(A, ref[p][0]) and np.array_equal(D, ref[p][1])
     ctx.close()
+
+
+def test_shared_memory_limits_per_context(tmp_path):
+    """Two contexts in one process (on two devices, in a program with two):
+    each raises the dynamic shared-memory limit of every kernel that it
+    launches beyond the default, since the limit belongs to the device.  The
+    calls are counted by a library loaded before the CUDA runtime."""
+    shim = _compile(tmp_path, "count", """
+#include <dlfcn.h>
+#include <map>
+static std::map<const void*, int> calls;
+extern "C" int cudaFuncSetAttribute(const void* f, int attr, int value)
+{
+    static auto real = reinterpret_cast<int (*)(const void*, int, int)>(dlsym(dlopen("libcudart.so.12", RTLD_NOW), "cudaFuncSetAttribute"));
+    calls[f]++;
+    return real(f, attr, value);
+}
+extern "C" int functions() { return (int)calls.size(); }
+extern "C" int fewest() { int n = 1 << 30; for (auto& c : calls) n = c.second < n ? c.second : n; return n; }
+""")
+    code = """
+import ctypes
+import numpy as np
+from sparselizard_b200 import abi
+import test_gpu_graphs as T
+shim = ctypes.CDLL(None)
+seen = []
+for k in range(2):
+    ctx = abi.Context(0)
+    for ntf, ndof, ndofs in ((4, 4, 3000), (9, 9, 60), (8, 8, 9000), (40, 40, 7000)):  # many entries per row, and rows of many columns
+        t = T._setup(ctx, np.random.Generator(np.random.PCG64(53)), 0, 40, ntf, ndof, 2, 2, ndofs)
+        for p in (abi.PREC_FP64, abi.PREC_SPLIT, abi.PREC_FP32):
+            T._process(ctx, t, p)
+    ctx.close()
+    seen.append(shim.functions())
+assert seen[0] >= 5 and seen[0] == seen[1], seen
+assert shim.fewest() >= 2, "a kernel's limit was not raised again in the second context"
+"""
+    env = dict(os.environ, LD_PRELOAD=shim, PYTHONPATH=os.pathsep.join([HERE, ROOT]))
+    subprocess.run([sys.executable, "-c", code], env=env, check=True, timeout=300)
