@@ -48,7 +48,9 @@ enum {
 enum {
     SLGPU_PREC_FP64 = 0,  /* plain FP64 */
     SLGPU_PREC_SPLIT = 1, /* FP64 operands split into 6 INT8 slices on the tensor cores (tcgen05 kind::i8), exact INT32
-                             accumulation, FP64 recombination; <= 1e-10 relative per element matrix */
+                             accumulation, FP64 recombination; <= 1e-10 relative per element matrix.  Operands are
+                             rounded to 48 bits below the largest of their row or column; where all of those have
+                             at most 21 significant bits (whole numbers, dyadic fractions) they are held exactly */
     SLGPU_PREC_FP32 = 2   /* same with 5 slices: FP32-level tier, <= 1e-6 */
 };
 

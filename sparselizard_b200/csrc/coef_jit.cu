@@ -330,13 +330,25 @@ std::string jit_slice_source(const std::vector<const GroupDev*>& batch, int tier
                 s << "  for (int n = threadIdx.x; n < " << Q16 - Q << " * E; n += blockDim.x) st[" << (k - r0) * place << " + " << Q + Q / 16
                   << " * E + n] = 0;\n";
         }
-        s << "  __syncthreads();\n  for (int n = " << r0 << " * E + threadIdx.x; n < " << r1 << " * E; n += blockDim.x)\n"
-          << "    if (grp.g[n / E].slices != nullptr) {\n      double unit;\n      fac[n] = slgpu::split_scale<" << B << ", " << S
-          << ">(top[n], &unit, &pre[n]);\n      grp.g[n / E].colscale[tile * 64 + base + n % E] = unit;\n    }\n  __syncthreads();\n";
-        // Chunks of 16 values of the round's groups, the groups' chunks side by
-        // side where they have equally many.
         bool same = true;
         for (size_t k = r0; k < r1; k++) same = same && batch[k]->nterms == batch[r0]->nterms;
+        // Scales.  The values of a column are looked at until the first that a
+        // scale by powers of two would not hold exactly, as a rule its first.
+        s << "  __syncthreads();\n  for (int n = " << r0 << " * E + threadIdx.x; n < " << r1 << " * E; n += blockDim.x)\n"
+          << "    if (grp.g[n / E].slices != nullptr) {\n";
+        if (B == 8) {
+            s << "      const int Q = ";
+            for (size_t k = r0; !same && k + 1 < r1; k++) s << "n < " << k + 1 << " * E ? " << batch[k]->nterms * ngp << " : ";
+            s << batch[r1 - 1]->nterms * ngp << ";\n      const double* v = st + (n / E - " << r0 << ") * " << place << " + n % E;\n"
+              << "      bool exact = top[n] > 0;\n"
+              << "      for (int q = 0; exact && q < Q; q++) exact = slgpu::split_exact(v[(q + (q >> 4)) * E], top[n]);\n";
+        } else {
+            s << "      const bool exact = false;\n";
+        }
+        s << "      double unit;\n      fac[n] = slgpu::split_scale<" << B << ", " << S
+          << ">(top[n], exact, &unit, &pre[n]);\n      grp.g[n / E].colscale[tile * 64 + base + n % E] = unit;\n    }\n  __syncthreads();\n";
+        // Chunks of 16 values of the round's groups, the groups' chunks side by
+        // side where they have equally many.
         auto chunks = [&](size_t a, size_t b) {
             const int Q = batch[a]->nterms * ngp, nc = (Q + 15) / 16, nchunk = (Q + 31) / 32 * 2;
             s << "  for (int n = threadIdx.x; n < " << (b - a) * (size_t)nc << " * E; n += blockDim.x) {\n";

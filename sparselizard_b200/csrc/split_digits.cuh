@@ -13,12 +13,19 @@ namespace slgpu {
 // magnitude in it: *q, the value that 2^(B S) units stand for (R and Q of
 // split_tc.cuh), and the factor that turns a value into those units.
 //   B = 8: |x| < the double of high word h + 1, so |x| / Q < 0.498 and its S
-//   balanced digits represent it (the largest such number is 0.49804);
+//   balanced digits represent it (the largest such number is 0.49804); or,
+//   where the digits then hold every value exactly (`exact`), four times the
+//   power of two above |x|: whole numbers and dyadic fractions stay what they
+//   are, and so do their sums of products;
 //   B = 7: the power of two above |x|.
 // Magnitudes below 2^-900 take a power of two and a factor below the
 // overflow: *pre, by which values are multiplied first (1 otherwise).
 // Nothing set (h = 0): digits and scale are zero.  Infinities and NaN (h from
 // 0x7ff00000): the scale is NaN, so that the results are.
+//
+// split_exact: whether B = 8 and the scale by powers of two hold x exactly, h
+// as above: at most 21 significant bits (the low word is zero), the last of
+// them not below the unit 2^(46 - B S) of the power of two above h.
 //
 // split_digits: the S digits of x in units of 1 / f, byte k the digit
 // S - 1 - k.
@@ -31,7 +38,12 @@ namespace slgpu {
 // split_words: word k4 of each slice, digit s of four values.
 SLGPU_DEVICE_SOURCE(
     kSplitDigitSource,
-    template <int B, int S> __device__ __forceinline__ double split_scale(int h, double* q, double* pre) {
+    __device__ __forceinline__ bool split_exact(double x, int h) {
+        const int hx = __double2hiint(x) & 0x7fffffff;
+        return __double2loint(x) == 0 && (hx == 0 || (h >> 20) - (hx >> 20) <= 25);
+    }
+
+    template <int B, int S> __device__ __forceinline__ double split_scale(int h, bool exact, double* q, double* pre) {
         const double unit = __longlong_as_double((long long)(1023 + B * S) << 52);
         *pre = 1.0;
         if (h <= 0) {
@@ -43,7 +55,7 @@ SLGPU_DEVICE_SOURCE(
             return 0.0;
         }
         const bool tiny = h < ((1023 - 900) << 20);
-        if (tiny || B == 7) {
+        if (tiny || exact || B == 7) {
             int ex;
             frexp(__hiloint2double(h, -1), &ex);
             ex += B == 7 ? 0 : 2;

@@ -147,17 +147,25 @@ __global__ void k_slice_rows(RowSliceParams p)
 {
     const int pe = blockIdx.x, o = blockIdx.y;
     const int src = pe >= p.nrows ? -1 : p.rowentry != nullptr ? p.rowentry[pe] : pe;
-    __shared__ int top;
-    if (threadIdx.x == 0)
+    __shared__ int top, rounded;
+    if (threadIdx.x == 0) {
         top = 0;
+        rounded = 0;
+    }
     __syncthreads();
     // Magnitudes compare as their bit patterns (NaN above infinity).
     int mx = 0;
     for (int q = threadIdx.x; q < p.Qpad; q += blockDim.x) mx = max(mx, __double2hiint(m_entry(p, o, src, q)) & 0x7fffffff);
     atomicMax(&top, mx);
     __syncthreads();
+    for (int q = threadIdx.x; B == 8 && q < p.Qpad; q += blockDim.x)
+        if (!split_exact(m_entry(p, o, src, q), top)) {
+            rounded = 1;
+            break;
+        }
+    __syncthreads();
     double unit, pre;
-    const double f = split_scale<B, S>(top, &unit, &pre);
+    const double f = split_scale<B, S>(top, B == 8 && rounded == 0, &unit, &pre);
     if (threadIdx.x == 0)
         p.rowscale[(int64_t)o * p.Ppad + pe] = ldexp(unit, -B * p.L);
     const int ntp = p.Ppad / kSplitM, nk = p.Qpad / kSplitKStep;
@@ -209,12 +217,15 @@ __global__ void k_slice_cols(const __grid_constant__ ColSliceParams pb)
     const Tile tile = p.tiles[t];
     const bool valid = slot < tile.ne;
     const int64_t e = tile.e0 + slot;
+    const double* col = p.C + e;
+    const int top = valid ? p.elemtop[e] : 0;
+    bool exact = B == 8 && top > 0;
+    for (int64_t q = 0; exact && q < (int64_t)p.nterms * p.ngp; q++) exact = split_exact(col[q * p.nelem], top);
     double unit, pre;
-    const double f = split_scale<B, S>(valid ? p.elemtop[e] : 0, &unit, &pre);
+    const double f = split_scale<B, S>(top, exact, &unit, &pre);
     p.colscale[t * 64 + slot] = unit;
     const int nchunk = p.Qpad / 16;
     uint4* out = reinterpret_cast<uint4*>(p.slices) + t * (int64_t)nchunk * S * kSplitNE + slot;
-    const double* col = p.C + e;
     for (int c = 0; c < nchunk; c++) {
         double x[16];
 #pragma unroll
