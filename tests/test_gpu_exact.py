@@ -1,4 +1,4 @@
-"""Split precision on operands of few significant bits."""
+"""Split precision on operands of few significant bits and on quotients that are exact."""
 import os
 import subprocess
 import sys
@@ -69,3 +69,13 @@ def test_whole_numbers_are_exact(interpreter):
     straight to slices or through memory."""
     env = dict(os.environ, SLGPU_COEF_INTERPRETER=interpreter, PYTHONPATH=os.pathsep.join([HERE, os.path.dirname(HERE)]))
     subprocess.run([sys.executable, "-c", "import test_gpu_exact as T; T.check_whole_all()"], env=env, check=True, timeout=300)
+
+
+@pytest.mark.parametrize("size", [(2.0, 98.0), (2.0, 206.0)])
+def test_inverse_jacobian_is_divided(size):
+    """Cofactors are divided by the determinant: 49 / 49 and 103 / 103 are 1
+    (times the rounded reciprocal, they are not), so the element matrices are
+    whole numbers, exact in each tier."""
+    ctx = abi.Context(0)
+    check_whole(ctx, seed=80, ntf=9, ndof=9, nterms=2, norient=1, grid=9, coef=6, size=size)
+    ctx.close()
