@@ -10,8 +10,9 @@ namespace slgpu {
     static const char* const name = SLGPU_TEXT(__VA_ARGS__);
 
 // split_scale: scale of a row or column from the high word h of the largest
-// magnitude in it: *q, the value that 2^(B S) units stand for (R and Q of
-// split_tc.cuh), and the factor that turns a value into those units.
+// magnitude in it: *q, 2^-8 of the value Q that 2^(B S) units stand for (R and
+// Q of split_tc.cuh; Q itself can be above the largest double), and the factor
+// that turns a value into those units.
 //   B = 8: |x| < the double of high word h + 1, so |x| / Q < 0.498 and its S
 //   balanced digits represent it (the largest such number is 0.49804); or,
 //   where the digits then hold every value exactly (`exact`), four times the
@@ -19,9 +20,10 @@ namespace slgpu {
 //   are, and so do their sums of products;
 //   B = 7: the power of two above |x|.
 // Magnitudes below 2^-900 take a power of two and a factor below the
-// overflow: *pre, by which values are multiplied first (1 otherwise).
-// Nothing set (h = 0): digits and scale are zero.  Infinities and NaN (h from
-// 0x7ff00000): the scale is NaN, so that the results are.
+// overflow: *pre, by which values are multiplied first (1 otherwise).  High
+// words 0 and 1 share a scale, so that the smallest doubles have digits.
+// Infinities and NaN (h from 0x7ff00000): the scale is NaN, so that the results
+// are.
 //
 // split_exact: whether B = 8 and the scale by powers of two hold x exactly, h
 // as above: at most 21 significant bits (the low word is zero), the last of
@@ -46,10 +48,7 @@ SLGPU_DEVICE_SOURCE(
     template <int B, int S> __device__ __forceinline__ double split_scale(int h, bool exact, double* q, double* pre) {
         const double unit = __longlong_as_double((long long)(1023 + B * S) << 52);
         *pre = 1.0;
-        if (h <= 0) {
-            *q = 0.0;
-            return 0.0;
-        }
+        h = max(h, 1);
         if (h >= 0x7ff00000) {
             *q = __longlong_as_double(0x7ff8000000000000ll);
             return 0.0;
@@ -59,12 +58,12 @@ SLGPU_DEVICE_SOURCE(
             int ex;
             frexp(__hiloint2double(h, -1), &ex);
             ex += B == 7 ? 0 : 2;
-            *q = ldexp(1.0, ex);
+            *q = ldexp(1.0, ex - 8);
             *pre = tiny ? 0x1p512 : 1.0;
             return ldexp(unit, -ex - (tiny ? 512 : 0));
         }
         const double top = h >= 0x7fefffff ? __longlong_as_double(0x7fefffffffffffffll) : __hiloint2double(h + 1, 0);
-        *q = top * (1.0 / 0.498);
+        *q = top * (0x1p-8 / 0.498);
         return 0.498 * unit / top;
     }
 

@@ -78,8 +78,8 @@ struct SplitGroup {
     const Tile* tiles;      // [nwork / ntp]
     const int8_t* A;        // row slices
     const int8_t* B;        // column slices
-    const double* rowscale;  // [norient][Ppad]: R_p 2^-(B L)
-    const double* colscale;  // [ntiles][64]: Q_e of each slot
+    const double* rowscale;  // [norient][Ppad]: R_p 2^(8 - B L)
+    const double* colscale;  // [ntiles][64]: Q_e 2^-8 of each slot
     double* out;            // [nelem][es]
     int64_t w0, nwork;
 };
@@ -167,7 +167,7 @@ __global__ void k_slice_rows(RowSliceParams p)
     double unit, pre;
     const double f = split_scale<B, S>(top, B == 8 && rounded == 0, &unit, &pre);
     if (threadIdx.x == 0)
-        p.rowscale[(int64_t)o * p.Ppad + pe] = ldexp(unit, -B * p.L);
+        p.rowscale[(int64_t)o * p.Ppad + pe] = ldexp(unit, 16 - B * p.L);
     const int ntp = p.Ppad / kSplitM, nk = p.Qpad / kSplitKStep;
     const int pt = pe / kSplitM, r = pe % kSplitM;
     for (int q = threadIdx.x; q < p.Qpad; q += blockDim.x) {
@@ -187,7 +187,7 @@ __global__ void k_slice_rows(RowSliceParams p)
 // (jit_slice_source) cannot evaluate.
 struct ColSliceGroup {
     const double* C;  // [Q][nelem]
-    const int32_t* elemtop;  // [nelem]; 0: the column is zero
+    const int32_t* elemtop;  // [nelem]; 0: no magnitude from 2^-1042 on
     const Tile* tiles;
     int nterms, ngp, Qpad;
     int64_t nelem, ntiles;
@@ -631,7 +631,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_contract_split(const __gri
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t col = lane_base + (uint32_t)c0;
-            // V = R_p Q_e 2^-(B L) T.
+            // V = R_p 2^(8 - B L) T Q_e 2^-8.
             double d[16];
 #pragma unroll
             for (int h = 0; h < 16; h += 8) {

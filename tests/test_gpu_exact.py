@@ -1,4 +1,4 @@
-"""Split precision on operands of few significant bits and on quotients that are exact."""
+"""Split precision on operands of few significant bits, on quotients that are exact, and at the ends of the range."""
 import os
 import subprocess
 import sys
@@ -78,4 +78,27 @@ def test_inverse_jacobian_is_divided(size):
     whole numbers, exact in each tier."""
     ctx = abi.Context(0)
     check_whole(ctx, seed=80, ntf=9, ndof=9, nterms=2, norient=1, grid=9, coef=6, size=size)
+    ctx.close()
+
+
+@pytest.mark.parametrize("largest,table", [(1.79e308, 1e-10), (1e308, 1e-10), (3e-315, 1.0)])
+def test_ends_of_the_range(largest, table):
+    """Coefficients up to the largest double, and ones of which none is a
+    normal double: within 1e-10 of FP64's element matrices; a zero column
+    stays zero."""
+    ctx = abi.Context(0)
+    gb, xyz, conn, _ = whole_numbers(seed=90, ntf=9, ndof=9, nterms=1, norient=1, grid=13, coef=5)
+    g = gb.g
+    g.terms[0].scale = 1.0
+    np.ctypeslib.as_array(g.weights, (4,))[:] = [4.0, 2.0, 1.0, 0.5]  # times the determinant 1/4
+    np.ctypeslib.as_array(g.tables[0].vals, (1, 9, 4))[:] *= table
+    e = np.ctypeslib.as_array(g.elemdata[0], (g.nelem,))
+    e[:] = largest * np.random.Generator(np.random.PCG64(91)).uniform(0.3, 1.0, g.nelem)
+    e[0], e[5] = largest, 0.0
+    ref = _element_matrices(ctx, gb, xyz, conn, abi.PREC_FP64)
+    got = _element_matrices(ctx, gb, xyz, conn, abi.PREC_SPLIT)
+    assert np.isfinite(ref).all() and np.isfinite(got).all() and not got[5].any()
+    size = np.abs(ref).max(axis=1)
+    assert (size > 0).sum() == g.nelem - 1
+    assert (np.abs(got - ref).max(axis=1) <= 1e-10 * size).all()
     ctx.close()
