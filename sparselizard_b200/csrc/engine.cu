@@ -1853,6 +1853,12 @@ static ComputedRows entry_rows(const GroupDev& g, int form, bool whole)
     return rows;
 }
 
+static int split_slices(int tier) { return tier == 0 ? 6 : 5; }
+static int split_qpad(const GroupDev& g)
+{
+    return std::max(kSplitKStep, (g.nterms * g.ngp + kSplitKStep - 1) / kSplitKStep * kSplitKStep);
+}
+
 // Row slices of a group for a tier (0 split, 1 FP32 level) and form (0 every
 // entry, 1 upper triangle of a symmetric group, 2 every entry with its
 // transposed partner's): slot tier + 2 form.
@@ -1863,10 +1869,9 @@ static GroupDev::Split& build_split(Ctx* ctx, GroupDev& g, int slot)
         return *sp;
     const int tier = slot & 1, form = slot >> 1;
     sp.reset(new GroupDev::Split());
-    sp->S = tier == 0 ? 6 : 5;
+    sp->S = split_slices(tier);
     sp->L = tier == 0 ? 7 : 6;
-    const int Q = g.nterms * g.ngp;
-    sp->Qpad = std::max(kSplitKStep, (Q + kSplitKStep - 1) / kSplitKStep * kSplitKStep);
+    sp->Qpad = split_qpad(g);
     const ComputedRows rows = entry_rows(g, form, tier == 0);
     sp->nrows = (int)rows.entry.size();
     sp->Ppad = (sp->nrows + kSplitM - 1) / kSplitM * kSplitM;
@@ -1970,9 +1975,9 @@ struct SplitJob {
 };
 
 // Column-slice bytes of one group in the scratch (256-byte aligned blocks).
-static size_t split_col_bytes(const GroupDev& g, const GroupDev::Split& sp)
+static size_t split_col_bytes(const GroupDev& g, int tier)
 {
-    return ((size_t)sp.S * sp.Qpad * g.tiles.size() * 64 + 255) & ~size_t(255);
+    return ((size_t)split_slices(tier) * split_qpad(g) * g.tiles.size() * 64 + 255) & ~size_t(255);
 }
 static size_t split_scale_bytes(const GroupDev& g) { return (g.tiles.size() * 64 * 8 + 255) & ~size_t(255); }
 
@@ -1984,8 +1989,8 @@ static void place_split_jobs(Ctx* ctx, std::vector<SplitJob>& jobs)
 {
     size_t colb = 0, scaleb = 0;
     for (const SplitJob& j : jobs) {
-        const GroupDev::Split& sp = ensure_split(ctx, *j.g, j.tier, j.paired);
-        colb += split_col_bytes(*j.g, sp);
+        ensure_split(ctx, *j.g, j.tier, j.paired);
+        colb += split_col_bytes(*j.g, j.tier);
         scaleb += split_scale_bytes(*j.g);
     }
     {
@@ -2000,7 +2005,7 @@ static void place_split_jobs(Ctx* ctx, std::vector<SplitJob>& jobs)
     for (SplitJob& j : jobs) {
         j.slices = cols;
         j.colscale = reinterpret_cast<double*>(scales);
-        cols += split_col_bytes(*j.g, *j.g->split[job_slot(j)]);
+        cols += split_col_bytes(*j.g, j.tier);
         scales += split_scale_bytes(*j.g);
     }
 }
@@ -2033,7 +2038,7 @@ static void slice_split_jobs(Ctx* ctx, const std::vector<SplitJob>& jobs)
             c.colscale = j.colscale;
             c.t0 = cs.ntiles;
             cs.ntiles += c.ntiles;
-            bytes += 8.0 * g.nterms * g.ngp * g.nelem + 4.0 * g.nelem + (double)split_col_bytes(g, s) + 8.0 * c.ntiles * 64;
+            bytes += 8.0 * g.nterms * g.ngp * g.nelem + 4.0 * g.nelem + (double)split_col_bytes(g, j.tier) + 8.0 * c.ntiles * 64;
         }
         if (cs.ngroups == 0)
             break;
@@ -2583,14 +2588,25 @@ static bool slice_fits(const GroupDev& g)
     return sh.smem <= kSliceSmemMax && (size_t)sh.E * (24 * (size_t)g.ncn + 20 * kSliceBatch) <= 30 * 1024;
 }
 
-// `skip`: groups without coefficients of their own (the second of a
-// transposed pair); they stay in their batch, whose kernel then serves both.
-static CoefPlan coef_plan(Ctx* ctx, const Matrix& M, int precision, const std::vector<char>& skip)
+// Whether a group's coefficients can be evaluated by runtime-compiled kernels,
+// and whether they then go straight to slices.
+static bool coef_compiled(const Ctx* ctx, const GroupDev& g)
 {
     static const bool interp_only = [] {
         const char* v = std::getenv("SLGPU_COEF_INTERPRETER");
         return v != nullptr && std::strcmp(v, "1") == 0;
     }();
+    return !interp_only && !ctx->jit_broken && g.elemdim == g.problemdim;
+}
+static bool coef_sliced(const Ctx* ctx, const GroupDev& g, int precision)
+{
+    return coef_compiled(ctx, g) && uses_split(g, precision) && slice_fits(g);
+}
+
+// `skip`: groups without coefficients of their own (the second of a
+// transposed pair); they stay in their batch, whose kernel then serves both.
+static CoefPlan coef_plan(Ctx* ctx, const Matrix& M, int precision, const std::vector<char>& skip)
+{
     const size_t ng = M.groups.size();
     const int tier = precision == SLGPU_PREC_FP32 ? 1 : 0;
     CoefPlan P;
@@ -2603,7 +2619,7 @@ static CoefPlan coef_plan(Ctx* ctx, const Matrix& M, int precision, const std::v
             continue;
         const size_t ns = P.slices.size(), nc = P.coefs.size();
         bool done = false;
-        if (!interp_only && !ctx->jit_broken && g0.elemdim == g0.problemdim) {
+        if (coef_compiled(ctx, g0)) {
             try {
                 std::vector<char> taken(k1 - k, 0);
                 for (size_t a = k; a < k1;) {
@@ -2612,7 +2628,7 @@ static CoefPlan coef_plan(Ctx* ctx, const Matrix& M, int precision, const std::v
                     bool wanted = false;
                     for (; a < k1 && list.size() < kSliceBatch; a++) {
                         const GroupDev& ga = *M.groups[a];
-                        if (!uses_split(ga, precision) || !slice_fits(ga))
+                        if (!coef_sliced(ctx, ga, precision))
                             continue;
                         taken[a - k] = 1;
                         b.groups.push_back(a);
@@ -2689,7 +2705,7 @@ static void launch_coefficients(Ctx* ctx, const Matrix& M, const CoefPlan& plan,
                 continue;
             }
             js.push_back(JitSlice{M.groups[j]->tables.as<double>(), elemdata(j), fielddata(j), scales(j), sj->slices, sj->colscale});
-            bytes += (double)split_col_bytes(*sj->g, *sj->g->split[job_slot(*sj)]) + 8.0 * sj->g->tiles.size() * 64;
+            bytes += (double)split_col_bytes(*sj->g, sj->tier) + 8.0 * sj->g->tiles.size() * 64;
         }
         void* args[] = {&geom, js.data(), &tiles};  // the group array is one by-value parameter
         const int kt = kstat_start(ctx, "slice_cols", bytes);
@@ -3147,11 +3163,11 @@ void prepare_value_path(Ctx* ctx, const Matrix& M, int precision)
     for (size_t gi = 0; gi < M.groups.size(); gi++) {
         GroupDev* g = M.groups[gi].get();
         if (g->nelem > 0 && uses_split(*g, precision)) {
-            const GroupDev::Split& sp = ensure_split(ctx, *g, tier, false);
+            ensure_split(ctx, *g, tier, false);
             if (pair[gi] > (int)gi)
                 ensure_split(ctx, *g, tier, true);
             // The groups of a step are sliced and contracted together.
-            colbytes += split_col_bytes(*g, sp);
+            colbytes += split_col_bytes(*g, tier);
             expbytes += split_scale_bytes(*g);
         }
     }
@@ -3161,6 +3177,23 @@ void prepare_value_path(Ctx* ctx, const Matrix& M, int precision)
     if (x.split_colscale.bytes() < expbytes)
         x.split_colscale.alloc(ctx, expbytes);
     ensure_split_state(ctx);
+}
+
+ValuePathBytes value_path_bytes(const Ctx* ctx, const Matrix& M, int precision)
+{
+    ValuePathBytes b;
+    std::vector<int64_t> gvb;
+    build_segments(M, &gvb, &b.step, float_values(M, precision));
+    b.step *= 8;
+    for (auto& g : M.groups) {
+        if (uses_split(*g, precision)) {
+            b.slices += (int64_t)split_col_bytes(*g, precision == SLGPU_PREC_SPLIT ? 0 : 1);
+            b.scales += (int64_t)split_scale_bytes(*g);
+        }
+        if (!coef_sliced(ctx, *g, precision))
+            b.step += (8 * (int64_t)g->nterms * g->ngp + 4) * g->nelem;
+    }
+    return b;
 }
 
 void compile_value_path(Ctx* ctx, const Matrix& M, int precision)

@@ -437,6 +437,13 @@ void htrace_mark(Ctx* ctx, const char* label);
 // current execution state's split scratch grown to fit them, so that the
 // value path allocates nothing for them.
 void prepare_value_path(Ctx* ctx, const Matrix& M, int precision);
+// Device bytes of a step with this precision: allocated for the step (element
+// values; coefficients that go through memory), and kept by the execution
+// state (column slices and scales).
+struct ValuePathBytes {
+    int64_t step = 0, slices = 0, scales = 0;
+};
+ValuePathBytes value_path_bytes(const Ctx* ctx, const Matrix& M, int precision);
 // The flag and counter of split contractions on the current execution state;
 // the flag cleared, before a call queues any; whether a wait of the call timed
 // out (the stream has been synchronised).

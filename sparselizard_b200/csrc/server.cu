@@ -71,7 +71,7 @@ struct Request {
     bool pinned_out = false;
     // Template state kept alive while the request runs.
     std::shared_ptr<Matrix> tmpl;
-    int64_t est_bytes = 0;
+    ValuePathBytes est;
     // Device and host resources while running.
     DevBuf vals, Avals, Dvals, upd;
     std::vector<DevBuf> ed, fd;
@@ -114,21 +114,12 @@ struct Server {
 
 namespace {
 
-// Device bytes a request allocates while it runs (r == nullptr: a request
-// that updates every per-element array of every group).
-int64_t estimate_bytes(const Matrix& M, int precision, const Request* r)
+// Device bytes a request takes: for its arena, and in the slot's column slices
+// and scales (r == nullptr: a request that updates every per-element array of
+// every group).
+ValuePathBytes estimate_bytes(const Ctx* ctx, const Matrix& M, int precision, const Request* r)
 {
-    int64_t vals = 0, coef = 0, exps = 0, split = 0;
-    for (auto& g : M.groups) {
-        vals += (int64_t)g->ntf * g->ld * g->nelem;
-        coef += (int64_t)g->nterms * g->ngp * g->nelem;
-        exps += g->nelem;
-        // The split groups of a request are sliced and contracted together:
-        // their column slices coexist.
-        const int64_t Qpad = ((int64_t)g->nterms * g->ngp + 31) / 32 * 32;
-        split += 7 * Qpad * (int64_t)g->tiles.size() * 64 + (int64_t)g->tiles.size() * 256 + 512;
-    }
-    for (auto& f : M.frags) vals += (int64_t)f->nr * f->nc;
+    ValuePathBytes b = value_path_bytes(ctx, M, precision);
     int64_t upd = 0, over = 0;
     if (r != nullptr) {
         upd = r->nin;
@@ -141,10 +132,8 @@ int64_t estimate_bytes(const Matrix& M, int precision, const Request* r)
         upd = over;
     }
     const int64_t csr = M.pattern ? M.pattern->nnzA + M.pattern->nnzD : 0;
-    int64_t b = 8 * (vals + coef + csr + upd + over) + 4 * exps;
-    if (precision != SLGPU_PREC_FP64)
-        b += split;
-    return b + (int64_t(1) << 20);
+    b.step += 8 * (csr + upd + over) + (int64_t(1) << 20);
+    return b;
 }
 
 void ensure_pinned(Slot& s, size_t bytes)
@@ -174,7 +163,7 @@ void launch(Server& S, Slot& s, Request& r)
     // Request buffers come from the slot's arena, grown (rarely, on this
     // slot's stream) to the largest request seen.
     {
-        const size_t want = std::max<size_t>(s.arena_need, (size_t)r.est_bytes);
+        const size_t want = std::max<size_t>(s.arena_need, (size_t)r.est.step);
         if (s.ex.arena.bytes() < want)
             s.ex.arena.alloc(ctx, want + want / 8);
         s.ex.arena_off = 0;
@@ -368,8 +357,12 @@ void server_loop(Server& S)
                 r = S.queue.front();
             }
             std::lock_guard<std::recursive_mutex> cl(ctx->mu);
-            // Device memory the request adds: what its slot's arena lacks.
-            const int64_t extra = std::max<int64_t>(0, r->est_bytes - (int64_t)free_slot->ex.arena.bytes());
+            // Device memory the request adds: what its slot's arena, slices and
+            // scales lack.
+            const Exec& fx = free_slot->ex;
+            const int64_t extra = std::max<int64_t>(0, r->est.step - (int64_t)fx.arena.bytes()) +
+                                  std::max<int64_t>(0, r->est.slices - (int64_t)fx.split_cols.bytes()) +
+                                  std::max<int64_t>(0, r->est.scales - (int64_t)fx.split_colscale.bytes());
             if (ctx->in_use + extra > (int64_t)ctx->budget) {
                 bool busy = false;
                 for (Slot& s : S.slots) busy = busy || (bool)s.req;
@@ -597,8 +590,8 @@ int slgpu_server_submit(slgpu_server* S, const slgpu_request* rq, int64_t* ticke
                         (cudaPointerGetAttributes(&pd, rq->Dvals) == cudaSuccess && pd.type == cudaMemoryTypeHost);
         cudaGetLastError();
         r->pinned_out = pA && pD;
-        r->est_bytes = estimate_bytes(M, rq->precision, r.get());
-        if (r->est_bytes > (int64_t)ctx->budget) {
+        r->est = estimate_bytes(ctx, M, rq->precision, r.get());
+        if (r->est.step + r->est.slices + r->est.scales > (int64_t)ctx->budget) {
             ctx->last_error = "a request needs more device memory than the whole HBM budget";
             return SLGPU_E_BUDGET;
         }
@@ -689,8 +682,8 @@ int slgpu_server_submit_template(slgpu_server* S, int handle, const uint8_t* isc
             ncoo += (int64_t)f->nr * f->nc;
             nvals += (int64_t)f->nr * f->nc;
         }
-        r->est_bytes = 40 * ncoo + 24 * nvals + 16 * M.ndofs + (int64_t(1) << 20);
-        if (r->est_bytes > (int64_t)ctx->budget) {
+        r->est.step = 40 * ncoo + 24 * nvals + 16 * M.ndofs + (int64_t(1) << 20);
+        if (r->est.step > (int64_t)ctx->budget) {
             ctx->last_error = "the template's first assembly needs more device memory than the whole HBM budget";
             return SLGPU_E_BUDGET;
         }
@@ -794,7 +787,7 @@ int slgpu_server_prepare(slgpu_server* S, int handle, int precision)
     const Matrix& M = *it->second;
     try {
         cudaSetDevice(ctx->device);
-        const size_t est = (size_t)estimate_bytes(M, precision, nullptr);
+        const size_t est = (size_t)estimate_bytes(ctx, M, precision, nullptr).step;
         for (Slot& s : S->slots) {
             ctx->x = &s.ex;
             compile_value_path(ctx, M, precision);

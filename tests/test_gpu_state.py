@@ -82,3 +82,32 @@ assert shim.fewest() >= 2, "a kernel's limit was not raised again in the second 
 """
     env = dict(os.environ, LD_PRELOAD=shim, PYTHONPATH=os.pathsep.join([HERE, ROOT]))
     subprocess.run([sys.executable, "-c", code], env=env, check=True, timeout=300)
+
+
+def test_server_arena_holds_what_requests_use():
+    """What preparing a template reserves for split-precision requests: the
+    element matrices, the values and the replaced data (an eighth more, for
+    the arena grows so), and the slices and their scales; not the
+    coefficients, which are never in memory.  A request then adds nothing."""
+    import test_gpu_serving as V
+    from sparselizard_b200 import serving
+
+    ctx = abi.Context(0)
+    rng = np.random.Generator(np.random.PCG64(54))
+    t = V._template(ctx, rng, 1, 150, 9, 9, 9, 4, 2500)
+    g, n = t["gb"].g, t["nmesh"]
+    srv = serving.Server(ctx.lib, ctx.h, 1)
+    b0 = ctx.lib.slgpu_bytes_in_use(ctx.h)
+    srv.prepare(t["handle"], abi.PREC_SPLIT)
+    b1 = ctx.lib.slgpu_bytes_in_use(ctx.h)
+    tiles = n // 64 + 2  # of each of two orientations
+    slices = 6 * (9 * 16 + 16) // 32 * 32 * tiles * 64 + 8 * 64 * tiles
+    rows = 2 * 7 * 128 * 160 + (1 << 20)  # row slices and small tables
+    arena = 8 * (81 * n + t["nnzA"] + t["nnzD"] + 2 * n) + (1 << 20)
+    assert b1 - b0 <= 9 * arena // 8 + slices + rows, f"{b1 - b0} bytes reserved"
+    A, D = np.zeros(t["nnzA"]), np.zeros(t["nnzD"])
+    up = serving.UpdateSpec(0, abi.UPDATE_ELEMDATA, 0, rng.lognormal(0.0, 0.4, n))
+    assert srv.wait(srv.submit(t["handle"], abi.PREC_SPLIT, [up], A, D)).status == abi.OK
+    assert ctx.lib.slgpu_bytes_in_use(ctx.h) <= b1
+    srv.close()
+    ctx.close()
