@@ -291,6 +291,11 @@ std::string jit_slice_source(const std::vector<const GroupDev*>& batch, int tier
           << (fast ? "" : " * pr") << ", f);\n    slgpu::split_words<" << B << ", " << S << ">(u, wd, k4);\n  }\n";
         s << "  #pragma unroll\n  for (int i = 0; i < " << S << "; i++) out[i * 64] = make_uint4(wd[i][0], wd[i][1], wd[i][2], wd[i][3]);\n}\n";
     }
+    // Loops over the block's work, which take a few turns each, stay loops:
+    // unrolled, nine groups of elasticity took 1.0 to 1.1 s to compile instead of
+    // 0.5 to 0.65, and the calls in them cost registers (48^3 hexahedra 0.66
+    // instead of 0.49 ms, FP32 tetrahedra 101 instead of 87 us).
+    const char* const kLoop = "#pragma unroll 1\n";
     s << "extern \"C\" __global__ void __launch_bounds__(" << sh.threads << ") slgpu_slices(JitGeom p, const JitSlices grp, const int4* tiles)\n{\n";
     s << "  constexpr int E = " << sh.E << ", NG = " << ng << ";\n";
     s << "  __shared__ double xs[" << 3 * ncn << " * E], fac[NG * E], pre[NG * E];\n  __shared__ int top[NG * E];\n";
@@ -298,10 +303,10 @@ std::string jit_slice_source(const std::vector<const GroupDev*>& batch, int tier
     s << "  const int base = (int)(blockIdx.x % (64 / E)) * E;\n  if (base >= tl.y) return;\n";
     s << "  const int o = tl.z;\n  (void)o;\n";
     // Slots past the end of a short tile repeat its last element.
-    s << "  for (int n = threadIdx.x; n < " << ncn << " * E; n += blockDim.x) { const int el = n % E, k = n / E;\n"
+    s << kLoop << "  for (int n = threadIdx.x; n < " << ncn << " * E; n += blockDim.x) { const int el = n % E, k = n / E;\n"
       << "    const i64 e = tl.x + (base + el < tl.y ? base + el : tl.y - 1);\n    const i64 nd = 3 * (i64)p.conn[(i64)p.elems[e] * " << ncn << " + k];\n"
       << "    xs[3 * k * E + el] = p.xyz[nd]; xs[(3 * k + 1) * E + el] = p.xyz[nd + 1]; xs[(3 * k + 2) * E + el] = p.xyz[nd + 2]; }\n";
-    s << "  for (int n = threadIdx.x; n < NG * E; n += blockDim.x) top[n] = 0;\n  __syncthreads();\n";
+    s << kLoop << "  for (int n = threadIdx.x; n < NG * E; n += blockDim.x) top[n] = 0;\n  __syncthreads();\n";
     auto point = [&](const char* indent) {
         s << indent << "const i64 e = tl.x + (base + el < tl.y ? base + el : tl.y - 1);\n";
         emit_geometry(s, dim, ncn, ngp, indent, true);
@@ -314,7 +319,7 @@ std::string jit_slice_source(const std::vector<const GroupDev*>& batch, int tier
     }
     for (size_t r0 = 0; r0 < ng; r0 += (size_t)sh.round) {
         const size_t r1 = std::min(ng, r0 + (size_t)sh.round);
-        s << (sh.single ? "  if (live) {\n" : "  for (int n = threadIdx.x; n < ") ;
+        s << (sh.single ? "" : kLoop) << (sh.single ? "  if (live) {\n" : "  for (int n = threadIdx.x; n < ");
         if (!sh.single) {
             s << ngp << " * E; n += blockDim.x) {\n    const int el = n % E, g = n / E;\n";
             point("    ");
@@ -333,21 +338,21 @@ std::string jit_slice_source(const std::vector<const GroupDev*>& batch, int tier
         for (size_t k = r0; k < r1; k++) {
             const int Q = batch[k]->nterms * ngp, Q16 = (Q + 15) / 16 * 16;
             if (Q16 > Q)
-                s << "  for (int n = threadIdx.x; n < " << Q16 - Q << " * E; n += blockDim.x) st[" << (k - r0) * place << " + " << Q + Q / 16
+                s << kLoop << "  for (int n = threadIdx.x; n < " << Q16 - Q << " * E; n += blockDim.x) st[" << (k - r0) * place << " + " << Q + Q / 16
                   << " * E + n] = 0;\n";
         }
         bool same = true;
         for (size_t k = r0; k < r1; k++) same = same && batch[k]->nterms == batch[r0]->nterms;
         // Scales.  The values of a column are looked at until the first that a
         // scale by powers of two would not hold exactly, as a rule its first.
-        s << "  __syncthreads();\n  for (int n = " << r0 << " * E + threadIdx.x; n < " << r1 << " * E; n += blockDim.x)\n"
+        s << "  __syncthreads();\n" << kLoop << "  for (int n = " << r0 << " * E + threadIdx.x; n < " << r1 << " * E; n += blockDim.x)\n"
           << "    if (grp.g[n / E].slices != nullptr) {\n";
         if (B == 8) {
             s << "      const int Q = ";
             for (size_t k = r0; !same && k + 1 < r1; k++) s << "n < " << k + 1 << " * E ? " << batch[k]->nterms * ngp << " : ";
             s << batch[r1 - 1]->nterms * ngp << ";\n      const double* v = st + (n / E - " << r0 << ") * " << place << " + n % E;\n"
               << "      bool exact = top[n] > 0;\n"
-              << "      for (int q = 0; exact && q < Q; q++) exact = slgpu::split_exact(v[(q + (q >> 4)) * E], top[n]);\n";
+              << kLoop << "      for (int q = 0; exact && q < Q; q++) exact = slgpu::split_exact(v[(q + (q >> 4)) * E], top[n]);\n";
         } else {
             s << "      const bool exact = false;\n";
         }
@@ -357,7 +362,7 @@ std::string jit_slice_source(const std::vector<const GroupDev*>& batch, int tier
         // side where they have equally many.
         auto chunks = [&](size_t a, size_t b) {
             const int Q = batch[a]->nterms * ngp, nc = (Q + 15) / 16, nchunk = (Q + 31) / 32 * 2;
-            s << "  for (int n = threadIdx.x; n < " << (b - a) * (size_t)nc << " * E; n += blockDim.x) {\n";
+            s << kLoop << "  for (int n = threadIdx.x; n < " << (b - a) * (size_t)nc << " * E; n += blockDim.x) {\n";
             s << "    const int el = n % E, gc = n / E, c = gc % " << nc << ", k = " << a << " + gc / " << nc << ";\n";
             s << "    uint4* out = grp.g[k].slices;\n    if (out == nullptr) continue;\n    out += ((tile * " << nchunk << " + c) * " << S
               << ") * 64 + base + el;\n";

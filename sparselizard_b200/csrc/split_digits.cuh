@@ -29,6 +29,8 @@ namespace slgpu {
 // as above: at most 21 significant bits (the low word is zero), the last of
 // them not below the unit 2^(46 - B S) of the power of two above h.
 //
+// split_pow2: 2^k, a normal double.
+//
 // split_digits: the S digits of x in units of 1 / f, byte k the digit
 // S - 1 - k.
 // B = 8, each plus 128: 1.5 2^52 + rint(x f) holds the integer in its low
@@ -45,8 +47,9 @@ SLGPU_DEVICE_SOURCE(
         return __double2loint(x) == 0 && (hx == 0 || (h >> 20) - (hx >> 20) <= 25);
     }
 
+    __device__ __forceinline__ double split_pow2(int k) { return __hiloint2double((1023 + k) << 20, 0); }
+
     template <int B, int S> __device__ __forceinline__ double split_scale(int h, bool exact, double* q, double* pre) {
-        const double unit = __longlong_as_double((long long)(1023 + B * S) << 52);
         *pre = 1.0;
         h = max(h, 1);
         if (h >= 0x7ff00000) {
@@ -55,16 +58,15 @@ SLGPU_DEVICE_SOURCE(
         }
         const bool tiny = h < ((1023 - 900) << 20);
         if (tiny || exact || B == 7) {
-            int ex;
-            frexp(__hiloint2double(h, -1), &ex);
-            ex += B == 7 ? 0 : 2;
-            *q = ldexp(1.0, ex - 8);
+            const int ex = (h < 0x100000 ? -1010 - __clz(h) : (h >> 20) - 1022) + (B == 7 ? 0 : 2);
+            const int up = tiny ? 512 : 0;
             *pre = tiny ? 0x1p512 : 1.0;
-            return ldexp(unit, -ex - (tiny ? 512 : 0));
+            *q = split_pow2(ex - 8 + up) * (tiny ? 0x1p-512 : 1.0);
+            return split_pow2(B * S - ex - up);
         }
         const double top = h >= 0x7fefffff ? __longlong_as_double(0x7fefffffffffffffll) : __hiloint2double(h + 1, 0);
         *q = top * (0x1p-8 / 0.498);
-        return 0.498 * unit / top;
+        return 0.498 * split_pow2(B * S) / top;
     }
 
     template <int B, int S> __device__ __forceinline__ unsigned long long split_digits(double x, double f) {
