@@ -2929,7 +2929,8 @@ void launch_contractions(Ctx* ctx, const Matrix& M, int precision, const std::ve
 // CSR value kernel: -1 = chosen per pattern by timing the candidates
 // (default), 0 = streaming warps (SLGPU_ROW_KERNEL=stream), 1 = warp per row
 // (SLGPU_ROW_KERNEL=warp), 2 = thread per row, rows of at most 32 entries
-// (SLGPU_ROW_KERNEL=thread).
+// (SLGPU_ROW_KERNEL=thread), 3 = warp per row with a window per row, float
+// values (SLGPU_ROW_KERNEL=row).
 static int row_kernel_forced()
 {
     static const int k = [] {
@@ -2940,6 +2941,8 @@ static int row_kernel_forced()
             return 0;
         if (v != nullptr && std::strcmp(v, "thread") == 0)
             return 2;
+        if (v != nullptr && std::strcmp(v, "row") == 0)
+            return 3;
         return -1;
     }();
     return k;
@@ -3024,14 +3027,14 @@ void launch_thread_rows(Ctx* ctx, const RowParams& rp, bool f32)
     ctx->launches++;
 }
 
-void launch_warp_rows(Ctx* ctx, RowParams rp, bool f32)
+void launch_warp_rows(Ctx* ctx, RowParams rp, bool f32, bool across)
 {
     // Consecutive rows per warp: up to kRowsPerWarp, fewer where that leaves
     // less than six times the warps that are resident: rows differ in length,
     // and the last warps run alone.  (One, four, eight, 16 times: tetrahedra of
     // FP32 elasticity 0.29, 0.117, 0.121, 0.120 ms; order-3 quadrangles 53, 43,
     // 49, 65 us; order-2 edge elements 0.354, 0.346, 0.342, 0.350 ms.)
-    const int64_t target = (int64_t)std::max(ctx->nsm, 1) * kRowBlocks * 8 * 6;
+    const int64_t target = (int64_t)std::max(ctx->nsm, 1) * (across ? kRowBlocks : kRowBlocksEach) * 8 * 6;
     rp.rows_per_warp = (int)std::min<int64_t>(kRowsPerWarp, std::max<int64_t>(1, rp.nrows / target));
     const size_t per_warp = (size_t)rp.lmax * 8;
     int wpb = (int)std::max<size_t>(1, std::min<size_t>(8, (48 * 1024) / per_warp));
@@ -3040,8 +3043,9 @@ void launch_warp_rows(Ctx* ctx, RowParams rp, bool f32)
         fail(SLGPU_E_UNSUPPORTED, "a CSR row is too long for the shared-memory row buffer");
     const unsigned grid = grid_for((rp.nrows + rp.rows_per_warp - 1) / rp.rows_per_warp, wpb);
     const bool U = rp.uniform_width > 0;
-    void (*kern)(RowParams) = f32 ? (U ? k_row_values<float, true> : k_row_values<float, false>)
-                                  : (U ? k_row_values<double, true> : k_row_values<double, false>);
+    void (*kern)(RowParams) = !f32     ? (U ? k_row_values<double, true> : k_row_values<double, false>)
+                              : across ? (U ? k_row_values<float, true> : k_row_values<float, false>)
+                                       : (U ? k_row_values_each<true> : k_row_values_each<false>);
     if (smem > 48 * 1024)
         raise_smem(ctx, kern, kSmemMax);
     kern<<<grid, 32 * wpb, smem, ctx->x->stream>>>(rp);
@@ -3093,23 +3097,27 @@ void launch_row_values(Ctx* ctx, const Matrix& M, Pattern& P, const std::vector<
     const StreamLaunch sl = stream_launch(ctx, rp, rsegs);
     const bool thread_ok = rp.lmax <= kThreadRowMax;
     // Candidates: warp per row always, streaming warps (double values) and
-    // thread per row where their shapes allow.
+    // thread per row where their shapes allow; a window per row for float
+    // values (k_row_values_each).
     std::vector<int> cand{1};
     if (sl.ok && !f32)
         cand.push_back(0);
     if (thread_ok)
         cand.push_back(2);
+    if (f32)
+        cand.push_back(3);
     auto launch = [&](int c) {
         if (c == 0)
             launch_stream_rows(ctx, sl);
         else if (c == 2)
             launch_thread_rows(ctx, rp, f32);
         else
-            launch_warp_rows(ctx, rp, f32);
+            launch_warp_rows(ctx, rp, f32, c == 1);
     };
     int choice = row_kernel_forced();
+    int& chosen = P.row_kernel[f32 ? 1 : 0];
     if (choice < 0)
-        choice = P.row_kernel;
+        choice = chosen;
     // A kernel this call cannot use (the streaming warps with float values):
     // warp per row.
     if (choice >= 0 && std::find(cand.begin(), cand.end(), choice) == cand.end())
@@ -3119,7 +3127,7 @@ void launch_row_values(Ctx* ctx, const Matrix& M, Pattern& P, const std::vector<
         // identical), warp per row being the default.
         const int kt = kstat_start(ctx, "row_values", 0.0);
         int runs = 0;
-        P.row_kernel = pick_by_timing(ctx, cand, [&](int c) {
+        chosen = pick_by_timing(ctx, cand, [&](int c) {
             launch(c);
             runs++;
         });
@@ -3228,7 +3236,7 @@ static std::vector<uint64_t> value_signature(Ctx* ctx, const Matrix& M, int prec
     u((uint64_t)precision);
     u(rhs ? 1 : 0);
     p(&P);
-    u((uint64_t)P.row_kernel + 1);
+    u((uint64_t)(P.row_kernel[0] + 1) << 8 | (uint64_t)(P.row_kernel[1] + 1));
     u((uint64_t)M.ndofs);
     p(M.vals.as<void>());
     p(M.Avals.as<void>());
@@ -3652,10 +3660,12 @@ int slgpu_tuned_tiles(slgpu_ctx* ctx, char* buf, size_t len)
             t += "fp64 rows/block=" + std::to_string(kv.second) + " for ntf " + std::to_string(k[0]) + " ndof " + std::to_string(k[1]) +
                  " ngp " + std::to_string(k[2]) + "\n";
         }
+        const char* const kernels[] = {"untimed", "stream", "warp", "thread", "row"};
         for (const auto& p : ctx->patterns)
-            if (p)
-                t += std::string("csr values kernel=") + (p->row_kernel == 0 ? "stream" : p->row_kernel == 1 ? "warp" : p->row_kernel == 2 ? "thread" : "untimed") +
-                     " for " + std::to_string(p->nA) + " rows\n";
+            for (int f32 = 0; p && f32 < 2; f32++)
+                if (f32 == 0 || p->row_kernel[1] >= 0)
+                    t += std::string("csr values kernel=") + kernels[p->row_kernel[f32] + 1] + " for " + std::to_string(p->nA) + " rows" +
+                         (f32 != 0 ? ", float values" : "") + "\n";
         if (buf != nullptr && len > 0)
             std::snprintf(buf, len, "%s", t.c_str());
     });

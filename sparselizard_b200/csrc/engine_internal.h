@@ -188,7 +188,7 @@ struct Pattern {
     uint64_t serial = 0;   // unique per pattern built by the context
     int64_t ndofs = 0, nA = 0, nD = 0, nnzA = 0, nnzD = 0, ncoo = 0, nvalid = 0, ninc = 0;
     int lmax = 0;          // longest row (A and D entries)
-    int row_kernel = -1;   // CSR value kernel chosen by timing: 0 streaming warps, 1 warp per row, -1 not yet
+    int row_kernel[2] = {-1, -1};  // CSR value kernel chosen by timing for double and for float values (-1: not yet)
     DevBuf Arows, Acols, Drows, Dcols;
     DevBuf ainds, dinds;   // int32 [nA], [nD]: global DOF of each local row of A / column of D
     DevBuf slotmap;        // int16 [ncoo]: position in the row's [A | D] segment, -1 = dropped

@@ -1343,4 +1343,126 @@ __global__ void __launch_bounds__(256, kRowBlocks) k_row_values(RowParams p)
     while (rr < nr) write_back();
 }
 
+// The same sums from float values with a window of incidences per row.  Rows of
+// many incidences leave few lanes of such a window idle, and with half the bytes
+// per gather the windows across rows are bound by their own instructions; this
+// loop needs fewer (and 40 registers, 48 warps per multiprocessor).  Order-2
+// elasticity, 48^3 hexahedra: 2.63 ms against 2.85 across rows; order-2 edge
+// elements on 162,000 tetrahedra 1.16 against 1.34; order-3 quadrangles, of 2
+// incidences a row, 60 against 48 us: picked by timing per pattern.  (Double
+// values: 2.80 against 2.84, 1.28 against 1.13 ms, 64 against 49 us.)
+constexpr int kRowBlocksEach = 6;
+
+template <bool U>
+__global__ void __launch_bounds__(256, kRowBlocksEach) k_row_values_each(RowParams p)
+{
+    const float* vals = reinterpret_cast<const float*>(p.vals);
+    extern __shared__ double rowbuf[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t r0 = ((int64_t)blockIdx.x * (blockDim.x >> 5) + warp) * p.rows_per_warp;
+    if (r0 >= p.nrows)
+        return;
+    const int nr = (int)min((int64_t)p.rows_per_warp, p.nrows - r0);
+    double* buf = rowbuf + (int64_t)warp * p.lmax;
+    // The row buffer is kept zero between rows (the write-back clears it).
+    for (int s = lane; s < p.lmax; s += 32) buf[s] = 0.0;
+    // Row bounds of the warp's rows, one per lane (lane nr: the end).
+    uint32_t a_lo = 0, d_lo = 0, i_lo = 0;
+    if (lane <= nr) {
+        a_lo = p.Arows[r0 + lane];
+        d_lo = p.Drows ? p.Drows[r0 + lane] : 0u;
+        i_lo = p.inc_ptr[r0 + lane];
+    }
+    __syncwarp();
+    constexpr uint32_t kGeneric = 1u << 17, kSerial = 1u << 16;
+    for (int rr = 0; rr < nr; rr++) {
+        // The CSR bounds are fetched after the incidences (only the
+        // write-back needs them): fewer registers live in the loop below.
+        const uint32_t k0 = __shfl_sync(0xffffffffu, i_lo, rr), k1 = __shfl_sync(0xffffffffu, i_lo, rr + 1);
+        for (uint32_t kb = k0; kb < k1; kb += 32) {
+            const int nkb = (int)min(32u, k1 - kb);
+            uint32_t voff = 0, coo = 0;
+            double mult = 0.0;
+            uint32_t info = 0;  // width | kSerial | kGeneric | value offset bits 32 .. 45 from bit 18
+            if (lane < nkb) {
+                const unsigned long long pk = p.inc[kb + lane];
+                const RowSeg sg = p.segs[(pk >> 40) & ((1ull << 23) - 1)];
+                const uint32_t n = (uint32_t)pk;  // fewer than 2^32 incidences
+                coo = (uint32_t)sg.coo_base + n * (uint32_t)sg.width;
+                const uint64_t v = 2 * (uint64_t)sg.val_base + (uint64_t)n * (uint32_t)sg.ld;
+                voff = (uint32_t)v;
+                mult = sg.mult;
+                const bool serial = (pk >> 63) != 0;
+                info = (uint32_t)sg.width | (serial ? kSerial : 0) | ((serial || sg.width > 32) ? kGeneric : 0) | (uint32_t)(v >> 32) << 18;
+            }
+            if (!__any_sync(0xffffffffu, (info & kGeneric) != 0)) {
+                for (int u = 0; u < nkb; u += kRowBatch) {
+                    double val[kRowBatch];
+                    int slot[kRowBatch];
+#pragma unroll
+                    for (int x = 0; x < kRowBatch; x++) {
+                        const int src = (u + x) & 31;
+                        uint64_t vo = __shfl_sync(0xffffffffu, voff, src);
+                        const uint32_t co = __shfl_sync(0xffffffffu, coo, src);
+                        int w = p.uniform_width;
+                        if constexpr (!U) {
+                            const uint32_t inf = __shfl_sync(0xffffffffu, info, src);
+                            w = (int)(inf & 0xffff);
+                            vo |= (uint64_t)(inf >> 18) << 32;
+                        }
+                        slot[x] = -1;
+                        val[x] = 0.0;
+                        if (u + x < nkb && lane < w) {
+                            slot[x] = p.slotmap[(uint64_t)co + lane];
+                            val[x] = (double)vals[vo + lane];
+                        }
+                    }
+#pragma unroll
+                    for (int x = 0; x < kRowBatch; x++) {
+                        if (u + x < nkb) {
+                            if constexpr (U) {
+                                if (slot[x] >= 0)
+                                    buf[slot[x]] = val[x] + buf[slot[x]];
+                            } else {
+                                const double m = __shfl_sync(0xffffffffu, mult, (u + x) & 31);
+                                if (slot[x] >= 0)
+                                    buf[slot[x]] = fma(val[x], m, buf[slot[x]]);
+                            }
+                            __syncwarp();
+                        }
+                    }
+                }
+            } else {
+                for (int x = 0; x < nkb; x++) {
+                    const uint32_t inf = __shfl_sync(0xffffffffu, info, x);
+                    const uint64_t vo = __shfl_sync(0xffffffffu, voff, x) | (uint64_t)(inf >> 18) << 32;
+                    const uint32_t co = __shfl_sync(0xffffffffu, coo, x);
+                    const double m = __shfl_sync(0xffffffffu, mult, x);
+                    row_add_generic(buf, (int)(inf & 0xffff), m, vals + vo, p.slotmap + co, (inf & kSerial) != 0, lane);
+                    __syncwarp();
+                }
+            }
+        }
+        const uint32_t a0 = __shfl_sync(0xffffffffu, a_lo, rr), a1 = __shfl_sync(0xffffffffu, a_lo, rr + 1);
+        const uint32_t d0 = __shfl_sync(0xffffffffu, d_lo, rr), d1 = __shfl_sync(0xffffffffu, d_lo, rr + 1);
+        const int la = (int)(a1 - a0), L = la + (int)(d1 - d0);
+        if (p.dense != nullptr) {
+            if (lane == 0)
+                p.dense[r0 + rr] = L > 0 ? -buf[0] : 0.0;
+            __syncwarp();
+            for (int s = lane; s < L; s += 32) buf[s] = 0.0;
+        } else {
+            for (int s = lane; s < L; s += 32) {
+                const double v = buf[s];
+                buf[s] = 0.0;
+                if (s < la)
+                    p.Avals[a0 + s] = v;
+                else
+                    p.Dvals[d0 + (s - la)] = v;
+            }
+        }
+        __syncwarp();
+    }
+}
+
 }  // namespace slgpu

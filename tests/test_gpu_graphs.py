@@ -417,3 +417,39 @@ np.savez(sys.argv[1], **out)
         assert np.abs(r[b + "0"]).max() > 0
         for k in range(10):
             assert np.array_equal(r[f"{b}{k}"], r[b + "0"] * (2.0 if 4 <= k < 8 else 1.0)), f"{b}, call {k}"
+
+
+def test_float_value_kernels_agree(tmp_path):
+    """FP32-level steps through the warp kernels with windows of incidences
+    across rows and per row, each forced in its own process: the same values
+    bit for bit.  Rows of one to thousands of incidences, 1 to 31 rows a warp,
+    widths up to and above a warp, repeated addresses, multipliers that are and
+    are not 1."""
+    import os
+    import subprocess
+    import sys
+
+    code = """
+import sys
+import numpy as np
+from sparselizard_b200 import abi
+import test_gpu_graphs as T
+ctx, out = abi.Context(0), {}
+for k, (grid, ntf, ndof, ndofs) in enumerate([(9, 8, 8, 40), (60, 9, 9, 3000), (150, 8, 8, 100000), (260, 8, 8, 400000), (30, 8, 40, 4000),
+                                              (40, 8, 32, 9000), (40, 8, 33, 9000)]):
+    t = T._setup(ctx, np.random.Generator(np.random.PCG64(63 + k)), k, grid, ntf, ndof, 1, 2, ndofs)
+    for mult in ([1.0, 1.0], [3.0, -2.5]):
+        ctx.check(ctx.lib.slgpu_matrix_set_scales(ctx.h, t["h"], 0, None, abi.f64p(np.array(mult))))
+        out["%d_%g_A" % (k, mult[0])], out["%d_%g_D" % (k, mult[0])] = T._process(ctx, t, abi.PREC_FP32)
+np.savez(sys.argv[1], **out)
+"""
+    here = os.path.dirname(os.path.abspath(__file__))
+    res = {}
+    for k in ("warp", "row"):
+        out = str(tmp_path / f"{k}.npz")
+        env = dict(os.environ, SLGPU_ROW_KERNEL=k, PYTHONPATH=os.pathsep.join([here, os.path.dirname(here)]))
+        subprocess.run([sys.executable, "-c", code, out], env=env, check=True, timeout=300)
+        res[k] = np.load(out)
+    for key in res["warp"].files:
+        a, b = res["warp"][key], res["row"][key]
+        assert np.all(np.isfinite(a)) and np.abs(a).max() > 0 and np.array_equal(a, b), key
