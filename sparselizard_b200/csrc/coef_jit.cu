@@ -223,9 +223,9 @@ std::string jit_coef_source(const std::vector<const GroupDev*>& batch)
 //   More: 4 elements (the 16-byte stores of 4 neighbouring slots are two whole
 //   sectors) and several points per thread.
 // A round holds as many groups as leave room for four blocks per
-// multiprocessor.  (Order-2 elasticity, 9 groups of 243 values on 27 points,
-// all staged at once: two blocks fit, and the kernel took 0.68 instead of
-// 0.49 ms at 48^3.)
+// multiprocessor, which the registers allow too (72).  (Order-2 elasticity, 9
+// groups of 243 values on 27 points, all staged at once: two blocks fit, and
+// the kernel took 0.68 instead of 0.49 ms at 48^3.)
 static size_t slice_staged(const GroupDev& g) { return ((size_t)g.nterms * g.ngp + 15) / 16 * 17; }
 
 SliceShape slice_shape(const std::vector<const GroupDev*>& batch)
@@ -255,7 +255,7 @@ SliceShape slice_shape(const std::vector<const GroupDev*>& batch)
 // writes them and one that slices them wrote 8, read 8 and wrote S; and an
 // element's nodes are gathered once, not once per point.  Orders 1-5, 48,000
 // tetrahedra: 0.42 -> 0.17 ms a step; order-2 elasticity, 48^3 hexahedra:
-// 0.65 -> 0.49 ms.  (Evaluating twice instead of staging
+// 0.65 -> 0.42 ms.  (Evaluating twice instead of staging
 // took 0.54 ms there.)
 //
 // Value q of element el of a group is at (q + q / 16) E + el of the group's
@@ -282,19 +282,19 @@ std::string jit_slice_source(const std::vector<const GroupDev*>& batch, int tier
       << "__device__ __forceinline__ double quotient(double a, double b, double r, bool wide)\n{\n"
       << "  if (wide) return divided(a, b);\n  const double q = a * r;\n  return fma(fma(-q, b, a), r, q);\n}\n";
     // One chunk: 16 staged values from `at` on, E apart, to the slices at out.
-    // Not inlined: one copy for all rounds (compile time).
+    // Not inlined: one copy for all rounds (compile time).  pr is 1 but for
+    // magnitudes below 2^-900 (split_scale); a second copy without the product
+    // took 50 ms more to compile and ran no faster.
     s << "extern __shared__ __align__(16) double st[];\n";
-    for (int fast = 1; fast >= 0; fast--) {
-        s << "__device__ __noinline__ void cut_" << (fast ? "plain" : "tiny") << "(int at, double f, double pr, uint4* out)\n{\n";
-        s << "  unsigned int wd[" << S << "][4];\n  #pragma unroll\n  for (int k4 = 0; k4 < 4; k4++) {\n    unsigned long long u[4];\n    #pragma unroll\n"
-          << "    for (int i = 0; i < 4; i++) u[i] = slgpu::split_digits<" << B << ", " << S << ">(st[at + (4 * k4 + i) * " << sh.E << "]"
-          << (fast ? "" : " * pr") << ", f);\n    slgpu::split_words<" << B << ", " << S << ">(u, wd, k4);\n  }\n";
-        s << "  #pragma unroll\n  for (int i = 0; i < " << S << "; i++) out[i * 64] = make_uint4(wd[i][0], wd[i][1], wd[i][2], wd[i][3]);\n}\n";
-    }
+    s << "__device__ __noinline__ void cut(int at, double f, double pr, uint4* out)\n{\n";
+    s << "  unsigned int wd[" << S << "][4];\n  #pragma unroll\n  for (int k4 = 0; k4 < 4; k4++) {\n    unsigned long long u[4];\n    #pragma unroll\n"
+      << "    for (int i = 0; i < 4; i++) u[i] = slgpu::split_digits<" << B << ", " << S << ">(st[at + (4 * k4 + i) * " << sh.E
+      << "] * pr, f);\n    slgpu::split_words<" << B << ", " << S << ">(u, wd, k4);\n  }\n";
+    s << "  #pragma unroll\n  for (int i = 0; i < " << S << "; i++) out[i * 64] = make_uint4(wd[i][0], wd[i][1], wd[i][2], wd[i][3]);\n}\n";
     // Loops over the block's work, which take a few turns each, stay loops:
     // unrolled, nine groups of elasticity took 1.0 to 1.1 s to compile instead of
-    // 0.5 to 0.65, and the calls in them cost registers (48^3 hexahedra 0.66
-    // instead of 0.49 ms, FP32 tetrahedra 101 instead of 87 us).
+    // 0.5 to 0.65, and the calls in them cost registers (94 instead of 72; 48^3
+    // hexahedra 0.66 instead of 0.49 ms, FP32 tetrahedra 101 instead of 87 us).
     const char* const kLoop = "#pragma unroll 1\n";
     s << "extern \"C\" __global__ void __launch_bounds__(" << sh.threads << ") slgpu_slices(JitGeom p, const JitSlices grp, const int4* tiles)\n{\n";
     s << "  constexpr int E = " << sh.E << ", NG = " << ng << ";\n";
@@ -367,7 +367,7 @@ std::string jit_slice_source(const std::vector<const GroupDev*>& batch, int tier
             s << "    uint4* out = grp.g[k].slices;\n    if (out == nullptr) continue;\n    out += ((tile * " << nchunk << " + c) * " << S
               << ") * 64 + base + el;\n";
             s << "    const double f = fac[k * E + el], pr = pre[k * E + el];\n    const int at = (k - " << r0 << ") * " << place
-              << " + 17 * c * E + el;\n    if (pr == 1.0) cut_plain(at, f, pr, out); else cut_tiny(at, f, pr, out);\n  }\n";
+              << " + 17 * c * E + el;\n    cut(at, f, pr, out);\n  }\n";
         };
         if (same)
             chunks(r0, r1);
