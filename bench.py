@@ -281,6 +281,10 @@ def run_reference(args, spec):
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
         return
+    if not os.path.exists(REF_LIB):
+        print(json.dumps({"impl": "reference", "unavailable": f"{os.path.relpath(REF_LIB, ROOT)} is not built (it is linked from sparselizard's "
+                          "sources, which are absent)"}), flush=True)
+        return
     threads = os.cpu_count() or 1
     n_sample = spec["ref_n"]
     # The W warm-up steps run the same path on the half-size mesh (untimed),
