@@ -106,10 +106,10 @@ void emit_geometry(std::ostringstream& s, int dim, int ncn, int ngp, const char*
                    {"I20", "(J10 * J21 - J11 * J20)"}, {"I21", "(J01 * J20 - J00 * J21)"}, {"I22", "(J00 * J11 - J01 * J10)"}};
         }
         if (staged)
-            s << indent << "const double rd = 1.0 / det;\n" << indent << "const bool wide = !(fabs(det) > 0x1p-500 && fabs(det) < 0x1p500);\n";
+            s << indent << "const double rd = 1.0 / det;\n" << indent << "const bool odd = !(fabs(det) >= 0x1p-1022 && fabs(det) < 0x1p1021);\n";
         for (const auto& i : inv)
             if (staged)
-                s << indent << "const double " << i.first << " = quotient(" << i.second << ", det, rd, wide);\n";
+                s << indent << "const double " << i.first << " = quotient(" << i.second << ", det, rd, odd);\n";
             else
                 s << indent << "const double " << i.first << " = " << i.second << " / det;\n";
     }
@@ -275,12 +275,13 @@ std::string jit_slice_source(const std::vector<const GroupDev*>& batch, int tier
     s << "struct JitSlices { JitSlice g[" << ng << "]; };\n";
     // quotient: a / b, r = 1 / b correctly rounded.  The residual of a r corrects
     // it to the rounded quotient (P. Markstein, IBM J. Res. Dev. 34, 1990), in two
-    // fma where a division takes its own reciprocal: slices of 48,000 tetrahedra of
-    // orders 1-5 193 us with divisions, 168 with this, 156 with a r alone, which
-    // misses the last place.  Outside of 2^+-500 it is a division.
-    s << "__device__ __noinline__ double divided(double a, double b) { return a / b; }\n"
-      << "__device__ __forceinline__ double quotient(double a, double b, double r, bool wide)\n{\n"
-      << "  if (wide) return divided(a, b);\n  const double q = a * r;\n  return fma(fma(-q, b, a), r, q);\n}\n";
+    // fma where a division takes its own reciprocal: with divisions the slices of
+    // 48,000 tetrahedra of orders 1-5 took 37 us more than with a r alone, which
+    // misses the last place; with this they take 151 us.  `odd` (b zero, no normal
+    // double, or within 8 of the overflow): a r.  (A division there instead, by a
+    // branch, held 64 registers instead of 47: 166 us.)
+    s << "__device__ __forceinline__ double quotient(double a, double b, double r, bool odd)\n{\n"
+      << "  const double q = a * r, c = fma(fma(-q, b, a), r, q);\n  return odd ? q : c;\n}\n";
     // One chunk: 16 staged values from `at` on, E apart, to the slices at out.
     // Not inlined: one copy for all rounds (compile time).  pr is 1 but for
     // magnitudes below 2^-900 (split_scale); a second copy without the product
