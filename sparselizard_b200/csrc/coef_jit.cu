@@ -254,8 +254,8 @@ SliceShape slice_shape(const std::vector<const GroupDev*>& batch)
 // never go to memory: per coefficient S bytes are written, where a kernel that
 // writes them and one that slices them wrote 8, read 8 and wrote S; and an
 // element's nodes are gathered once, not once per point.  Orders 1-5, 48,000
-// tetrahedra: 0.42 -> 0.17 ms a step; order-2 elasticity, 48^3 hexahedra:
-// 0.65 -> 0.42 ms.  (Evaluating twice instead of staging
+// tetrahedra: 0.42 -> 0.15 ms a step; order-2 elasticity, 48^3 hexahedra:
+// 0.65 -> 0.47 ms.  (Evaluating twice instead of staging
 // took 0.54 ms there.)
 //
 // Value q of element el of a group is at (q + q / 16) E + el of the group's

@@ -152,31 +152,48 @@ __global__ void k_slice_rows(RowSliceParams p)
         top = 0;
         rounded = 0;
     }
+    // The thread's first kRowKeep entries stay in registers (Q <= 1024); later
+    // ones are formed again in every pass.
+    constexpr int kRowKeep = 4;
+    double kept[kRowKeep];
+#pragma unroll
+    for (int k = 0; k < kRowKeep; k++) {
+        const int q = threadIdx.x + k * blockDim.x;
+        kept[k] = q < p.Qpad ? m_entry(p, o, src, q) : 0.0;
+    }
+    auto each = [&](auto f) {
+#pragma unroll
+        for (int k = 0; k < kRowKeep; k++)
+            if ((int)(threadIdx.x + k * blockDim.x) < p.Qpad)
+                f((int)(threadIdx.x + k * blockDim.x), kept[k]);
+        for (int q = threadIdx.x + kRowKeep * blockDim.x; q < p.Qpad; q += blockDim.x) f(q, m_entry(p, o, src, q));
+    };
     __syncthreads();
     // Magnitudes compare as their bit patterns (NaN above infinity).
     int mx = 0;
-    for (int q = threadIdx.x; q < p.Qpad; q += blockDim.x) mx = max(mx, __double2hiint(m_entry(p, o, src, q)) & 0x7fffffff);
+    each([&](int, double x) { mx = max(mx, __double2hiint(x) & 0x7fffffff); });
     atomicMax(&top, mx);
     __syncthreads();
-    for (int q = threadIdx.x; B == 8 && q < p.Qpad; q += blockDim.x)
-        if (!split_exact(m_entry(p, o, src, q), top)) {
+    if constexpr (B == 8) {
+        bool exact = true;
+        each([&](int, double x) { exact = exact && split_exact(x, top); });
+        if (!exact)
             rounded = 1;
-            break;
-        }
-    __syncthreads();
+        __syncthreads();
+    }
     double unit, pre;
     const double f = split_scale<B, S>(top, B == 8 && rounded == 0, &unit, &pre);
     if (threadIdx.x == 0)
         p.rowscale[(int64_t)o * p.Ppad + pe] = ldexp(unit, 16 - B * p.L);
     const int ntp = p.Ppad / kSplitM, nk = p.Qpad / kSplitKStep;
     const int pt = pe / kSplitM, r = pe % kSplitM;
-    for (int q = threadIdx.x; q < p.Qpad; q += blockDim.x) {
-        const unsigned long long u = split_digits<B, S>(m_entry(p, o, src, q) * pre, f);
+    each([&](int q, double x) {
+        const unsigned long long u = split_digits<B, S>(x * pre, f);
         const int ks = q / kSplitKStep, c = (q / 16) & 1;
         for (int s = 0; s < S; s++)
             p.slices[(((((int64_t)o * ntp + pt) * nk + ks) * S + s) * 2 + c) * (kSplitM * 16) + r * 16 + (q & 15)] =
                 (int8_t)((u >> (8 * (S - 1 - s))) ^ split_flip<B>());
-    }
+    });
 }
 
 // Column slices of coefficients in memory: thread per (64-element tile, slot); C[q][e] is read
