@@ -158,13 +158,11 @@ def peaks():
 # launch's group (traffic grows in proportion to the elements).  Summaries
 # and the commands that made them are under profiles/.
 TRAFFIC_PER_ELEMENT = {
-    # profiles/k_contract_split_elasticity_hex32.md, 32768 elements: the one
-    # launch of a step (all six contracted groups) reads 417.57 MB and writes
-    # 1721.87 MB.
-    ("c2", "contract_split"): (417.574912e6 + 1721.872e6) / 32768,
-    # profiles/k_row_values_elasticity_hex32.md: 3.140 GB read + 1.187 GB
-    # written by the launch over all 9 groups of 32768 elements.
-    ("c2", "row_values"): (3.140404e9 + 1.187079e9) / 32768,
+    # profiles/step_elasticity_hex32_split.md, 32768 elements: the one
+    # contraction launch of a step reads 310.22 MB and writes 1726.88 MB, the
+    # value launch over all 9 groups 3.457 GB and 1.184 GB.
+    ("c2", "contract_split"): (310.222592e6 + 1726.877952e6) / 32768,
+    ("c2", "row_values"): (3.457268e9 + 1.184208e9) / 32768,
 }
 
 

@@ -223,9 +223,10 @@ std::string jit_coef_source(const std::vector<const GroupDev*>& batch)
 //   More: 4 elements (the 16-byte stores of 4 neighbouring slots are two whole
 //   sectors) and several points per thread.
 // A round holds as many groups as leave room for four blocks per
-// multiprocessor, which the registers allow too (72).  (Order-2 elasticity, 9
-// groups of 243 values on 27 points, all staged at once: two blocks fit, and
-// the kernel took 0.68 instead of 0.49 ms at 48^3.)
+// multiprocessor in shared memory.  (Order-2 elasticity, 9 groups of 243 values
+// on 27 points, all staged at once: two blocks fit, and the kernel took 0.68
+// instead of 0.49 ms at 48^3.  Its 80 registers then allow three blocks, those
+// of the smaller kernels, 47 to 56, four or more.)
 static size_t slice_staged(const GroupDev& g) { return ((size_t)g.nterms * g.ngp + 15) / 16 * 17; }
 
 SliceShape slice_shape(const std::vector<const GroupDev*>& batch)
@@ -294,8 +295,8 @@ std::string jit_slice_source(const std::vector<const GroupDev*>& batch, int tier
     s << "  #pragma unroll\n  for (int i = 0; i < " << S << "; i++) out[i * 64] = make_uint4(wd[i][0], wd[i][1], wd[i][2], wd[i][3]);\n}\n";
     // Loops over the block's work, which take a few turns each, stay loops:
     // unrolled, nine groups of elasticity took 1.0 to 1.1 s to compile instead of
-    // 0.5 to 0.65, and the calls in them cost registers (94 instead of 72; 48^3
-    // hexahedra 0.66 instead of 0.49 ms, FP32 tetrahedra 101 instead of 87 us).
+    // 0.5 to 0.65, and the calls in them cost 22 registers (48^3 hexahedra 0.66
+    // instead of 0.49 ms, FP32 tetrahedra 101 instead of 87 us).
     const char* const kLoop = "#pragma unroll 1\n";
     s << "extern \"C\" __global__ void __launch_bounds__(" << sh.threads << ") slgpu_slices(JitGeom p, const JitSlices grp, const int4* tiles)\n{\n";
     s << "  constexpr int E = " << sh.E << ", NG = " << ng << ";\n";

@@ -3056,9 +3056,9 @@ void launch_warp_rows(Ctx* ctx, RowParams rp, bool f32, bool across)
 
 // Step 4 on the current execution state's stream: A/D values (or the dense
 // right-hand side) from the element values through the resident pattern.
-// `dsegs` is the device copy of `rsegs`.  The two value kernels add in the
+// `dsegs` is the device copy of `rsegs`.  The value kernels all add in the
 // same order (bit-identical results); the first process() of a pattern on
-// the context's own stream times both on its data and keeps the faster one
+// the context's own stream times them on its data and keeps the fastest one
 // for the pattern.
 void launch_row_values(Ctx* ctx, const Matrix& M, Pattern& P, const std::vector<RowSeg>& rsegs, const RowSeg* dsegs, bool rhs,
                        bool f32, const double* vals, double* Avals, double* Dvals)
